@@ -9,11 +9,18 @@
 
 namespace pb {
 
+// row of element t of an n x nvec view with tot elements: a 32-bit division
+// (a few instructions instead of some eighty) while the count allows
+__device__ __forceinline__ int64_t pb_elem_row(int64_t t, int nvec, int64_t tot)
+{
+  return tot <= 0xffffffffll ? (int64_t)((uint32_t)t / (uint32_t)nvec) : t / nvec;
+}
+
 // grid-stride over all (row, col) elements of an n x nvec view
 #define PB_FOR_ELEMS(n, nvec, i, j)                                                  \
   for (int64_t t_ = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, tot_ = (n) * (nvec); \
        t_ < tot_; t_ += (int64_t)gridDim.x * blockDim.x)                              \
-    for (int64_t i = t_ / (nvec), j = t_ - i * (nvec), once_ = 0; once_ < 1; once_++)
+    for (int64_t i = pb_elem_row(t_, (nvec), tot_), j = t_ - i * (nvec), once_ = 0; once_ < 1; once_++)
 
 template <class T>
 __global__ void k_put_value(T* v, int64_t ld, int64_t n, int nvec, T val)
