@@ -20,6 +20,7 @@
 #include "pb_prec.cuh"
 #include "pb_tile.cuh"
 #include "pb_dmma.cuh"
+#include "pb_frag.cuh"
 
 namespace pb {
 
@@ -1175,6 +1176,7 @@ template <class T>
 void launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const T* W,
                   int64_t ldw, T beta, T* Cd, int64_t ldc)
 {
+  if (frag_mvTmv<T>(n, m, k, alpha, V, ldv, W, ldw, beta, Cd, ldc)) return;
   MvTmvArgs<T> a;
   a.n = n; a.m = m; a.k = k; a.V = V; a.ldv = ldv; a.W = W; a.ldw = ldw;
   a.alpha = alpha; a.beta = beta; a.Cd = Cd; a.ldc = ldc;
@@ -1203,7 +1205,10 @@ void launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, con
       return;
     }
   }
-  if (m <= 64 && k <= 64 && vec_ok(V, ldv, m) && vec_ok(W, ldw, k)) {
+  // thin blocks: one thread per row (n = 2,097,152, staged -> per row: FP64
+  // 2 x 2 39 -> 30 us, FP32 4 x 4 41 -> 29, 8 x 4 49 -> 39)
+  const bool thin = std::min(m, k) <= 4 && std::max(m, k) <= (sizeof(T) == 4 ? 8 : 4);
+  if (!thin && m <= 64 && k <= 64 && vec_ok(V, ldv, m) && vec_ok(W, ldw, k)) {
     // multi-stage asynchronously staged row tiles, widths padded to 4..64
     mvtmv_async<T>(a, n, pad_width5(m), pad_width5(k));
     PB_LAUNCH_CHECK();
@@ -1251,86 +1256,6 @@ void launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, con
     kern<<<grid, BLK_BS, smem, stream()>>>(a);
   }
   PB_LAUNCH_CHECK();
-}
-
-// k_mvsd_async launch for padded widths BM x BK: TC output columns per
-// thread (TX = BK/TC threads per row), TR rows per thread, sized for about
-// 24 KiB of staged input rows per stage; 4 stages (3 where a stage is
-// larger), two blocks per SM
-template <class T, int BM, int BK>
-void mvsd_async_launch(RowGemmArgs<T>& a)
-{
-  constexpr int TC = BK >= 16 ? 4 : BK / 4;
-  constexpr int TX = BK / TC, TY = 256 / TX;
-  constexpr int AP = BM + 16 / (int)sizeof(T);
-  constexpr int TR0 = 24576 / (TY * AP * (int)sizeof(T));
-  constexpr int TR = TR0 < 1 ? 1 : TR0 > 8 ? 8 : TR0;
-  constexpr int R = TY * TR;
-  constexpr int S = (R * AP * (int)sizeof(T) > 30000) ? 3 : 4;
-  const size_t smem = sizeof(T) * ((size_t)BM * BK + (size_t)S * R * AP);
-  const int grid = (int)std::min<int64_t>(ceil_div(a.n > 0 ? a.n : 1, R), (int64_t)rt().num_sms() * 2);
-  if constexpr (std::is_same<T, double>::value && BM >= 8 && BK >= 8) {
-    // FP64 on the tensor cores (DMMA), rows staged by TMA
-    constexpr int DAP = BM + 4, DCP = BK + 4;
-    constexpr int DR = (DAP * 8 * 128 <= 24576) ? 128 : 64;
-    constexpr int DS = (DR * DAP * 8 > 30000) ? 3 : 4;
-    constexpr int DCSZ = (BM * DCP * 8 + 127) / 128 * 128 / 8;
-    const T* A = (a.mode == RM_MVSDI) ? (const T*)a.W : a.V;
-    const int64_t lda = (a.mode == RM_MVSDI) ? a.ldw : a.ldv;
-    CUtensorMap mA;
-    if (rt().use_tma && rt().use_dmma && make_rows_tmap<T>(&mA, A, a.n, a.m, lda, DAP, DR)) {
-      const size_t dsmem = sizeof(T) * ((size_t)DCSZ + (size_t)DS * DR * DAP) + 8 * DS;
-      const int dgrid = (int)std::min<int64_t>(ceil_div(a.n, DR), (int64_t)rt().num_sms() * 2);
-      auto kd = k_mvsd_dmma<BM, BK, DR, DS>;
-      set_smem(kd, dsmem);
-      kd<<<dgrid, BLK_BS, dsmem, stream()>>>(a, mA, rt().device_error_word());
-      return;
-    }
-  }
-  {
-    // TMA staging of the input rows where a tensor map describes them
-    constexpr int TRT = (TY * TR > 256) ? 256 / TY : TR;
-    constexpr int RT = TY * TRT;
-    const T* A = (a.mode == RM_MVSDI) ? (const T*)a.W : a.V;
-    const int64_t lda = (a.mode == RM_MVSDI) ? a.ldw : a.ldv;
-    CUtensorMap mapA;
-    if (rt().use_tma && make_rows_tmap<T>(&mapA, A, a.n, a.m, lda, AP, RT)) {
-      constexpr int CSZ = (BM * BK * (int)sizeof(T) + 127) / 128 * 128 / (int)sizeof(T);
-      const size_t tsmem = sizeof(T) * ((size_t)CSZ + (size_t)S * RT * AP) + 8 * S;
-      const int tgrid = (int)std::min<int64_t>(ceil_div(a.n, RT), (int64_t)rt().num_sms() * 2);
-      auto kt = k_mvsd_tma<T, BM, BK, TRT, TC, S>;
-      set_smem(kt, tsmem);
-      kt<<<tgrid, BLK_BS, tsmem, stream()>>>(a, mapA, rt().device_error_word());
-      return;
-    }
-  }
-  auto kern = k_mvsd_async<T, BM, BK, TR, TC, S>;
-  set_smem(kern, smem);
-  kern<<<grid, BLK_BS, smem, stream()>>>(a);
-}
-
-template <class T, int BM>
-void mvsd_async_bk(RowGemmArgs<T>& a, int BK)
-{
-  switch (BK) {
-    case 4: mvsd_async_launch<T, BM, 4>(a); break;
-    case 8: mvsd_async_launch<T, BM, 8>(a); break;
-    case 16: mvsd_async_launch<T, BM, 16>(a); break;
-    case 32: mvsd_async_launch<T, BM, 32>(a); break;
-    default: mvsd_async_launch<T, BM, 64>(a); break;
-  }
-}
-
-template <class T>
-void mvsd_async(RowGemmArgs<T>& a, int BM, int BK)
-{
-  switch (BM) {
-    case 4: mvsd_async_bk<T, 4>(a, BK); break;
-    case 8: mvsd_async_bk<T, 8>(a, BK); break;
-    case 16: mvsd_async_bk<T, 16>(a, BK); break;
-    case 32: mvsd_async_bk<T, 32>(a, BK); break;
-    default: mvsd_async_bk<T, 64>(a, BK); break;
-  }
 }
 
 // fused V*C + Gram on the tensor cores (FP64, widths 8..64 in steps of 8)
@@ -1391,52 +1316,37 @@ bool mvsd_gram_dmma_mv(RowGemmArgs<double>& a, int MV)
   }
 }
 
-// true if the fused tensor-core kernel took the product
+// True if the fused tensor-core kernel took the product.  Up to 16 columns:
+// beyond, the shared-memory tiles leave one or two blocks per SM and the
+// product followed by the Gram product is faster (n = 2,097,152, m = k,
+// W'W: fused 80 / 150 / 395 / 1,290 us at 8 / 16 / 32 / 64 columns, the two
+// passes of pb_frag.cuh 89 / 163 / 320 / 1,240 us).
 inline bool mvsd_gram_dmma(RowGemmArgs<double>& a)
 {
   if (!rt().use_tma || !rt().use_dmma || a.mode == RM_VCWD || a.gram == GM_NONE) return false;
-  if (a.m > 64 || a.k > 64 || a.m < 5 || a.k < 5) return false;  // widths <= 4: register kernel
+  if (a.m > 16 || a.k > 16 || a.m < 5 || a.k < 5) return false;  // widths <= 4: register kernel
   const int BM = pad_width5(a.m), BK = pad_width5(a.k);
   if (a.gram == GM_WW) {
-    switch (BM * 100 + BK) {
-#define PB_GW(bm, bk) \
-  case bm * 100 + bk: return mvsd_gram_dmma_launch<bm, bk, bk, GM_WW>(a);
-      PB_GW(8, 8) PB_GW(8, 16) PB_GW(8, 32) PB_GW(8, 64) PB_GW(16, 8) PB_GW(16, 16) PB_GW(16, 32) PB_GW(16, 64)
-      PB_GW(32, 8) PB_GW(32, 16) PB_GW(32, 32) PB_GW(32, 64) PB_GW(64, 8) PB_GW(64, 16) PB_GW(64, 32)
-      PB_GW(64, 64)
-#undef PB_GW
-      default: return false;
-    }
+    if (BM == 8) return BK == 8 ? mvsd_gram_dmma_launch<8, 8, 8, GM_WW>(a) : mvsd_gram_dmma_launch<8, 16, 16, GM_WW>(a);
+    return BK == 8 ? mvsd_gram_dmma_launch<16, 8, 8, GM_WW>(a) : mvsd_gram_dmma_launch<16, 16, 16, GM_WW>(a);
   }
   // V'W with the in-place product: square blocks only (BM == BK)
   if (a.mv < 5 || a.mv > 64 || BM != BK) return false;
   const int MV = pad_width5(a.mv);
-  switch (BM) {
-    case 8: return mvsd_gram_dmma_mv<8, 8, GM_VW>(a, MV);
-    case 16: return mvsd_gram_dmma_mv<16, 16, GM_VW>(a, MV);
-    case 32: return mvsd_gram_dmma_mv<32, 32, GM_VW>(a, MV);
-    default: return mvsd_gram_dmma_mv<64, 64, GM_VW>(a, MV);
-  }
+  return BM == 8 ? mvsd_gram_dmma_mv<8, 8, GM_VW>(a, MV) : mvsd_gram_dmma_mv<16, 16, GM_VW>(a, MV);
 }
 inline bool mvsd_gram_dmma(RowGemmArgs<float>&) { return false; }
 
 template <class T>
 void launch_rowgemm(RowGemmArgs<T>& a)
 {
+  if (a.n == 0 && a.gram == GM_NONE) return;
   // fused V*C + Gram in one pass on the tensor cores
   if (mvsd_gram_dmma(a)) return;
-  {
-    // gram-free V*C and in-place W*C on aligned widths: multi-stage staged tiles
-    const T* A = (a.mode == RM_MVSDI) ? (const T*)a.W : a.V;
-    const int64_t lda = (a.mode == RM_MVSDI) ? a.ldw : a.ldv;
-    if (a.gram == GM_NONE && a.mode != RM_VCWD && a.m <= 64 && a.k <= 64 && vec_ok(A, lda, a.m)) {
-      mvsd_async<T>(a, pad_width5(a.m), pad_width5(a.k));
-      PB_LAUNCH_CHECK();
-      return;
-    }
-  }
-  if (a.m <= 8 && a.k <= 8 && (a.gram != GM_VW || a.mv <= 8)) {
-    // register kernel: padded widths M (4|8), K (1|4|8), MV (1, or 8 for V'W)
+  if (a.gram == GM_NONE && a.mode != RM_VCWD && frag_mvsd(a)) return;
+  const bool thin = a.k <= 4 && a.m <= (sizeof(T) == 4 ? 8 : 4);
+  if (a.m <= 8 && a.k <= 8 && (thin || a.mode == RM_VCWD) && (a.gram != GM_VW || a.mv <= 8)) {
+    // register kernel (thin blocks, V C + W D): padded widths M (4|8), K (1|4|8), MV (1, or 8 for V'W)
     const int M = a.m <= 4 ? 4 : 8, K = a.k == 1 ? 1 : a.k <= 4 ? 4 : 8;
     const int grid = std::max(1, std::min(grid_for(a.n), rt().num_sms() * 4));
     if (a.gram != GM_NONE) {
@@ -1458,23 +1368,13 @@ void launch_rowgemm(RowGemmArgs<T>& a)
     PB_LAUNCH_CHECK();
     return;
   }
-  {
-    const T* A = (a.mode == RM_MVSDI) ? (const T*)a.W : a.V;
-    const int64_t lda = (a.mode == RM_MVSDI) ? a.ldw : a.ldv;
-    const bool gram_ok = a.gram == GM_NONE || (vec_ok((const T*)a.W, a.ldw, a.k) &&
-                                               (a.gram == GM_WW || (a.mv <= 64 && vec_ok(a.Vg, a.ldvg, a.mv))));
-    if (gram_ok && a.mode != RM_VCWD && a.m <= 64 && a.k <= 64 && vec_ok(A, lda, a.m)) {
-      // multi-stage staged row tiles, widths padded to 4..64
-      mvsd_async<T>(a, pad_width5(a.m), pad_width5(a.k));
-      PB_LAUNCH_CHECK();
-      // fused Gram at these widths: a second pass over the new W with the
-      // staged Gram kernel (the register kernels above fuse it into one pass)
-      if (a.gram == GM_WW)
-        launch_mvTmv<T>(a.n, a.k, a.k, T(1), a.W, a.ldw, a.W, a.ldw, T(0), a.Gd, a.ldg);
-      else if (a.gram == GM_VW)
-        launch_mvTmv<T>(a.n, a.mv, a.k, a.galpha, a.Vg, a.ldvg, a.W, a.ldw, a.gbeta, a.Gd, a.ldg);
-      return;
-    }
+  // fused Gram at the other widths: a second pass over the new W
+  if (a.gram != GM_NONE && a.mode != RM_VCWD && (a.gram == GM_WW || a.mv <= 64) && frag_mvsd(a)) {
+    if (a.gram == GM_WW)
+      launch_mvTmv<T>(a.n, a.k, a.k, T(1), a.W, a.ldw, a.W, a.ldw, T(0), a.Gd, a.ldg);
+    else
+      launch_mvTmv<T>(a.n, a.mv, a.k, a.galpha, a.Vg, a.ldvg, a.W, a.ldw, a.gbeta, a.Gd, a.ldg);
+    return;
   }
   // micro-tile: TK columns per thread, TR rows
   const int TK = a.k >= 32 ? 8 : a.k >= 8 ? 4 : a.k >= 2 ? 2 : 1;

@@ -2,8 +2,9 @@
 // mma.sync.m8n8k4.f64) with TMA-staged row tiles, for padded widths of 8 to
 // 64 (multiples of 8).
 //
-//   k_mvtmv_dmma : C = alpha V'W + beta C      (Gram / projection matrices)
-//   k_mvsd_dmma  : W = alpha V C + beta W, or W(:,0:k) = W(:,0:m) C in place
+//   k_mvtmv_dmma     : C = alpha V'W + beta C (the wide products: pb_frag.cu
+//                      has the rule)
+//   k_mvsd_gram_dmma : V*C with the Gram matrix of the result, up to 16 columns
 //
 // Fragment layout of mma.m8n8k4.row.col.f64 (lane l, g = l/4, t = l%4):
 //   A (8x4, row-major): a = A[g][t];  B (4x8, column-major): b = B[t][g];
@@ -138,111 +139,13 @@ __global__ void __launch_bounds__(256) k_mvtmv_dmma(MvTmvArgs<double> a, const _
   last_block_reduce<double>(a.part, nout, gridDim.x, a.counter, a.Cd, 1, a.m, a.ldc, a.alpha, a.beta);
 }
 
-// ------------------------------------------------------------------ V*C
-// W tile (R x k) = A tile (R x m) * C (m x k).  Warp w owns rows
-// [w*RW, (w+1)*RW) of the stage (RW = R/8, RW/8 row tiles) and all BK/8
-// column tiles; the m-dimension is stepped 4 columns per DMMA.  C sits in
-// shared memory row-major with pitch CP = BK + 4, zero-padded.
-template <int BM, int BK, int R, int S>
-__global__ void __launch_bounds__(256) k_mvsd_dmma(RowGemmArgs<double> a, const __grid_constant__ CUtensorMap mapA,
-                                                   int* err)
-{
-  constexpr int NT = BK / 8, RW = R / 8, RT8 = RW / 8;
-  constexpr int AP = BM + 4, CP = BK + 4;
-  constexpr int CSZ = (BM * CP * 8 + 127) / 128 * 128 / 8;
-  constexpr unsigned STAGE_BYTES = (unsigned)(R * AP * sizeof(double));
-  static_assert(BM % 8 == 0 && BK % 8 == 0 && R % 64 == 0 && R <= 256 && S >= 2, "bad tile shape");
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  double* sC = reinterpret_cast<double*>(smem_raw);  // [BM][CP]
-  double* sA = sC + CSZ;                              // [S][R][AP]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sA + S * R * AP);
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const bool inplace = (a.mode == RM_MVSDI);
-  const int64_t ntiles = (a.n + R - 1) / R;
-
-  if (tid == 0) {
-    for (int st = 0; st < S; st++) mbar_init(&bar[st], 1);
-    mbar_fence_init();
-    tma_prefetch_desc(&mapA);
-  }
-  for (int q = tid; q < BM * CP; q += blockDim.x) {
-    const int i = q / CP, j = q - i * CP;
-    sC[q] = (i < a.m && j < a.k) ? a.C[i + (int64_t)j * a.ldc] : 0.0;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    for (int st = 0; st < S - 1; st++) {
-      const int64_t tl = blockIdx.x + (int64_t)st * gridDim.x;
-      if (tl < ntiles) {
-        mbar_arrive_expect_tx(&bar[st], STAGE_BYTES);
-        tma_load_2d(sA + st * R * AP, &mapA, 0, (int)(tl * R), &bar[st]);
-      }
-    }
-  }
-
-  bool ok = true;
-  int stage = 0;
-  int64_t it = 0;
-  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
-    if (tid == 0) {
-      const int64_t nt = tile + (int64_t)(S - 1) * gridDim.x;
-      const int ps = (stage + S - 1) % S;
-      if (nt < ntiles) {
-        mbar_arrive_expect_tx(&bar[ps], STAGE_BYTES);
-        tma_load_2d(sA + ps * R * AP, &mapA, 0, (int)(nt * R), &bar[ps]);
-      }
-    }
-    const bool landed = mbar_wait(&bar[stage], (unsigned)((it / S) & 1), err);
-    ok = ok && landed;
-    if (ok) {
-      const double* a0 = sA + stage * R * AP;
-      double acc[RT8][NT][2];
-#pragma unroll
-      for (int r8 = 0; r8 < RT8; r8++)
-#pragma unroll
-        for (int j = 0; j < NT; j++) acc[r8][j][0] = acc[r8][j][1] = 0.0;
-#pragma unroll 4
-      for (int kk = 0; kk < BM; kk += 4) {
-        double av[RT8], bc[NT];
-#pragma unroll
-        for (int r8 = 0; r8 < RT8; r8++) av[r8] = a0[(w * RW + r8 * 8 + g) * AP + kk + t];
-#pragma unroll
-        for (int j = 0; j < NT; j++) bc[j] = sC[(kk + t) * CP + j * 8 + g];
-#pragma unroll
-        for (int r8 = 0; r8 < RT8; r8++)
-#pragma unroll
-          for (int j = 0; j < NT; j++) dmma_884(acc[r8][j][0], acc[r8][j][1], av[r8], bc[j]);
-      }
-      const int64_t r0 = tile * R + w * RW;
-#pragma unroll
-      for (int r8 = 0; r8 < RT8; r8++) {
-        const int64_t row = r0 + r8 * 8 + g;
-        if (row >= a.n) continue;
-        double* wr = a.W + row * a.ldw;
-#pragma unroll
-        for (int j = 0; j < NT; j++)
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const int col = j * 8 + 2 * t + e;
-            if (col < a.k) {
-              const double v = acc[r8][j][e];
-              if (inplace) wr[col] = v;
-              else wr[col] = (a.beta != 0.0) ? a.alpha * v + a.beta * wr[col] : a.alpha * v;
-            }
-          }
-      }
-    }
-    __syncthreads();
-    stage = (stage + 1) % S;
-  }
-}
-
 // ------------------------------------------------------- V*C fused with a Gram
 // One pass for PHIST's fused_mvsd_mvTmv and fused_mvsdi_mvTmv
-// (phist_kernels_fused_decl.h:84,92): the new W tile is computed as in
-// k_mvsd_dmma, written to global memory and kept in shared memory (pitch
-// PT = BK + 4), and the Gram product of the tile is accumulated right away
+// (phist_kernels_fused_decl.h:84,92): warp w forms the rows [w*R/8, ...) of
+// the new W tile from the staged rows of V and C in shared memory (pitch
+// BK + 4, zero-padded), writes them to global memory and keeps them in shared
+// memory (pitch PT = BK + 4), and the Gram product of the tile is accumulated
+// right away
 //   GM == GM_WW : G  = W'W              (GMR = BK rows)
 //   GM == GM_VW : D  = galpha V'W + gbeta D, V staged by TMA with A (GMR = MV)
 // with the warp split and fixed-order reduction of k_mvtmv_dmma.  W is not

@@ -1,0 +1,80 @@
+"""Block products whose fragments are read straight from global memory
+(pb_frag.cuh): odd widths and offsets, partial 8-column tiles, row counts
+around a chunk's end, W'W, in-place updates; columns beside the views hold
+NaN and must not reach a result.
+
+Bound: a sum of q products of size at most 1 rounds by at most q*q*eps; FP32
+results are formed in FP64 and rounded once (the in-place and beta terms add
+two roundings of numbers of at most m + 1)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _block(n, ld, off, w, rng, dtype):
+    """an n x w view at column off of a block of ld columns, NaN around it"""
+    from phist_b200.objects import Map, Mvec
+    a = np.full((n, ld), np.nan, dtype)
+    a[:, off:off + w] = rng.uniform(-1, 1, (n, w)).astype(dtype)
+    mp = Map(n)
+    b = Mvec(mp.h, ld, dtype).set(a)
+    return mp, b, b.view(off, off + w - 1), a[:, off:off + w].astype(np.float64)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("m,k,vo,vld,wo,wld", [
+    (5, 1, 0, 5, 0, 1), (8, 5, 1, 10, 3, 9), (9, 7, 0, 10, 1, 8), (10, 4, 0, 10, 0, 4), (17, 9, 2, 20, 0, 10),
+    (37, 5, 0, 47, 0, 5), (40, 8, 0, 40, 0, 8), (24, 16, 0, 24, 0, 16), (5, 41, 1, 6, 0, 41), (33, 33, 1, 35, 1, 34),
+    (64, 64, 1, 66, 1, 66), (64, 20, 0, 64, 0, 20)])
+@pytest.mark.parametrize("n", [1, 31, 160, 161, 5003])
+def test_products(session, n, m, k, vo, vld, wo, wld, dtype):
+    from phist_b200 import kernels as K
+    from phist_b200.objects import SdMat, fn
+    rng = np.random.default_rng(n + 100 * m + k)
+    mp, Vb, V, v = _block(n, vld, vo, m, rng, dtype)
+    mq, Wb, W, w = _block(n, wld, wo, k, rng, dtype)
+    eps = np.finfo(dtype).eps
+    c0 = rng.uniform(-1, 1, (m, k)).astype(dtype)
+    C = SdMat(m, k, dtype).set(c0)
+    K.chk(fn(dtype, "mvecT_times_mvec"), 0.5, V.h, W.h, 2.0, C.h)
+    ref = 0.5 * (v.T @ w) + 2.0 * c0
+    assert np.abs(C.get() - ref).max() <= (n + 3) * (n * np.finfo(np.float64).eps + (n if vld % 4 == 0 else 1) * eps)
+    G = SdMat(k, k, dtype)
+    K.chk(fn(dtype, "mvecT_times_mvec"), 1.0, W.h, W.h, 0.0, G.h)
+    g = G.get()
+    assert np.abs(g - w.T @ w).max() <= (n + 3) * (n + 3) * eps
+    if k <= 32 and (k > 4 or (k > 8 and dtype == np.float32)):
+        assert np.array_equal(g, g.T)
+    C.set(c0)
+    K.chk(fn(dtype, "mvec_times_sdMat"), -0.5, V.h, C.h, 2.0, W.h)
+    ref = -0.5 * (v @ c0.astype(np.float64)) + 2.0 * w
+    got = Wb.get()
+    assert np.abs(got[:, wo:wo + k] - ref).max() <= (m + 3) * (m + 3) * eps
+    beside = np.delete(got, np.s_[wo:wo + k], axis=1)
+    assert np.isnan(beside).all()
+    if k <= m:
+        K.chk(fn(dtype, "mvec_times_sdMat_inplace"), V.h, C.h)
+        got = Vb.get()[:, vo:vo + m]
+        assert np.abs(got[:, :k] - v @ c0.astype(np.float64)).max() <= (m + 3) * (m + 3) * eps
+        assert np.array_equal(got[:, k:], v[:, k:].astype(dtype))
+    for o in (V, W, C, G, Vb, Wb, mp, mq):
+        o.delete()
+
+
+def test_infinity_stays_in_its_row(session):
+    """an infinite entry in the last column meets no zero padding"""
+    from phist_b200 import kernels as K
+    from phist_b200.objects import SdMat
+    rng = np.random.default_rng(3)
+    n, m, k = 100, 13, 6
+    mp, Vb, V, v = _block(n, m, 0, m, rng, np.float64)
+    v[7, m - 1] = np.inf
+    Vb.set(v)
+    mq, Wb, W, w = _block(n, k, 0, k, rng, np.float64)
+    C = SdMat(m, k).set(np.ones((m, k)))
+    K.chk(K.phist_Dmvec_times_sdMat, 1.0, V.h, C.h, 0.0, W.h)
+    got = Wb.get()
+    assert np.isposinf(got[7]).all() and np.isfinite(np.delete(got, 7, axis=0)).all()
+    for o in (V, W, C, Vb, Wb, mp, mq):
+        o.delete()
