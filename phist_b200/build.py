@@ -27,7 +27,7 @@ LIBPATH = os.path.join(LIBDIR, LIBNAME)
 
 SOURCES = ["pb_runtime.cu", "pb_api_D.cu", "pb_api_S.cu", "pb_api_mixed.cu", "pb_matfuncs.cu",
            "pb_noalloc.cu", "pb_carpcg.cu", "pb_tune.cu",
-           "pb_gmres.cu", "pb_frag.cu"]
+           "pb_gmres_D.cu", "pb_gmres_S.cu", "pb_frag.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O3",
               "--expt-relaxed-constexpr", "-diag-suppress", "550,177"]

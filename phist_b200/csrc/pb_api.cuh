@@ -722,7 +722,7 @@ void launch_spmv_nv(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p, 
   if constexpr (NV >= 8 && NV <= 32) {
     // wide block vectors: X rows staged in shared memory by cp.async
     const bool staged = A->tune_staged[LG] >= 0 ? A->tune_staged[LG] != 0 : NV >= rt().spmv_staged_min_nvec;
-    if (fast && vec && !dots && !p.u && staged) {
+    if (fast && vec && !dots && !p.u && !p.cscale && staged) {
       const size_t smem = StagedSmem<T, NV>::bytes;
       const int bps = std::max(1, std::min(8, (int)((200 * 1024) / smem)));
       const int sgrid = (int)std::min<int64_t>(A->nchunks > 0 ? A->nchunks : 1, (int64_t)rt().num_sms() * bps);
@@ -903,10 +903,11 @@ bool spmv_gram_fused(T alpha, const SparseMat<T>* A, const Mvec<T>* V, T beta, M
   return true;
 }
 
-// general entry: tiles of <= 32 columns; dots returned to host arrays
+// general entry: tiles of <= 32 columns; dots returned to host arrays;
+// cscale: device factors on alpha per column (beta = 0)
 template <class T>
 void spmv_general(T alpha, const SparseMat<T>* A, const T* shifts, const Mvec<T>* X, T beta,
-                  Mvec<T>* Y, T* WdotW, T* VdotW, T gamma, T delta, Mvec<T>* U)
+                  Mvec<T>* Y, T* WdotW, T* VdotW, T gamma, T delta, Mvec<T>* U, const T* cscale = nullptr)
 {
   PB_REQUIRE(X->nvec == Y->nvec, PB_INVALID_INPUT, "X has %d columns, Y %d", X->nvec, Y->nvec);
   PB_REQUIRE(X->nrows == A->ncols && Y->nrows == A->nrows, PB_INVALID_INPUT,
@@ -968,6 +969,7 @@ void spmv_general(T alpha, const SparseMat<T>* A, const T* shifts, const Mvec<T>
     p.delta = delta;
     p.u = U ? U->d() : nullptr;
     p.ldu = U ? U->lda : 0;
+    p.cscale = cscale;
     if (shifts) {
       p.has_shift = 1;
       for (int j = 0; j < nv; j++) p.sh[j] = shifts[c0 + j];

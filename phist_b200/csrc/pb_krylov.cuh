@@ -1,0 +1,448 @@
+// pb_krylov.cuh -- the passes over the basis of the device GMRES and MINRES
+// (pb_gmres.cuh): all that happens between two SpMMVs, in one kernel body.
+//
+// The k systems are the k columns of every block: basis block V_i is n x k,
+// contiguous.  The new direction W is the storage of the next block and
+// stays unnormalised: v_i = F_i V_i with the factors F_i (one per system) on
+// the device; the SpMMV multiplies by F_j, dots and coefficients carry F_i,
+// so no pass is spent on scaling.
+//
+//   k_kry<MQ, MJ, UPD, DOTS> over the blocks V_0..V_{nb-1} it is given:
+//     UPD : W -= Q cq + sum_i V_i hv_i          (cq: nq x k, hv: nb x k)
+//     DOTS: Q'W (only without UPD) and V_i'W of every system
+//     always ||W||^2 (after the update)
+//
+// The last block to finish holds the sums and goes on with the small dense
+// work of the step (kry_epilogue): Lanczos or Gram-Schmidt coefficients, the
+// column of H, rotations, residual estimate, convergence test, F_{j+1}.  A
+// MINRES step is SpMMV + 2 launches, a GMRES step SpMMV + 3.
+//
+// A warp takes 32 rows at a time.  Q (row-major, any stride) meets W on the
+// FP64 tensor pipe with fragments straight from global memory as in
+// pb_frag.cuh; Q cq goes through a warp's own shared-memory tile into the
+// layout of the basis part, where lane = (row, system) so that every load of
+// V_i or W is one contiguous segment.  Bound by HBM, or for bases that fit it
+// by the L2.
+//
+// Sums: lanes, warps and blocks in fixed order, FP64 from the lane sums on.
+#pragma once
+#include "pb_frag.cuh"
+
+namespace pb {
+
+constexpr int KRY_MAXQ = 32;  // projection columns of one launch
+constexpr int KRY_MAXJ = 24;  // basis blocks of one launch
+constexpr int KRY_MAXC = 8;   // systems of one launch
+constexpr int KRY_MAXOUT = (KRY_MAXQ + KRY_MAXJ + 1) * KRY_MAXC;
+
+struct GmTol {
+  double v[32];
+};
+struct GmIndex {
+  int v[32];
+};
+
+// what the block holding the sums does
+enum KryKind {
+  KE_NONE = 0,    // nothing (the update alone)
+  KE_START,       // beta = ||W||, g = beta e_1, F_0
+  KE_LZ,          // Lanczos coefficients of step j
+  KE_GS,          // first Gram-Schmidt coefficients (blocks i0..), ||W|| before
+  KE_GS2,         // second coefficients; with last also the decision on a second pass
+  KE_STEP,        // rotations, residual estimate, convergence
+  KE_NORM         // finv = 1/||W||
+};
+
+// H(:, :, s) at H[(i*m + j)*k + s]; per-system arrays have stride k and are
+// indexed by the system number (c0 + the launch's column)
+template <class T>
+struct KryEpi {
+  int kind, last;             // last: last launch of a group of chunks (KE_GS2) / of systems (flags)
+  int c0, k, m, j, i0;
+  int lanczos, first;
+  double *H, *cs, *sn, *g, *bnorm;
+  double *h1, *h2;            // [i*k + s] coefficients of the two Gram-Schmidt passes
+  double *nrm0, *nf;          // ||W||^2 before the first pass; after the step
+  T *F;                       // [i*k + s]
+  T *cq, *hv, *hv2;           // coefficients for the update passes
+  T *finv;
+  int *conv, *jcount, *reorth;
+  double eps_abs;
+  GmTol tol;
+  volatile int* flags;        // mapped host memory: step, converged systems
+};
+
+template <class T>
+struct KryArgs {
+  int64_t n;
+  int k, kc, kp;              // row stride of W and V_i; systems here; kc rounded up to a power of two
+  int nq; const T* Q; int64_t ldq;
+  const T* V; int64_t vstep; int nb;   // blocks at V + i*vstep
+  const T* Win;               // NULL: W starts from zero
+  T* W;
+  const T* cq; const T* hv;
+  const int* skip;            // the kernel does nothing when *skip == 0
+  double* part; int gsz; unsigned int* counters;
+  KryEpi<T> e;
+  // KE_START: W = R(:, idx) (- W on a restart, converged systems zero)
+  const T* R; int64_t ldr; GmIndex idx; int restart;
+};
+
+__device__ __forceinline__ void kry_ldp(const double* p, bool ok, double& v)
+{
+  asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\nmov.f64 %0, 0d0000000000000000;\n@p ld.global.f64 %0, [%1];\n}\n"
+               : "=d"(v)
+               : "l"(p), "r"((int)ok));
+}
+__device__ __forceinline__ void kry_ldp(const float* p, bool ok, float& v)
+{
+  asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\nmov.f32 %0, 0f00000000;\n@p ld.global.f32 %0, [%1];\n}\n"
+               : "=f"(v)
+               : "l"(p), "r"((int)ok));
+}
+
+// Column j of every system's H is complete up to the new norm hn: apply the
+// earlier rotations, zero h(j+1, j) with a new one, test for convergence.
+// nrm: ||W||^2 per column of the launch; sm: shared scratch, 3*64*8 doubles.
+// A Lanczos column is zero above j-1, so only the rotations from j-2 on act.
+template <class T>
+__device__ __forceinline__ void kry_step(const KryEpi<T>& e, int kc, const double* nrm, double* sm)
+{
+  const int tid = threadIdx.x, j = e.j, k = e.k, m = e.m;
+  const int lo = e.lanczos ? max(0, j - 2) : 0;
+  double* sh = sm;
+  double* sc = sm + 64 * KRY_MAXC;
+  double* ss = sc + 64 * KRY_MAXC;
+  __syncthreads();
+  for (int q = tid; q < (j + 1 - lo) * kc; q += FRAG_BS) {
+    const int i = lo + q / kc, c = q % kc, s = e.c0 + c;
+    sh[i * kc + c] = __ldcg(&e.H[((int64_t)i * m + j) * k + s]);
+    if (i < j) {
+      sc[i * kc + c] = __ldcg(&e.cs[i * k + s]);
+      ss[i * kc + c] = __ldcg(&e.sn[i * k + s]);
+    }
+  }
+  __syncthreads();
+  if (tid < kc) {
+    const int c = tid, s = e.c0 + c;
+    const double n2 = fmax(nrm[c], 0.0), hn = sqrt(n2);
+    double a = sh[lo * kc + c];
+    for (int i = lo; i < j; i++) {
+      const double b = sh[(i + 1) * kc + c], rc = sc[i * kc + c], rs = ss[i * kc + c];
+      sh[i * kc + c] = rc * a + rs * b;
+      a = -rs * a + rc * b;
+    }
+    double co = 1.0, si = 0.0;
+    const double r = hypot(a, hn);
+    if (r > 0.0) {
+      co = a / r;
+      si = hn / r;
+    }
+    sh[j * kc + c] = r;
+    e.cs[j * k + s] = co;
+    e.sn[j * k + s] = si;
+    const double gj = e.g[j * k + s];
+    const double gn = -si * gj;
+    e.g[j * k + s] = co * gj;
+    e.g[(j + 1) * k + s] = gn;
+    if (!e.conv[s]) {
+      e.jcount[s] = j + 1;
+      const double res = fabs(gn);
+      if (res < e.eps_abs || (e.bnorm[s] > 0.0 && res / e.bnorm[s] < e.tol.v[s])) e.conv[s] = 1;
+    }
+    e.nf[s] = n2;
+    e.F[(j + 1) * k + s] = (hn > 0.0) ? (T)(1.0 / hn) : T(0);
+  }
+  __syncthreads();
+  for (int q = tid; q < (j + 1 - lo) * kc; q += FRAG_BS) {
+    const int i = lo + q / kc, c = q % kc;
+    e.H[((int64_t)i * m + j) * k + e.c0 + c] = sh[i * kc + c];
+  }
+  if (tid == 0 && e.last) {
+    int nconv = 0;
+    for (int s = 0; s < k; s++) nconv += e.conv[s] ? 1 : 0;
+    e.flags[1] = nconv;
+    __threadfence_system();
+    e.flags[0] = j;
+  }
+}
+
+// out: the sums in shared memory, [Q'W | V'W | ||W||^2] as nqo + nb + 1 rows
+// of kc; sm: further shared scratch
+template <class T>
+__device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int nbo, const double* out, double* sm)
+{
+  const KryEpi<T>& e = a.e;
+  const int tid = threadIdx.x, kc = a.kc, k = e.k, j = e.j, m = e.m;
+  const double* nrm = out + (nqo + nbo) * kc;
+  if (e.kind == KE_START) {
+    if (tid < kc) {
+      const int s = e.c0 + tid;
+      const double beta = sqrt(fmax(nrm[tid], 0.0));
+      if (e.first) {
+        e.bnorm[s] = beta;
+        e.conv[s] = (beta < e.eps_abs) ? 1 : 0;
+      }
+      e.jcount[s] = 0;
+      for (int i = 1; i <= m; i++) e.g[i * k + s] = 0.0;
+      e.g[s] = e.conv[s] ? 0.0 : beta;
+      e.F[s] = (beta > 0.0 && !e.conv[s]) ? (T)(1.0 / beta) : T(0);
+    }
+  } else if (e.kind == KE_LZ) {
+    for (int q = tid; q < nqo * kc; q += FRAG_BS) e.cq[(q / kc) * k + e.c0 + q % kc] = (T)out[q];
+    if (tid < kc) {
+      // alpha = v_j'w, beta = the previous step's norm; the update
+      // subtracts V_j (F_j alpha), then V_{j-1} (F_{j-1} beta)
+      const int s = e.c0 + tid;
+      const double alpha = (double)e.F[j * k + s] * out[nqo * kc + tid];
+      const double beta = j > 0 ? sqrt(e.nf[s]) : 0.0;
+      for (int i = 0; i + 1 < j; i++) e.H[((int64_t)i * m + j) * k + s] = 0.0;
+      if (j > 0) e.H[((int64_t)(j - 1) * m + j) * k + s] = beta;
+      e.H[((int64_t)j * m + j) * k + s] = alpha;
+      e.hv[s] = (T)((double)e.F[j * k + s] * alpha);
+      e.hv[k + s] = j > 0 ? (T)((double)e.F[(j - 1) * k + s] * beta) : T(0);
+    }
+  } else if (e.kind == KE_GS) {
+    for (int q = tid; q < nqo * kc; q += FRAG_BS) e.cq[(q / kc) * k + e.c0 + q % kc] = (T)out[q];
+    for (int q = tid; q < nbo * kc; q += FRAG_BS) {
+      const int p = (e.i0 + q / kc) * k + e.c0 + q % kc;
+      const double h = (double)e.F[p] * out[nqo * kc + q];
+      e.h1[p] = h;
+      e.hv[p] = (T)((double)e.F[p] * h);
+    }
+    if (tid < kc) e.nrm0[e.c0 + tid] = nrm[tid];
+  } else if (e.kind == KE_GS2) {
+    for (int q = tid; q < nbo * kc; q += FRAG_BS) {
+      const int p = (e.i0 + q / kc) * k + e.c0 + q % kc;
+      const double h = (double)e.F[p] * out[nqo * kc + q];
+      e.h2[p] = h;
+      e.hv2[p] = (T)((double)e.F[p] * h);
+    }
+    if (!e.last) return;
+    // a second subtraction where some norm fell below 1/sqrt(2) of its value
+    // before the pass ("twice is enough")
+    const int need = tid < kc && nrm[tid] < 0.5 * e.nrm0[e.c0 + tid];
+    __threadfence_block();
+    const int any = __syncthreads_or(need);
+    for (int q = tid; q < (j + 1) * kc; q += FRAG_BS) {
+      const int i = q / kc, s = e.c0 + q % kc;
+      e.H[((int64_t)i * m + j) * k + s] = __ldcg(&e.h1[i * k + s]) + (any ? __ldcg(&e.h2[i * k + s]) : 0.0);
+    }
+    if (tid == 0) *e.reorth = any;
+    __threadfence();
+    if (!any) kry_step<T>(e, kc, nrm, sm);
+  } else if (e.kind == KE_STEP) {
+    kry_step<T>(e, kc, nrm, sm);
+  } else if (e.kind == KE_NORM) {
+    if (tid < kc) {
+      const double nr = sqrt(fmax(nrm[tid], 0.0));
+      e.finv[e.c0 + tid] = nr > 0.0 ? (T)(1.0 / nr) : T(0);
+    }
+  }
+}
+
+constexpr int KRY_RED = FRAG_NW * KRY_MAXOUT;
+constexpr int KRY_TILE = 32 * 9;                                // a warp's Q cq tile
+constexpr int KRY_SC = FRAG_NW * KRY_TILE;                      // coefficients of Q, fragment order
+constexpr int KRY_SH = KRY_SC + 2 * (KRY_MAXQ / 8) * 32;        // coefficients of V
+static_assert(KRY_SH + KRY_MAXJ * KRY_MAXC <= KRY_RED, "tiles fit the reduction buffer");
+static_assert(KRY_MAXOUT + 3 * 64 * KRY_MAXC <= KRY_RED, "epilogue scratch fits the reduction buffer");
+
+// after the row loop: the lanes' sums to the block's, the blocks' to the
+// totals, and the epilogue in the block that holds them
+template <class T, int MQ, int MJ>
+__device__ __forceinline__ void kry_finish(const KryArgs<T>& a, int nqo, int nbo, double (&qa)[MQ > 0 ? MQ : 1][2],
+                                           T (&va)[MJ], T na, double* sm)
+{
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int kc = a.kc, kp = a.kp, s = lane & (kp - 1);
+  const int nout = (nqo + nbo + 1) * kc;
+  double nd = (double)na, vd[MJ];
+#pragma unroll
+  for (int i = 0; i < MJ; i++) vd[i] = i < nbo ? (double)va[i] : 0.0;
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) {
+    if (off < kp) break;
+#pragma unroll
+    for (int i = 0; i < MJ; i++)
+      if (i < nbo) vd[i] += __shfl_xor_sync(0xffffffffu, vd[i], off);
+    nd += __shfl_xor_sync(0xffffffffu, nd, off);
+  }
+  __syncthreads();  // tiles and coefficients no longer read
+  double* red = sm + w * KRY_MAXOUT;
+  if (MQ > 0 && nqo > 0) {
+#pragma unroll
+    for (int i = 0; i < MQ; i++)
+#pragma unroll
+      for (int e = 0; e < 2; e++)
+        if (i * 8 + g < nqo && 2 * t + e < kc) red[(i * 8 + g) * kc + 2 * t + e] = qa[i][e];
+  }
+  if (lane < kp && s < kc) {
+#pragma unroll
+    for (int i = 0; i < MJ; i++)
+      if (i < nbo) red[(nqo + i) * kc + s] = vd[i];
+    red[(nqo + nbo) * kc + s] = nd;
+  }
+  __syncthreads();
+  double tot[2];
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int o = tid + q * FRAG_BS;
+    tot[q] = 0.0;
+    if (o < nout) {
+#pragma unroll
+      for (int b = 0; b < FRAG_NW; b++) tot[q] += sm[b * KRY_MAXOUT + o];
+      a.part[(int64_t)blockIdx.x * nout + o] = tot[q];
+    }
+  }
+  if (!frag_tree_sum<2>(a.part, nout, a.gsz, a.counters, tot)) return;
+#pragma unroll
+  for (int q = 0; q < 2; q++)
+    if (tid + q * FRAG_BS < nout) sm[tid + q * FRAG_BS] = tot[q];
+  __syncthreads();
+  kry_epilogue<T>(a, nqo, nbo, sm, sm + KRY_MAXOUT);
+}
+
+template <class T, int MQ, int MJ, bool UPD, bool DOTS>
+__global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryArgs<T> a)
+{
+  if (a.skip && *a.skip == 0) return;
+  constexpr int UB = MJ <= 2 ? 4 : MJ <= 8 ? 2 : 1;  // packed steps of loads in flight
+  constexpr int MQ1 = MQ > 0 ? MQ : 1;
+  constexpr int RTB = MQ <= 2 ? 4 : 2;               // row tiles of Q in flight
+  __shared__ double sm[KRY_RED];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int kc = a.kc, kp = a.kp, k = a.k, nb = a.nb, nq = a.nq;
+  const int s = lane & (kp - 1), rr = lane / kp, rs = 32 / kp;
+  const bool mine = s < kc;
+  double* sC = sm + KRY_SC;
+  T* sH = reinterpret_cast<T*>(sm + KRY_SH);
+  double* tile = sm + w * KRY_TILE;
+  if (UPD) {
+    for (int q = tid; q < 2 * MQ * 32; q += FRAG_BS) {
+      const int l = q & 31, i = 4 * (q >> 5) + (l & 3), c = l >> 2;
+      sC[q] = (i < nq && c < kc) ? (double)a.cq[i * k + c] : 0.0;
+    }
+    for (int q = tid; q < MJ * KRY_MAXC; q += FRAG_BS) {
+      const int i = q / KRY_MAXC, c = q % KRY_MAXC;
+      sH[q] = (i < nb && c < kc) ? a.hv[i * k + c] : T(0);
+    }
+    __syncthreads();
+  }
+  double qa[MQ1][2];
+  T va[MJ], na = T(0);
+#pragma unroll
+  for (int i = 0; i < MQ1; i++) qa[i][0] = qa[i][1] = 0.0;
+#pragma unroll
+  for (int i = 0; i < MJ; i++) va[i] = T(0);
+  const int64_t nch = (a.n + 31) / 32, GW = gridDim.x * (int64_t)FRAG_NW;
+  for (int64_t ch = blockIdx.x * (int64_t)FRAG_NW + w; ch < nch; ch += GW) {
+    const int64_t r0 = ch * 32;
+    if (MQ > 0 && !UPD && DOTS) {
+      // Q'W: 4-row steps, half of the chunk's loads at a time
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        T qv[4][MQ1], wv[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int64_t row = r0 + 16 * h + 4 * u + t;
+          const bool ok = row < a.n;
+          const T* pq = a.Q + (ok ? row : 0) * a.ldq;
+#pragma unroll
+          for (int i = 0; i < MQ; i++) kry_ldp(pq + min(8 * i + g, nq - 1), ok, qv[u][i]);
+          kry_ldp(a.W + (ok ? row : 0) * k + min(g, kc - 1), ok, wv[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+          for (int i = 0; i < MQ; i++) dmma_884(qa[i][0], qa[i][1], (double)qv[u][i], (double)wv[u]);
+      }
+    }
+    if (MQ > 0 && UPD) {
+      // Q cq of the chunk's rows, 8 rows per tensor tile, into the warp's tile
+#pragma unroll
+      for (int h = 0; h < 4; h += RTB) {
+        T qv[RTB][2 * MQ1];
+#pragma unroll
+        for (int u = 0; u < RTB; u++) {
+          const int64_t row = r0 + 8 * (h + u) + g;
+          const T* pq = a.Q + (row < a.n ? row : 0) * a.ldq;
+#pragma unroll
+          for (int i = 0; i < 2 * MQ; i++) kry_ldp(pq + min(4 * i + t, nq - 1), row < a.n && 4 * i + t < nq, qv[u][i]);
+        }
+#pragma unroll
+        for (int u = 0; u < RTB; u++) {
+          double d0 = 0.0, d1 = 0.0;
+#pragma unroll
+          for (int i = 0; i < 2 * MQ; i++) dmma_884(d0, d1, (double)qv[u][i], sC[i * 32 + lane]);
+          tile[(8 * (h + u) + g) * 9 + 2 * t] = d0;
+          tile[(8 * (h + u) + g) * 9 + 2 * t + 1] = d1;
+        }
+      }
+      __syncwarp();
+    }
+    // lane = (row, system)
+    for (int u0 = 0; u0 < kp; u0 += UB) {
+      T v[UB][MJ], wv[UB];
+#pragma unroll
+      for (int u = 0; u < UB; u++) {
+        const int64_t row = r0 + (int64_t)(u0 + u) * rs + rr;
+        const bool ok = mine && u0 + u < kp && row < a.n;
+        const int64_t at = ok ? row * k + s : 0;
+        kry_ldp(a.Win + at, ok && a.Win, wv[u]);
+#pragma unroll
+        for (int i = 0; i < MJ; i++) kry_ldp(a.V + i * a.vstep + at, ok && i < nb, v[u][i]);
+      }
+#pragma unroll
+      for (int u = 0; u < UB; u++) {
+        const int lr = (u0 + u) * rs + rr;
+        const int64_t row = r0 + lr;
+        const bool ok = mine && u0 + u < kp && row < a.n;
+        T x = wv[u];
+        if (UPD) {
+          if (MQ > 0 && ok) x -= (T)tile[lr * 9 + s];
+#pragma unroll
+          for (int i = 0; i < MJ; i++) x -= v[u][i] * sH[i * KRY_MAXC + s];
+          if (ok) a.W[row * k + s] = x;
+          else x = T(0);
+        }
+        if (DOTS) {
+#pragma unroll
+          for (int i = 0; i < MJ; i++) va[i] += v[u][i] * x;
+        }
+        na += x * x;
+      }
+    }
+    if (MQ > 0 && UPD) __syncwarp();
+  }
+  kry_finish<T, MQ, MJ>(a, (DOTS && !UPD && MQ > 0) ? nq : 0, DOTS ? nb : 0, qa, va, na, sm);
+}
+
+// W = R(:, idx) at the start, W = R(:, idx) - W (0 for converged systems) on
+// a restart, and the norms
+template <class T>
+__global__ void __launch_bounds__(FRAG_BS) k_kry_start(const __grid_constant__ KryArgs<T> a)
+{
+  __shared__ double sm[KRY_RED];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int kc = a.kc, kp = a.kp, k = a.k;
+  const int s = lane & (kp - 1), rs = 32 / kp;
+  T na = T(0);
+  if (s < kc) {
+    const int col = a.idx.v[a.e.c0 + s];
+    const bool zero = a.restart && a.e.conv[a.e.c0 + s];
+    const int64_t step = gridDim.x * (int64_t)FRAG_NW * rs;
+#pragma unroll 4
+    for (int64_t row = (blockIdx.x * (int64_t)FRAG_NW + w) * rs + lane / kp; row < a.n; row += step) {
+      T x = a.R[row * a.ldr + col];
+      if (a.restart) x = zero ? T(0) : x - a.W[row * k + s];
+      a.W[row * k + s] = x;
+      na += x * x;
+    }
+  }
+  double qa[1][2];
+  T va[1] = {T(0)};
+  kry_finish<T, 0, 1>(a, 0, 0, qa, va, na, sm);
+}
+
+}  // namespace pb

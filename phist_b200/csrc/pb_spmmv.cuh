@@ -38,6 +38,7 @@ struct SpmvArgs {
   T alpha, beta;
   int has_shift;                 // shifts sh[0..nvec) present
   T sh[32];                      // per-column shifts of this column tile
+  const T* __restrict__ cscale;  // device factors on alpha per column (nullptr: 1)
   const T* __restrict__ x;
   int64_t ldx;
   T* y;
@@ -202,6 +203,17 @@ __device__ __forceinline__ int spmv_col(int s, int v, int w)
   return VW * (s + v * TPR) + w;
 }
 
+// the device factors on the columns of a product (beta == 0): VW columns from
+// column c of the launch
+template <int VW, class T, class AT>
+__device__ __forceinline__ void spmv_cscale(const SpmvArgs<T>& p, int c, AT* acc)
+{
+  if (p.cscale) {
+#pragma unroll
+    for (int w = 0; w < VW; w++) acc[w] *= AT(__ldg(p.cscale + p.col0 + c + w));
+  }
+}
+
 constexpr int SPMV_BS = 256;
 
 // KMAX > 0: every chunk of the matrix is at most KMAX entries long (fully
@@ -340,6 +352,7 @@ k_sell_spmmv(SellDev<T> A, SpmvArgs<T> p)
     for (int v = 0; v < NVV; v++) {
       const int c = spmv_col<TPR, VW>(s, v, 0);
       if (!(VEC || c < nv)) continue;
+      spmv_cscale<VW>(p, c, &acc[v * VW]);
       T yv[VW];
       if (p.beta != T(0)) {
         Vec<T, VW>::ld_plain(yr + c, yv);

@@ -379,6 +379,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
 #pragma unroll
         for (int v = 0; v < NVV; v++) {
           const int c = spmv_col<TPR, VW>(s, v, 0);
+          spmv_cscale<VW>(p, c, &acc[v * VW]);
           T yv[VW];
           if (p.beta != T(0)) {
             Vec<T, VW>::ld_plain(yr + c, yv);
