@@ -770,6 +770,24 @@ void launch_spmv_nv(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p, 
     PB_LAUNCH_CHECK();
     return;
   }
+  if (unroll && A->C == 32 && !fast && !dots && !p.u && rt().spmv_pf && (vec || (NV == 1 && p.nvec == 1)) &&
+      TPR == (NV <= 4 ? 1 : NV == 8 ? 2 : 4)) {
+    constexpr int NT = TPR == 1 ? 128 : 256;
+    constexpr int V32 = 32 / (int)sizeof(T);
+    const bool v256 = (NV / TPR) * (int)sizeof(T) >= 32 && rt().spmv_v256 && ((uintptr_t)(p.x + p.col0) & 31u) == 0 &&
+                      ((uintptr_t)(p.y + p.col0) & 31u) == 0 && p.ldx % V32 == 0 && p.ldy % V32 == 0;
+    const int lgrid = (int)ceil_div(npad > 0 ? npad : 1, NT / TPR);
+    if constexpr ((NV / TPR) * sizeof(T) >= 32) {
+      if (v256) {
+        k_sell_spmmv_long<T, NV, TPR, NT, 32, false><<<lgrid, NT, 0, stream()>>>(S, p);
+        PB_LAUNCH_CHECK();
+        return;
+      }
+    }
+    k_sell_spmmv_long<T, NV, TPR, NT, 16, false><<<lgrid, NT, 0, stream()>>>(S, p);
+    PB_LAUNCH_CHECK();
+    return;
+  }
 #define PB_SPMV(VECv, KMAXv, CCv)                                                         \
   if (dots)                                                                             \
     k_sell_spmmv<T, NV, TPR, VECv, KMAXv, CCv, true><<<grid, SPMV_BS, 0, stream()>>>(S, p); \
@@ -782,6 +800,54 @@ void launch_spmv_nv(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p, 
   }
 #undef PB_SPMV
   PB_LAUNCH_CHECK();
+}
+
+// Column split of the any-width kernels: vectors of VW columns, TPR threads a
+// row, UPT vectors a thread (at most 8 columns in registers per thread)
+template <class T, int VW, int TPR, int UPT>
+void launch_spmv_any(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p)
+{
+  constexpr int NV = VW * TPR * UPT, NT = TPR == 1 ? 128 : 256, RPB = NT / TPR, VB = VW * (int)sizeof(T);
+  if (A->max_row_len <= 8) {
+    auto kern = k_sell_spmmv_pf_any<T, NV, TPR, NT, VB>;
+    static std::atomic<int> occ{0};
+    if (occ.load() == 0) {
+      int o = 0;
+      PB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, NT, 0));
+      occ.store(std::max(1, o));
+    }
+    const int64_t ntiles = ceil_div(A->nchunks, RPB / 32);
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rt().num_sms() * occ.load()));
+    kern<<<grid, NT, 0, stream()>>>(S, p);
+  } else {
+    k_sell_spmmv_long<T, NV, TPR, NT, VB, true><<<(int)ceil_div(A->nchunks * 32, RPB), NT, 0, stream()>>>(S, p);
+  }
+  PB_LAUNCH_CHECK();
+}
+
+template <class T>
+void spmv_any(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p)
+{
+  const int vw = 2 * (int)sizeof(T);
+  const bool pairs = p.nvec % 2 == 0 && p.ldx % 2 == 0 && p.ldy % 2 == 0 && (uintptr_t)(p.x + p.col0) % vw == 0 &&
+                     (uintptr_t)(p.y + p.col0) % vw == 0;
+#define PB_ANY(VWv, TPRv, UPTv) \
+  case UPTv: launch_spmv_any<T, VWv, TPRv, UPTv>(A, S, p); return;
+  if (pairs) {
+    const int u = p.nvec / 2;
+    if (u <= 4) switch (u) { PB_ANY(2, 1, 1) PB_ANY(2, 1, 2) PB_ANY(2, 1, 3) PB_ANY(2, 1, 4) }
+    else if (u <= 8) switch ((u + 1) / 2) { PB_ANY(2, 2, 3) PB_ANY(2, 2, 4) }
+    else switch ((u + 3) / 4) { PB_ANY(2, 4, 3) PB_ANY(2, 4, 4) }
+  } else {
+    const int u = p.nvec;
+    if (u <= 8) switch (u) {
+        PB_ANY(1, 1, 1) PB_ANY(1, 1, 2) PB_ANY(1, 1, 3) PB_ANY(1, 1, 4) PB_ANY(1, 1, 5) PB_ANY(1, 1, 6)
+        PB_ANY(1, 1, 7) PB_ANY(1, 1, 8)
+      }
+    else if (u <= 16) switch ((u + 1) / 2) { PB_ANY(1, 2, 5) PB_ANY(1, 2, 6) PB_ANY(1, 2, 7) PB_ANY(1, 2, 8) }
+    else switch ((u + 3) / 4) { PB_ANY(1, 4, 5) PB_ANY(1, 4, 6) PB_ANY(1, 4, 7) PB_ANY(1, 4, 8) }
+  }
+#undef PB_ANY
 }
 
 template <class T>
@@ -808,6 +874,13 @@ void spmv_tile(const SparseMat<T>* A, SpmvArgs<T>& p, int nv)
     if (sizeof(T) == 4 && NV == 2) vec = false;
   }
   const int tpr = A->tune_tpr[lg] > 0 ? A->tune_tpr[lg] : rt().spmv_tpr[lg];
+  // widths that are no power of two, rows that start on no vector boundary
+  const bool unroll = A->tune_unroll[lg] >= 0 ? A->tune_unroll[lg] != 0 : rt().spmv_unroll;
+  const bool plain = A->C == 32 && rt().spmv_pf && unroll && !p.want_wdw && !p.want_vdw && !p.u;
+  if (plain && !vec && NV > 1) {
+    spmv_any<T>(A, S, p);
+    return;
+  }
   switch (NV) {
     case 1: launch_spmv_nv<T, 1, 1>(A, S, p, false); break;
     case 2: launch_spmv_nv<T, 2, 1>(A, S, p, vec); break;

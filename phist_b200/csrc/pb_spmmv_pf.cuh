@@ -213,7 +213,10 @@ struct GramPick<double, NV, NT, RPB> {
 
 // VB: bytes per vector load and store of an X or Y row segment (16, or 32
 // with the 256-bit forms when rows start on 32-byte boundaries)
-template <class T, int NV, int TPR, int NT, bool GRAM, int VB>
+// ANY: p.nvec <= NV columns of any alignment that VB allows; a thread's
+// vectors past the last column read that column again (no predicate between
+// the gathers) and are not stored
+template <class T, int NV, int TPR, int NT, bool GRAM, int VB, bool ANY>
 __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArgs<T>& p)
 {
   constexpr int KMAX = 8, CC = 32;
@@ -226,6 +229,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
   constexpr int EPT = NCH * KMAX * CC; // entries per tile at most
   static_assert(RPB % CC == 0, "a tile is a whole number of chunks");
   typedef typename Acc<T>::type AT;
+  static_assert(VPT % VW == 0 && !(ANY && GRAM), "bad column split");
   __shared__ __align__(16) T sval[2][EPT];
   __shared__ __align__(16) int scol[2][EPT];
   __shared__ int64_t smeta[3][NCH + 1];  // chunk pointers of three tiles
@@ -244,6 +248,11 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
   const int64_t ntiles = (nch + NCH - 1) / NCH;
   const int64_t G = gridDim.x;
   const T* __restrict__ x = p.x + p.col0;
+  // first column of this thread's vector v, for loads
+  auto lcol = [&](int v) {
+    const int c = spmv_col<TPR, VW>(s, v, 0);
+    return ANY ? min(c, p.nvec - VW) : c;
+  };
 
   // chunk pointer tid (0..NCH) of tile t, clamped to the end of the arrays
   auto meta_load = [&](int64_t t) -> int64_t {
@@ -331,14 +340,11 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
         if (i >= 0 && p.has_shift) {
           T xs[VPT];
 #pragma unroll
-          for (int v = 0; v < NVV; v++) Vec<T, VW>::ld(x + i * p.ldx + spmv_col<TPR, VW>(s, v, 0), &xs[v * VW]);
+          for (int v = 0; v < NVV; v++) Vec<T, VW>::ld(x + i * p.ldx + lcol(v), &xs[v * VW]);
 #pragma unroll
           for (int v = 0; v < NVV; v++)
 #pragma unroll
-            for (int w = 0; w < VW; w++) {
-              const int c = spmv_col<TPR, VW>(s, v, w);
-              acc[v * VW + w] = AT(p.sh[c]) * AT(xs[v * VW + w]);
-            }
+            for (int w = 0; w < VW; w++) acc[v * VW + w] = AT(p.sh[lcol(v) + w]) * AT(xs[v * VW + w]);
         }
       }
       const int lc = lr / CC, l = lr % CC;
@@ -363,7 +369,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
       for (int k = 0; k < KMAX; k++) {
         const T* xr = x + (int64_t)cv[k] * p.ldx;
 #pragma unroll
-        for (int v = 0; v < NVV; v++) Vec<T, VW>::ld_ordered(xr + spmv_col<TPR, VW>(s, v, 0), &xv[k][v * VW]);
+        for (int v = 0; v < NVV; v++) Vec<T, VW>::ld_ordered(xr + lcol(v), &xv[k][v * VW]);
       }
 #pragma unroll
       for (int k = 0; k < KMAX; k++)
@@ -379,6 +385,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
 #pragma unroll
         for (int v = 0; v < NVV; v++) {
           const int c = spmv_col<TPR, VW>(s, v, 0);
+          if (ANY && c >= p.nvec) continue;
           spmv_cscale<VW>(p, c, &acc[v * VW]);
           T yv[VW];
           if (p.beta != T(0)) {
@@ -433,13 +440,27 @@ constexpr int pf_min_blocks()
 template <class T, int NV, int TPR, int NT, bool GRAM = false, int VB = 16>
 __global__ void __launch_bounds__(NT) k_sell_spmmv_pf(SellDev<T> A, SpmvArgs<T> p)
 {
-  sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB>(A, p);
+  sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB, false>(A, p);
 }
 
 template <class T, int NV, int TPR, int NT, bool GRAM, int VB, int MB>
 __global__ void __launch_bounds__(NT, MB) k_sell_spmmv_pf_mb(SellDev<T> A, SpmvArgs<T> p)
 {
-  sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB>(A, p);
+  sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB, false>(A, p);
+}
+
+// Any width and alignment: NV >= p.nvec columns, TPR threads a row, vectors
+// of VB bytes.  The minimum of resident blocks is what the registers of a
+// row's gathers leave, so that ptxas keeps all of them in flight.
+template <class T, int VPT, int NT>
+constexpr int pf_any_blocks()
+{
+  return 65536 / (NT * (VPT * 8 * (int)sizeof(T) / 4 + 48)) > 0 ? 65536 / (NT * (VPT * 8 * (int)sizeof(T) / 4 + 48)) : 1;
+}
+template <class T, int NV, int TPR, int NT, int VB>
+__global__ void __launch_bounds__(NT, (pf_any_blocks<T, NV / TPR, NT>())) k_sell_spmmv_pf_any(SellDev<T> A, SpmvArgs<T> p)
+{
+  sell_spmmv_pf<T, NV, TPR, NT, false, VB, true>(A, p);
 }
 
 // the entry point of a form
@@ -451,6 +472,100 @@ constexpr auto pf_kernel()
     return &k_sell_spmmv_pf_mb<T, NV, TPR, NT, GRAM, VB, mb>;
   else
     return &k_sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB>;
+}
+
+// ------------------------------------------------------------ longer rows
+// Rows of more than 8 entries (C = 32): the entries come in batches of KB.
+// The values and columns of the next batch are loaded before the X rows of
+// the current one, so that a batch costs one memory latency instead of two,
+// and KB gathers are in flight instead of four.  Arithmetic and order as
+// k_sell_spmmv (same bits).
+template <class T, int NV, int TPR, int NT, int VB, bool ANY>
+__global__ void __launch_bounds__(NT) k_sell_spmmv_long(SellDev<T> A, SpmvArgs<T> p)
+{
+  constexpr int CC = 32;
+  constexpr int VPT = NV / TPR;
+  constexpr int VWMAX = VB / sizeof(T);
+  constexpr int VW = VPT < VWMAX ? VPT : VWMAX;
+  constexpr int NVV = VPT / VW;
+  constexpr int RPB = NT / TPR;
+  constexpr int KB = VPT * (int)sizeof(T) <= 32 ? 8 : 4;
+  static_assert(VPT % VW == 0, "bad column split");
+  typedef typename Acc<T>::type AT;
+  const int s = threadIdx.x % TPR;
+  const int64_t r = blockIdx.x * (int64_t)RPB + threadIdx.x / TPR;  // SELL row
+  if (r >= A.nchunks * (int64_t)CC) return;
+  const int64_t ch = r / CC;
+  const int64_t base = A.chunk_ptr[ch] + (r - ch * CC);
+  const int len = A.chunk_len[ch];
+  const int64_t i = (r < A.nrows) ? (A.perm ? (int64_t)A.perm[r] : r) : -1;
+  const T* __restrict__ x = p.x + p.col0;
+  auto lcol = [&](int v) {
+    const int c = spmv_col<TPR, VW>(s, v, 0);
+    return ANY ? min(c, p.nvec - VW) : c;
+  };
+  T av[KB];
+  int cv[KB];
+  // entries [k0, k0 + KB) of the row; past the end entry len - 1 again
+  auto entries = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < KB; q++) {
+      const int64_t at = base + (int64_t)min(k0 + q, len - 1) * CC;
+      av[q] = __ldcs(A.val + at);
+      cv[q] = __ldcs(A.col + at);
+    }
+  };
+  AT acc[VPT];
+#pragma unroll
+  for (int q = 0; q < VPT; q++) acc[q] = AT(0);
+  if (len > 0) entries(0);
+  if (i >= 0 && p.has_shift) {
+    T xs[VPT];
+#pragma unroll
+    for (int v = 0; v < NVV; v++) Vec<T, VW>::ld(x + i * p.ldx + lcol(v), &xs[v * VW]);
+#pragma unroll
+    for (int v = 0; v < NVV; v++)
+#pragma unroll
+      for (int w = 0; w < VW; w++) acc[v * VW + w] = AT(p.sh[lcol(v) + w]) * AT(xs[v * VW + w]);
+  }
+  for (int k0 = 0; k0 < len; k0 += KB) {
+    T a[KB], xv[KB][VPT];
+#pragma unroll
+    for (int q = 0; q < KB; q++) {
+      a[q] = av[q];
+      const T* xr = x + (int64_t)cv[q] * p.ldx;
+#pragma unroll
+      for (int v = 0; v < NVV; v++) Vec<T, VW>::ld_ordered(xr + lcol(v), &xv[q][v * VW]);
+    }
+    if (k0 + KB < len) entries(k0 + KB);
+#pragma unroll
+    for (int q = 0; q < KB; q++)
+#pragma unroll
+      for (int v = 0; v < VPT; v++) reg_fence(xv[q][v]);
+#pragma unroll
+    for (int q = 0; q < KB; q++)
+      if (k0 + q < len)
+#pragma unroll
+        for (int v = 0; v < VPT; v++) acc[v] += AT(a[q]) * AT(xv[q][v]);
+  }
+  if (i < 0) return;
+  T* yr = p.y + p.col0 + i * p.ldy;
+#pragma unroll
+  for (int v = 0; v < NVV; v++) {
+    const int c = spmv_col<TPR, VW>(s, v, 0);
+    if (ANY && c >= p.nvec) continue;
+    spmv_cscale<VW>(p, c, &acc[v * VW]);
+    T yv[VW];
+    if (p.beta != T(0)) {
+      Vec<T, VW>::ld_plain(yr + c, yv);
+#pragma unroll
+      for (int w = 0; w < VW; w++) yv[w] = T(AT(p.alpha) * acc[v * VW + w] + AT(p.beta) * AT(yv[w]));
+    } else {
+#pragma unroll
+      for (int w = 0; w < VW; w++) yv[w] = T(AT(p.alpha) * acc[v * VW + w]);
+    }
+    Vec<T, VW>::st(yr + c, yv);
+  }
 }
 
 }  // namespace pb
