@@ -5,6 +5,7 @@
 #include <type_traits>
 
 #include "pb_frag.cuh"
+#include "pb_prec.cuh"
 
 namespace pb {
 namespace {
@@ -113,7 +114,61 @@ bool nn_mc(const FragNnArgs<T>& a)
   return false;
 }
 
+template <int MT, int TJ>
+void prec_launch(MvTmvPrecArgs& a)
+{
+  constexpr int U = MT <= 2 ? 8 : MT <= 4 ? 4 : 2;
+  const int64_t want = ceil_div(a.n > 0 ? a.n : 1, U * FRAG_NW);
+  const int grid = (int)std::min<int64_t>(want, 2 * (int64_t)rt().num_sms());
+  a.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
+  a.part = (double*)rt().scratch(2 * sizeof(double) * (size_t)(grid + ceil_div(grid, a.gsz)) * a.m * a.k);
+  a.counters = rt().counters();
+  k_mvTmv_prec<MT, TJ><<<grid, FRAG_BS, 0, stream()>>>(a);
+  PB_LAUNCH_CHECK();
+}
+
+template <int TJ>
+void prec_mt(MvTmvPrecArgs& a)
+{
+  switch ((a.m + 7) / 8) {
+    case 1: prec_launch<1, TJ>(a); return;
+    case 2: prec_launch<2, TJ>(a); return;
+    case 3: prec_launch<3, TJ>(a); return;
+    case 4: prec_launch<4, TJ>(a); return;
+    case 5: prec_launch<5, TJ>(a); return;
+    case 6: prec_launch<6, TJ>(a); return;
+    case 7: prec_launch<7, TJ>(a); return;
+    default: prec_launch<8, TJ>(a); return;
+  }
+}
+
 }  // namespace
+
+// Up to 64 columns of the wider block against 8 of the other per launch.  W'W
+// forms, for the columns j0.. of the result, only the rows up to j0 + 8 and
+// mirrors them.
+void launch_mvTmv_prec(int64_t n, int m, int k, double alpha, const double* V, int64_t ldv, const double* W,
+                       int64_t ldw, double beta, double* C, int64_t ldc)
+{
+  const bool swap = k > m;
+  const bool sym = V == W && ldv == ldw && m == k && m <= 64 && beta == 0.0;
+  for (int i0 = 0; i0 < std::max(m, k); i0 += 64)
+    for (int j0 = 0; j0 < std::min(m, k); j0 += 8) {
+      MvTmvPrecArgs a;
+      a.n = n;
+      a.m = sym ? std::min(m, j0 + 8) : std::min(64, std::max(m, k) - i0);
+      a.mirror = sym ? j0 : 0;
+      a.Cm = C + j0;
+      a.k = std::min(8, std::min(m, k) - j0);
+      a.V = (swap ? W : V) + i0; a.ldv = swap ? ldw : ldv;
+      a.W = (swap ? V : W) + j0; a.ldw = swap ? ldv : ldw;
+      a.alpha = alpha; a.beta = beta;
+      a.sr = swap ? ldc : 1; a.sc = swap ? 1 : ldc;
+      a.C = C + i0 * a.sr + j0 * a.sc;
+      if (a.k <= 4) prec_mt<1>(a);
+      else prec_mt<2>(a);
+    }
+}
 
 // Which products go here (us at n = 2,097,152, fragment | other kernel):
 //   * thin ones (at most 4 columns against 4, FP32 8) stay with the register

@@ -10,15 +10,20 @@
 // (Ogita, Rump and Oishi, "Accurate sum and dot product", SIAM J. Sci.
 // Comput. 26(6), 2005): every product is split exactly into p + e by an FMA
 // (TwoProduct), p is added to the running sum with TwoSum, and the rounding
-// errors of both are collected in a second accumulator.  Blocks stage row
-// tiles of V and W in shared memory; each thread owns up to NQ outputs, or,
-// for fewer outputs than threads, one output and a group of the tile's rows.
-// Per-block (sum, error) pairs are combined by the last block to arrive, in
-// block order with TwoSum, so the result does not depend on the schedule.
-// Finally C = alpha*(s + c) + beta*C is evaluated in double-double and
-// rounded once.
+// errors of both are collected in a second accumulator.
+//
+// Ten FP64 operations per product make the kernel bound by the FP64 pipe.
+// A warp streams its own rows straight from global memory: lane (li, lj)
+// owns, in each of MT tiles of 8 columns of V, column li against TJ columns
+// of W, so a loaded value serves a whole tile and nothing is staged or
+// synchronised (staging 32-row tiles through shared memory, one output per
+// thread, took 84 us for 8 x 8 at n = 262,144, most of it waiting).  The
+// (sum, error) pairs of warps and blocks are combined in fixed order with
+// TwoSum, the blocks in two levels of about sqrt(blocks), so the result does
+// not depend on the schedule.  Finally C = alpha*(s + c) + beta*C is
+// evaluated in double-double and rounded once.
 #pragma once
-#include "pb_core.hpp"
+#include "pb_frag.cuh"
 
 namespace pb {
 
@@ -51,108 +56,159 @@ __device__ __forceinline__ void dd_add(double& s, double& c, double s2, double c
 
 struct MvTmvPrecArgs {
   int64_t n;
-  int m, k;
+  int m, k;           // columns of V (at most 64) and W (at most 8)
   const double* V;
   int64_t ldv;
   const double* W;
   int64_t ldw;
   double alpha, beta;
-  double* C;          // device, column-major, ldc
-  int64_t ldc;
-  double* part;       // [gridDim.x][m*k][2]
-  unsigned int* counter;
+  double* C;          // C(i, j) at C[i*sr + j*sc]
+  int64_t sr, sc;
+  int mirror;         // W'W: outputs with i < mirror also go to
+  double* Cm;         // Cm[j*sr + i*sc]
+  double* part;       // [blocks + groups][m*k][2]
+  int gsz;
+  unsigned int* counters;
 };
 
-constexpr int PREC_BS = 256;
-constexpr int PREC_R = 32;  // rows per staged tile
-
-// Thread t owns output o = t mod nout (NQ = 1, nout <= PREC_BS) and takes the
-// rows g, g + G, ... of every tile, g = t / nout, G = PREC_BS / nout row
-// groups; with more outputs than threads (NQ > 1) every thread owns NQ
-// outputs and all rows.  The groups are combined in group order at the end.
+// the two-level sum of frag_tree_sum on (sum, error) pairs
 template <int NQ>
-__global__ void __launch_bounds__(PREC_BS) k_mvTmv_prec(MvTmvPrecArgs a)
+__device__ __forceinline__ bool prec_tree_sum(double* part, int nout, int gsz, unsigned int* counters, double (&s)[NQ],
+                                              double (&c)[NQ])
 {
-  __shared__ double vs[PREC_R][64 + 1];
-  __shared__ double ws[PREC_R][64 + 1];
-  const int tid = threadIdx.x;
-  const int m = a.m, k = a.k, nout = m * k;
-  const int G = NQ == 1 ? PREC_BS / nout : 1;  // row groups
-  const int g = NQ == 1 ? tid / nout : 0;
-  const bool active = g < G;
-  double s[NQ], c[NQ];
-  int orow[NQ], ocol[NQ];
+  __shared__ int last;
+  const int nb = gridDim.x, tid = threadIdx.x;
+  const int grp = blockIdx.x / gsz, ngrp = (nb + gsz - 1) / gsz;
+  const int b0 = grp * gsz, cnt = min(gsz, nb - b0);
+  auto arrive = [&](unsigned int* ctr, int total) {
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+      last = (atomicAdd(ctr, 1u) == (unsigned)total - 1);
+      if (last) *ctr = 0u;  // ready for the next launch
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0;
+  };
+  auto sum = [&](const double* p, int count) {
+#pragma unroll
+    for (int q = 0; q < NQ; q++) s[q] = c[q] = 0.0;
+    for (int b = 0; b < count; b += 4) {
+      double2 v[NQ][4];
+#pragma unroll
+      for (int q = 0; q < NQ; q++)
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int o = tid + q * FRAG_BS;
+          v[q][u] = make_double2(0.0, 0.0);
+          if (b + u < count && o < nout)
+            v[q][u] = __ldcg(reinterpret_cast<const double2*>(p) + (int64_t)(b + u) * nout + o);
+        }
+#pragma unroll
+      for (int q = 0; q < NQ; q++)
+#pragma unroll
+        for (int u = 0; u < 4; u++) dd_add(s[q], c[q], v[q][u].x, v[q][u].y);
+    }
+  };
+  auto put = [&](int64_t slot) {
+#pragma unroll
+    for (int q = 0; q < NQ; q++)
+      if (tid + q * FRAG_BS < nout)
+        reinterpret_cast<double2*>(part)[slot * nout + tid + q * FRAG_BS] = make_double2(s[q], c[q]);
+  };
+  put(blockIdx.x);
+  if (!arrive(counters + 1 + grp, cnt)) return false;
+  sum(part + 2 * (int64_t)b0 * nout, cnt);
+  put(nb + grp);
+  if (!arrive(counters, ngrp)) return false;
+  sum(part + 2 * (int64_t)nb * nout, ngrp);
+  return true;
+}
+
+template <int MT, int TJ>
+__global__ void __launch_bounds__(FRAG_BS, 2) k_mvTmv_prec(const __grid_constant__ MvTmvPrecArgs a)
+{
+  constexpr int U = MT <= 2 ? 8 : MT <= 4 ? 4 : 2;  // rows of loads in flight
+  constexpr int NO = MT * TJ * 32;                  // outputs, padded
+  constexpr int NQ = (NO + FRAG_BS - 1) / FRAG_BS;
+  constexpr int WB = NO <= 256 ? 8 : 4;             // warps combined at a time
+  __shared__ double2 red[WB * NO];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int li = lane & 7, lj = lane >> 3;
+  double s[MT][TJ], c[MT][TJ];
+#pragma unroll
+  for (int i = 0; i < MT; i++)
+#pragma unroll
+    for (int e = 0; e < TJ; e++) s[i][e] = c[i][e] = 0.0;
+  // columns past the blocks' ends read a column inside (outputs not stored)
+  int ci[MT], cj[TJ];
+#pragma unroll
+  for (int i = 0; i < MT; i++) ci[i] = min(8 * i + li, a.m - 1);
+#pragma unroll
+  for (int e = 0; e < TJ; e++) cj[e] = min(lj * TJ + e, a.k - 1);
+  const int64_t nch = (a.n + U - 1) / U;
+  const int64_t GW = gridDim.x * (int64_t)FRAG_NW;
+  for (int64_t ch = blockIdx.x * (int64_t)FRAG_NW + w; ch < nch; ch += GW) {
+    double x[U][MT], y[U][TJ];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      // rows past the end repeat the last one, times zero
+      const int64_t row = min(ch * U + u, a.n - 1);
+#pragma unroll
+      for (int i = 0; i < MT; i++) frag_ld1(a.V + row * a.ldv + ci[i], x[u][i]);
+#pragma unroll
+      for (int e = 0; e < TJ; e++) frag_ld1(a.W + row * a.ldw + cj[e], y[u][e]);
+    }
+    if ((ch + 1) * U > a.n)
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (ch * U + u >= a.n) {
+#pragma unroll
+          for (int i = 0; i < MT; i++) x[u][i] = 0.0;
+#pragma unroll
+          for (int e = 0; e < TJ; e++) y[u][e] = 0.0;
+        }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int e = 0; e < TJ; e++) dd_dot_step(x[u][i], y[u][e], s[i][e], c[i][e]);
+  }
+  // the warps in order; output (8i + li, lj*TJ + e) of the block at o = row + m*col
+  const int nout = a.m * a.k;
+  double ts[NQ], tc[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; q++) ts[q] = tc[q] = 0.0;
+#pragma unroll
+  for (int w0 = 0; w0 < FRAG_NW; w0 += WB) {
+    __syncthreads();
+    if (w >= w0 && w < w0 + WB)
+#pragma unroll
+      for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int e = 0; e < TJ; e++)
+          if (8 * i + li < a.m && lj * TJ + e < a.k)
+            red[(w - w0) * NO + 8 * i + li + (lj * TJ + e) * a.m] = make_double2(s[i][e], c[i][e]);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+      const int o = tid + q * FRAG_BS;
+      if (o < nout)
+#pragma unroll
+        for (int b = 0; b < WB; b++) dd_add(ts[q], tc[q], red[b * NO + o].x, red[b * NO + o].y);
+    }
+  }
+  if (!prec_tree_sum<NQ>(a.part, nout, a.gsz, a.counters, ts, tc)) return;
 #pragma unroll
   for (int q = 0; q < NQ; q++) {
-    s[q] = 0.0;
-    c[q] = 0.0;
-    const int o = NQ == 1 ? tid % nout : tid + q * PREC_BS;
-    orow[q] = o < nout ? o % m : 0;
-    ocol[q] = o < nout ? o / m : 0;
-  }
-  const int64_t ntiles = (a.n + PREC_R - 1) / PREC_R;
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int64_t i0 = t * PREC_R;
-    const int rows = a.n - i0 < PREC_R ? (int)(a.n - i0) : PREC_R;
-    __syncthreads();  // the previous tile has been consumed
-    for (int e = tid; e < PREC_R * m; e += PREC_BS) {
-      const int ii = e / m, r = e % m;
-      vs[ii][r] = ii < rows ? a.V[(i0 + ii) * a.ldv + r] : 0.0;
-    }
-    for (int e = tid; e < PREC_R * k; e += PREC_BS) {
-      const int ii = e / k, j = e % k;
-      ws[ii][j] = ii < rows ? a.W[(i0 + ii) * a.ldw + j] : 0.0;
-    }
-    __syncthreads();
-    if (active) {
-      for (int ii = g; ii < rows; ii += G) {
-#pragma unroll
-        for (int q = 0; q < NQ; q++)
-          if (NQ == 1 || tid + q * PREC_BS < nout) dd_dot_step(vs[ii][orow[q]], ws[ii][ocol[q]], s[q], c[q]);
-      }
-    }
-  }
-  if (NQ == 1 && G > 1) {
-    // row groups of one output, combined in group order
-    double* red = &vs[0][0];  // 2*PREC_BS <= PREC_R*65 entries
-    __syncthreads();
-    red[2 * tid] = s[0];
-    red[2 * tid + 1] = c[0];
-    __syncthreads();
-    if (tid < nout) {
-      double ss = 0.0, cc = 0.0;
-      for (int q = 0; q < G; q++) dd_add(ss, cc, red[2 * (q * nout + tid)], red[2 * (q * nout + tid) + 1]);
-      s[0] = ss;
-      c[0] = cc;
-    }
-  }
-  double* part = a.part + (int64_t)blockIdx.x * nout * 2;
-#pragma unroll
-  for (int q = 0; q < NQ; q++) {
-    const int o = tid + q * PREC_BS;
-    if (o < nout && (NQ > 1 || g == 0)) {
-      part[2 * o] = s[q];
-      part[2 * o + 1] = c[q];
-    }
-  }
-  __shared__ bool am_last;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) am_last = (atomicAdd(a.counter, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  for (int o = tid; o < nout; o += PREC_BS) {
-    double ss = 0.0, cc = 0.0;
-    for (int b = 0; b < (int)gridDim.x; b++) {
-      const double* pb = a.part + (int64_t)b * nout * 2;
-      dd_add(ss, cc, __ldcg(pb + 2 * o), __ldcg(pb + 2 * o + 1));
-    }
-    // alpha*(ss + cc) + beta*C in double-double, rounded once
-    const int r = o % m, j = o / m;
-    double* cp = a.C + r + (int64_t)j * a.ldc;
-    const double p = a.alpha * ss;
-    double ep = fma(a.alpha, ss, -p) + a.alpha * cc;
+    const int o = tid + q * FRAG_BS;
+    if (o >= nout) continue;
+    // alpha*(s + c) + beta*C in double-double, rounded once
+    double* cp = a.C + (o % a.m) * a.sr + (o / a.m) * a.sc;
+    const double p = a.alpha * ts[q];
+    const double ep = fma(a.alpha, ts[q], -p) + a.alpha * tc[q];
     double qv = 0.0, eq = 0.0;
     if (a.beta != 0.0) {
       qv = a.beta * *cp;
@@ -160,9 +216,14 @@ __global__ void __launch_bounds__(PREC_BS) k_mvTmv_prec(MvTmvPrecArgs a)
     }
     double t, et;
     dd_two_sum(p, qv, t, et);
-    *cp = t + (et + ep + eq);
+    const double r = t + (et + ep + eq);
+    *cp = r;
+    if (o % a.m < a.mirror) a.Cm[(o / a.m) * a.sr + (o % a.m) * a.sc] = r;
   }
-  if (tid == 0) *a.counter = 0u;
 }
+
+// C = alpha*V'W + beta*C with compensated sums (pb_frag.cu)
+void launch_mvTmv_prec(int64_t n, int m, int k, double alpha, const double* V, int64_t ldv, const double* W,
+                       int64_t ldw, double beta, double* C, int64_t ldc);
 
 }  // namespace pb
