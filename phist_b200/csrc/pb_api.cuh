@@ -321,15 +321,18 @@ void sd_upload(SdMat<T>* M)
 // Device -> host copy of an sdMat.  Small matrices (all the solvers' Gram and
 // projection matrices) go through the pinned mailbox: one asynchronous DMA,
 // one stream synchronisation and a host copy, instead of a pageable transfer.
+// in_mailbox: the kernel that made the values has put a copy there (dense,
+// column-major), so the synchronisation is all that is left.
 template <class T>
-void sd_download(SdMat<T>* M)
+void sd_download(SdMat<T>* M, bool in_mailbox = false)
 {
   if (M->nrows == 0 || M->ncols == 0) return;
   const size_t col = sizeof(T) * (size_t)M->nrows;
   if (col * (size_t)M->ncols <= Runtime::kMailboxResultBytes) {
     char* hb = (char*)rt().mailbox_host();
-    PB_CUDA(cudaMemcpy2DAsync(hb, col, M->d(), M->lda * sizeof(T), col, M->ncols, cudaMemcpyDeviceToHost,
-                              stream()));
+    if (!in_mailbox)
+      PB_CUDA(cudaMemcpy2DAsync(hb, col, M->d(), M->lda * sizeof(T), col, M->ncols, cudaMemcpyDeviceToHost,
+                                stream()));
     rt().sync();
     for (int j = 0; j < M->ncols; j++) memcpy(M->h() + (int64_t)j * M->lda, hb + col * j, col);
     return;
@@ -1217,11 +1220,13 @@ bool robust_requested(int flags_in)
   return (flags_in & PB_ROBUST_REDUCTIONS) && std::is_same<T, double>::value;
 }
 
+// mbox: mapped host memory for a dense copy of C, or NULL; true when the
+// kernels wrote it
 template <class T>
-void launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const T* W,
-                  int64_t ldw, T beta, T* Cd, int64_t ldc)
+bool launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const T* W,
+                  int64_t ldw, T beta, T* Cd, int64_t ldc, T* mbox = nullptr)
 {
-  if (frag_mvTmv<T>(n, m, k, alpha, V, ldv, W, ldw, beta, Cd, ldc)) return;
+  if (frag_mvTmv<T>(n, m, k, alpha, V, ldv, W, ldw, beta, Cd, ldc, mbox)) return mbox != nullptr;
   MvTmvArgs<T> a;
   a.n = n; a.m = m; a.k = k; a.V = V; a.ldv = ldv; a.W = W; a.ldw = ldw;
   a.alpha = alpha; a.beta = beta; a.Cd = Cd; a.ldc = ldc;
@@ -1243,11 +1248,12 @@ void launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, con
         a.part = (T*)rt().scratch(sizeof(T) * (size_t)grid * m * k);
         a.counter = rt().counters();
         a.R = 0;
+        a.mbox = mbox;
         kern<<<grid, 256, 0, stream()>>>(a);
         PB_LAUNCH_CHECK();
       };
       run(k_mvTmv_v4<4, 4, 4>, occ[0]);
-      return;
+      return mbox != nullptr;
     }
   }
   // thin blocks: one thread per row (n = 2,097,152, staged -> per row: FP64
@@ -1257,7 +1263,7 @@ void launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, con
     // multi-stage asynchronously staged row tiles, widths padded to 4..64
     mvtmv_async<T>(a, n, pad_width5(m), pad_width5(k));
     PB_LAUNCH_CHECK();
-    return;
+    return false;
   }
   if (m <= 8 && k <= 8) {
     // register kernel (odd or unaligned widths): padded widths M (4|8) and K (1|4|8)
@@ -1266,6 +1272,7 @@ void launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, con
     a.part = (T*)rt().scratch(sizeof(T) * (size_t)grid * M * K);
     a.counter = rt().counters();
     a.R = 0;
+    a.mbox = mbox;
 #define PB_MVR(Mv, Kv) k_mvTmv_reg<T, Mv, Kv><<<grid, 256, 0, stream()>>>(a)
     if (M == 4) {
       if (K == 1) PB_MVR(4, 1); else if (K == 4) PB_MVR(4, 4); else PB_MVR(4, 8);
@@ -1274,7 +1281,7 @@ void launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, con
     }
 #undef PB_MVR
     PB_LAUNCH_CHECK();
-    return;
+    return mbox != nullptr;
   }
   const bool big = (int64_t)m * k >= 256;
   const int TM = big ? 8 : 4, TK = big ? 8 : 4;
@@ -1301,6 +1308,24 @@ void launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, con
     kern<<<grid, BLK_BS, smem, stream()>>>(a);
   }
   PB_LAUNCH_CHECK();
+  return false;
+}
+
+// C = alpha*V'W + beta*C into an sdMat, compensated sums when robust, and the
+// host copy unless the flags leave the result on the device
+template <class T>
+void gram_to_sdmat(const Mvec<T>* V, const Mvec<T>* W, int k, T alpha, T beta, SdMat<T>* C, int flags)
+{
+  const bool host = !sd_device_only(flags);
+  T* mbox = host ? (T*)rt().mailbox_dev() : nullptr;
+  bool there = mbox != nullptr;
+  if (sizeof(T) * (size_t)V->nvec * k > Runtime::kMailboxResultBytes) mbox = nullptr;
+  if (robust_requested<T>(flags))
+    launch_mvTmv_prec(V->nrows, V->nvec, k, (double)alpha, (const double*)V->d(), V->lda, (const double*)W->d(),
+                      W->lda, (double)beta, (double*)C->d(), C->lda, (double*)mbox);
+  else
+    there = launch_mvTmv<T>(V->nrows, V->nvec, k, alpha, V->d(), V->lda, W->d(), W->lda, beta, C->d(), C->lda, mbox);
+  if (host) sd_download(C, there && mbox);
 }
 
 // fused V*C + Gram on the tensor cores (FP64, widths 8..64 in steps of 8)

@@ -73,6 +73,7 @@ struct MvTmvArgs {
   T* part; unsigned int* counter;
   int R;                        // rows per tile
   int ext_reduce;               // k_mvtmv_async: leave the partials to k_reduce_partials
+  T* mbox = nullptr;            // register kernels: the result's copy in mapped host memory
 };
 
 // thread (tm, tk, g): output micro-tile rows [tm*TM, +TM) of V' and columns
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(256) k_mvTmv_reg(MvTmvArgs<T> a)
     for (int p = 0; p < M; p++) vals[p + q * M] = acc[p + q * M];
   block_partial<T, M * K>(vals, a.part, M * K);
   // outputs are laid out with row stride M in the partials: map to (m, k)
-  last_block_reduce<T>(a.part, M * K, gridDim.x, a.counter, a.Cd, 1, M, a.ldc, a.alpha, a.beta, a.m, a.k);
+  last_block_reduce<T>(a.part, M * K, gridDim.x, a.counter, a.Cd, 1, M, a.ldc, a.alpha, a.beta, a.m, a.k, a.mbox);
 }
 
 // Thin blocks of exactly M and K columns (multiples of 4) whose rows start
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(256) k_mvTmv_v4(MvTmvArgs<double> a)
       for (int p = 0; p < M; p++) acc[p + q * M] += v[p] * w[q];
   }
   block_partial<double, M * K>(acc, a.part, M * K);
-  last_block_reduce<double>(a.part, M * K, gridDim.x, a.counter, a.Cd, 1, M, a.ldc, a.alpha, a.beta, a.m, a.k);
+  last_block_reduce<double>(a.part, M * K, gridDim.x, a.counter, a.Cd, 1, M, a.ldc, a.alpha, a.beta, a.m, a.k, a.mbox);
 }
 
 // row-local products for m, k, mv <= 8 (modes and Gram as k_rowgemm)

@@ -148,7 +148,7 @@ void prec_mt(MvTmvPrecArgs& a)
 // forms, for the columns j0.. of the result, only the rows up to j0 + 8 and
 // mirrors them.
 void launch_mvTmv_prec(int64_t n, int m, int k, double alpha, const double* V, int64_t ldv, const double* W,
-                       int64_t ldw, double beta, double* C, int64_t ldc)
+                       int64_t ldw, double beta, double* C, int64_t ldc, double* mbox)
 {
   const bool swap = k > m;
   const bool sym = V == W && ldv == ldw && m == k && m <= 64 && beta == 0.0;
@@ -159,6 +159,9 @@ void launch_mvTmv_prec(int64_t n, int m, int k, double alpha, const double* V, i
       a.m = sym ? std::min(m, j0 + 8) : std::min(64, std::max(m, k) - i0);
       a.mirror = sym ? j0 : 0;
       a.Cm = C + j0;
+      a.mr = swap ? m : 1; a.mc = swap ? 1 : m;
+      a.mbox = mbox ? mbox + i0 * a.mr + j0 * a.mc : nullptr;
+      a.mboxm = mbox ? mbox + j0 : nullptr;
       a.k = std::min(8, std::min(m, k) - j0);
       a.V = (swap ? W : V) + i0; a.ldv = swap ? ldw : ldv;
       a.W = (swap ? V : W) + j0; a.ldw = swap ? ldv : ldw;
@@ -181,7 +184,7 @@ void launch_mvTmv_prec(int64_t n, int m, int k, double alpha, const double* V, i
 //     other kernels stage element by element (37 x 5 141 | 850).
 template <class T>
 bool frag_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const T* W, int64_t ldw, T beta, T* C,
-                int64_t ldc)
+                int64_t ldc, T* mbox)
 {
   if (n < 1 || m < 1 || k < 1 || m > 64 || k > 64) return false;
   const bool sym = V == W && ldv == ldw && m == k;
@@ -197,6 +200,7 @@ bool frag_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const
     a.m = a.k = m;
     a.V = a.W = V; a.ldv = a.ldw = ldv;
     a.C = C; a.sr = 1; a.sc = ldc;
+    a.mbox = mbox; a.mr = 1; a.mc = m;
     return pair_ok(V, ldv, m) ? tn_sym<T, true>(a) : tn_sym<T, false>(a);
   }
   // the wider block supplies the rows of the product, the narrower one at
@@ -206,10 +210,12 @@ bool frag_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const
   a.V = swap ? W : V; a.ldv = swap ? ldw : ldv;
   a.ldw = swap ? ldv : ldw;
   a.sr = swap ? ldc : 1; a.sc = swap ? 1 : ldc;
+  a.mr = swap ? m : 1; a.mc = swap ? 1 : m;
   for (int j0 = 0; j0 < small; j0 += 16) {
     a.k = std::min(16, small - j0);
     a.W = (swap ? V : W) + j0;
     a.C = C + j0 * a.sc;
+    a.mbox = mbox ? mbox + j0 * a.mc : nullptr;
     const bool vec = pair_ok(a.V, a.ldv, a.m) && pair_ok(a.W, a.ldw, a.k);
     if (a.k <= 8) vec ? tn_mt<T, 1, true>(a) : tn_mt<T, 1, false>(a);
     else vec ? tn_mt<T, 2, true>(a) : tn_mt<T, 2, false>(a);
@@ -241,9 +247,9 @@ bool frag_mvsd(const RowGemmArgs<T>& r)
 }
 
 template bool frag_mvTmv<double>(int64_t, int, int, double, const double*, int64_t, const double*, int64_t, double,
-                                 double*, int64_t);
+                                 double*, int64_t, double*);
 template bool frag_mvTmv<float>(int64_t, int, int, float, const float*, int64_t, const float*, int64_t, float, float*,
-                                int64_t);
+                                int64_t, float*);
 template bool frag_mvsd<double>(const RowGemmArgs<double>&);
 template bool frag_mvsd<float>(const RowGemmArgs<float>&);
 

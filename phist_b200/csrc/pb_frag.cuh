@@ -49,6 +49,7 @@ struct FragTnArgs {
   const T* W; int64_t ldw;
   T alpha, beta;
   T* C; int64_t sr, sc;         // C(i, j) at C[i*sr + j*sc] for V column i, W column j
+  T* mbox; int mr, mc;          // copy of the result in mapped host memory (or NULL), strides mr, mc
   double* part;                 // (blocks + groups) x m*k partial sums
   int gsz;                      // blocks per group of the first reduction level
   unsigned int* counters;       // 1 + groups, zero between launches
@@ -275,7 +276,9 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_tn_frag(const __grid_constant__ 
     if (o < nout) {
       T* dst = a.C + (o % a.m) * a.sr + (o / a.m) * a.sc;
       const double s = (double)a.alpha * tot[q];
-      *dst = (T)(a.beta == T(0) ? s : s + (double)a.beta * (double)*dst);
+      const T r = (T)(a.beta == T(0) ? s : s + (double)a.beta * (double)*dst);
+      *dst = r;
+      if (a.mbox) a.mbox[(o % a.m) * a.mr + (o / a.m) * a.mc] = r;
     }
   }
 }
@@ -375,10 +378,11 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_nn_frag(const __grid_constant__ 
 }
 
 // C = alpha V'W + beta C / W = alpha V C + beta W with the kernels above;
-// false when the shape is not theirs (pb_frag.cu holds the rule)
+// false when the shape is not theirs (pb_frag.cu holds the rule).  mbox: C
+// also goes there, dense and column-major (mapped host memory), or NULL.
 template <class T>
 bool frag_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const T* W, int64_t ldw, T beta, T* C,
-                int64_t ldc);
+                int64_t ldc, T* mbox);
 template <class T>
 bool frag_mvsd(const RowGemmArgs<T>& a);
 

@@ -66,6 +66,7 @@ struct MvTmvPrecArgs {
   int64_t sr, sc;
   int mirror;         // W'W: outputs with i < mirror also go to
   double* Cm;         // Cm[j*sr + i*sc]
+  double *mbox, *mboxm; int mr, mc;  // copies of C and Cm in mapped host memory (or NULL), strides mr, mc
   double* part;       // [blocks + groups][m*k][2]
   int gsz;
   unsigned int* counters;
@@ -218,12 +219,16 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_mvTmv_prec(const __grid_constant
     dd_two_sum(p, qv, t, et);
     const double r = t + (et + ep + eq);
     *cp = r;
-    if (o % a.m < a.mirror) a.Cm[(o / a.m) * a.sr + (o % a.m) * a.sc] = r;
+    if (a.mbox) a.mbox[(o % a.m) * a.mr + (o / a.m) * a.mc] = r;
+    if (o % a.m < a.mirror) {
+      a.Cm[(o / a.m) * a.sr + (o % a.m) * a.sc] = r;
+      if (a.mboxm) a.mboxm[(o / a.m) * a.mr + (o % a.m) * a.mc] = r;
+    }
   }
 }
 
 // C = alpha*V'W + beta*C with compensated sums (pb_frag.cu)
 void launch_mvTmv_prec(int64_t n, int m, int k, double alpha, const double* V, int64_t ldv, const double* W,
-                       int64_t ldw, double beta, double* C, int64_t ldc);
+                       int64_t ldw, double beta, double* C, int64_t ldc, double* mbox);
 
 }  // namespace pb

@@ -27,7 +27,8 @@ struct Acc<float> { typedef float type; };
 // with out[o] not read when beta == 0).  Output o goes to
 // out[(o % out_rows)*out_stride_rows + (o / out_rows)*ld_out].
 // Outputs whose row is >= vrows or whose column is >= vcols are padding and
-// are not written.
+// are not written.  mbox: further copy of the result, column-major and dense
+// (mapped host memory).
 // Sum of v over the threads t == c (mod w) of a 256-thread block, for each
 // residue c < w (w a power of two <= 256), returned to thread c; other threads
 // get an unspecified value.  Fixed order: a butterfly over the lanes of each
@@ -52,7 +53,7 @@ __device__ __forceinline__ bool last_block_reduce(const T* part, int nout, int n
                                                   unsigned int* counter, T* out,
                                                   int64_t out_stride_rows, int out_rows,
                                                   int64_t ld_out, T alpha, T beta,
-                                                  int vrows = 1 << 30, int vcols = 1 << 30)
+                                                  int vrows = 1 << 30, int vcols = 1 << 30, T* mbox = nullptr)
 {
   __shared__ bool am_last;
   __shared__ T red[256];  // all callers launch at most 256 threads per block
@@ -111,7 +112,9 @@ __device__ __forceinline__ bool last_block_reduce(const T* part, int nout, int n
       const int r = o % out_rows, c = o / out_rows;
       if (r < vrows && c < vcols) {
         T* dst = out + r * out_stride_rows + (int64_t)c * ld_out;
-        *dst = (beta == T(0)) ? alpha * s : alpha * s + beta * (*dst);
+        const T v = (beta == T(0)) ? alpha * s : alpha * s + beta * (*dst);
+        *dst = v;
+        if (mbox) mbox[r + c * min(vrows, out_rows)] = v;
       }
     }
   }
