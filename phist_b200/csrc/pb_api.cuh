@@ -1386,34 +1386,32 @@ bool mvsd_gram_dmma_mv(RowGemmArgs<double>& a, int MV)
   }
 }
 
-// True if the fused tensor-core kernel took the product.  Up to 16 columns:
-// beyond, the shared-memory tiles leave one or two blocks per SM and the
-// product followed by the Gram product is faster (n = 2,097,152, m = k,
-// W'W: fused 80 / 150 / 395 / 1,290 us at 8 / 16 / 32 / 64 columns, the two
-// passes of pb_frag.cuh 89 / 163 / 320 / 1,240 us).
+// True if the fused tensor-core kernel took W(:,0:k) = W C with V'W of another
+// block V.  Up to 16 columns: beyond, its shared-memory tiles leave one or two
+// blocks per SM and the product followed by V'W is faster (n = 2,097,152,
+// square: fused 80 / 150 / 395 us at 8 / 16 / 32 columns, the two passes of
+// pb_frag.cuh 113 / 208 / 389 us).
 inline bool mvsd_gram_dmma(RowGemmArgs<double>& a)
 {
-  if (!rt().use_tma || !rt().use_dmma || a.mode == RM_VCWD || a.gram == GM_NONE) return false;
+  if (!rt().use_tma || !rt().use_dmma || a.mode == RM_VCWD || a.gram != GM_VW) return false;
   if (a.m > 16 || a.k > 16 || a.m < 5 || a.k < 5) return false;  // widths <= 4: register kernel
   const int BM = pad_width5(a.m), BK = pad_width5(a.k);
-  if (a.gram == GM_WW) {
-    if (BM == 8) return BK == 8 ? mvsd_gram_dmma_launch<8, 8, 8, GM_WW>(a) : mvsd_gram_dmma_launch<8, 16, 16, GM_WW>(a);
-    return BK == 8 ? mvsd_gram_dmma_launch<16, 8, 8, GM_WW>(a) : mvsd_gram_dmma_launch<16, 16, 16, GM_WW>(a);
-  }
-  // V'W with the in-place product: square blocks only (BM == BK)
-  if (a.mv < 5 || a.mv > 64 || BM != BK) return false;
+  if (a.mv < 5 || a.mv > 64 || BM != BK) return false;  // square blocks only
   const int MV = pad_width5(a.mv);
   return BM == 8 ? mvsd_gram_dmma_mv<8, 8, GM_VW>(a, MV) : mvsd_gram_dmma_mv<16, 16, GM_VW>(a, MV);
 }
 inline bool mvsd_gram_dmma(RowGemmArgs<float>&) { return false; }
 
+// mbox: mapped host memory for a dense copy of the Gram matrix, or NULL; true
+// when the kernel wrote it
 template <class T>
-void launch_rowgemm(RowGemmArgs<T>& a)
+bool launch_rowgemm(RowGemmArgs<T>& a, T* mbox = nullptr)
 {
-  if (a.n == 0 && a.gram == GM_NONE) return;
+  if (a.n == 0 && a.gram == GM_NONE) return false;
   // fused V*C + Gram in one pass on the tensor cores
-  if (mvsd_gram_dmma(a)) return;
-  if (a.gram == GM_NONE && a.mode != RM_VCWD && frag_mvsd(a)) return;
+  if (a.gram == GM_WW && a.mode != RM_VCWD && frag_mvsd_gram<T>(a, mbox)) return mbox != nullptr;
+  if (mvsd_gram_dmma(a)) return false;
+  if (a.gram == GM_NONE && a.mode != RM_VCWD && frag_mvsd(a)) return false;
   const bool thin = a.k <= 4 && a.m <= (sizeof(T) == 4 ? 8 : 4);
   if (a.m <= 8 && a.k <= 8 && (thin || a.mode == RM_VCWD) && (a.gram != GM_VW || a.mv <= 8)) {
     // register kernel (thin blocks, V C + W D): padded widths M (4|8), K (1|4|8), MV (1, or 8 for V'W)
@@ -1436,7 +1434,7 @@ void launch_rowgemm(RowGemmArgs<T>& a)
 #undef PB_RGR_K
 #undef PB_RGR
     PB_LAUNCH_CHECK();
-    return;
+    return false;
   }
   // fused Gram at the other widths: a second pass over the new W
   if (a.gram != GM_NONE && a.mode != RM_VCWD && (a.gram == GM_WW || a.mv <= 64) && frag_mvsd(a)) {
@@ -1444,7 +1442,7 @@ void launch_rowgemm(RowGemmArgs<T>& a)
       launch_mvTmv<T>(a.n, a.k, a.k, T(1), a.W, a.ldw, a.W, a.ldw, T(0), a.Gd, a.ldg);
     else
       launch_mvTmv<T>(a.n, a.mv, a.k, a.galpha, a.Vg, a.ldvg, a.W, a.ldw, a.gbeta, a.Gd, a.ldg);
-    return;
+    return false;
   }
   // micro-tile: TK columns per thread, TR rows
   const int TK = a.k >= 32 ? 8 : a.k >= 8 ? 4 : a.k >= 2 ? 2 : 1;
@@ -1480,6 +1478,7 @@ void launch_rowgemm(RowGemmArgs<T>& a)
   else PB_RG_LAUNCH(1, 1)
 #undef PB_RG_LAUNCH
   PB_LAUNCH_CHECK();
+  return false;
 }
 
 template <class T>

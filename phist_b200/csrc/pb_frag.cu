@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
 #include <type_traits>
 
 #include "pb_frag.cuh"
@@ -112,6 +113,32 @@ bool nn_mc(const FragNnArgs<T>& a)
     case 8: nn_launch<T, 8, KT, VEC>(a); return true;
   }
   return false;
+}
+
+template <class T, int MC, int KT, bool VEC>
+void nn_gram_launch(const FragNnArgs<T>& a, FragTnArgs<T>& go)
+{
+  constexpr int RT = 2;
+  auto kern = k_nn_gram_frag<T, MC, KT, VEC, RT>;
+  static std::atomic<int> occ{0};
+  const int64_t want = ceil_div(a.n, 8 * RT * FRAG_NW);
+  const int grid = (int)std::min<int64_t>(want, (int64_t)rt().num_sms() * std::min(3, frag_occ(kern, occ)));
+  go.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
+  go.part = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ceil_div(grid, go.gsz)) * a.k * a.k);
+  go.counters = rt().counters();
+  kern<<<grid, FRAG_BS, 0, stream()>>>(a, go);
+  PB_LAUNCH_CHECK();
+}
+
+template <class T, int KT, bool VEC>
+void nn_gram_mc(const FragNnArgs<T>& a, FragTnArgs<T>& go)
+{
+  switch ((a.m + 7) / 8) {
+    case 1: nn_gram_launch<T, 1, KT, VEC>(a, go); return;
+    case 2: nn_gram_launch<T, 2, KT, VEC>(a, go); return;
+    case 3: nn_gram_launch<T, 3, KT, VEC>(a, go); return;
+    default: nn_gram_launch<T, 4, KT, VEC>(a, go); return;
+  }
 }
 
 template <int MT, int TJ>
@@ -246,11 +273,42 @@ bool frag_mvsd(const RowGemmArgs<T>& r)
   return vec ? nn_mc<T, 8, true>(a) : nn_mc<T, 8, false>(a);
 }
 
+template <class T>
+bool frag_mvsd_gram(const RowGemmArgs<T>& r, T* mbox)
+{
+  const bool inplace = r.mode == RM_MVSDI;
+  if (r.n < 1 || r.m < 1 || r.k < 1 || r.m > 32 || r.k > 32) return false;
+  FragNnArgs<T> a;
+  a.n = r.n; a.m = r.m; a.k = r.k;
+  a.V = inplace ? (const T*)r.W : r.V;
+  a.ldv = inplace ? r.ldw : r.ldv;
+  a.W = r.W; a.ldw = r.ldw;
+  a.C = r.C; a.ldc = r.ldc;
+  a.alpha = inplace ? T(1) : r.alpha;
+  a.beta = inplace ? T(0) : r.beta;
+  FragTnArgs<T> go;
+  memset(&go, 0, sizeof(go));
+  go.n = r.n; go.m = go.k = r.k;
+  go.alpha = r.galpha; go.beta = r.gbeta;
+  go.C = r.Gd; go.sr = 1; go.sc = r.ldg;
+  go.mbox = mbox; go.mr = 1; go.mc = r.k;
+  const bool vec = pair_ok(a.V, a.ldv, a.m) && pair_ok((const T*)a.W, a.ldw, a.k);
+  switch ((a.k + 7) / 8) {
+    case 1: vec ? nn_gram_mc<T, 1, true>(a, go) : nn_gram_mc<T, 1, false>(a, go); break;
+    case 2: vec ? nn_gram_mc<T, 2, true>(a, go) : nn_gram_mc<T, 2, false>(a, go); break;
+    case 3: vec ? nn_gram_mc<T, 3, true>(a, go) : nn_gram_mc<T, 3, false>(a, go); break;
+    default: vec ? nn_gram_mc<T, 4, true>(a, go) : nn_gram_mc<T, 4, false>(a, go); break;
+  }
+  return true;
+}
+
 template bool frag_mvTmv<double>(int64_t, int, int, double, const double*, int64_t, const double*, int64_t, double,
                                  double*, int64_t, double*);
 template bool frag_mvTmv<float>(int64_t, int, int, float, const float*, int64_t, const float*, int64_t, float, float*,
                                 int64_t, float*);
 template bool frag_mvsd<double>(const RowGemmArgs<double>&);
 template bool frag_mvsd<float>(const RowGemmArgs<float>&);
+template bool frag_mvsd_gram<double>(const RowGemmArgs<double>&, double*);
+template bool frag_mvsd_gram<float>(const RowGemmArgs<float>&, float*);
 
 }  // namespace pb

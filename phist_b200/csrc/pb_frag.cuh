@@ -177,62 +177,28 @@ __device__ __forceinline__ void frag_row(const T* row, int ncol, int g, T* v)
   }
 }
 
-// C = alpha V'W + beta C.  Warps take chunks of 4U rows in grid-stride
-// order.  SYM: W is V, the fragments of V serve both operands and only the
-// tiles on and above the diagonal are formed.
-template <class T, int MT, int KT, bool SYM, bool VEC, int U>
-__global__ void __launch_bounds__(FRAG_BS, 2) k_tn_frag(const __grid_constant__ FragTnArgs<T> a)
+// shared memory of frag_finish: WB warps' outputs
+template <int MT, int KT>
+constexpr int frag_wb()
 {
-  static_assert(!SYM || MT == KT, "a symmetric product is square");
-  constexpr int NTILE = SYM ? MT * (MT + 1) / 2 : MT * KT;
-  constexpr int NOUT = MT * KT * 64;
-  constexpr int WB = NOUT <= 512 ? 8 : NOUT <= 1024 ? 4 : 2;
-  __shared__ double red[WB * NOUT];  // of each warp: column-major, MT*8 rows
+  return MT * KT <= 8 ? 8 : MT * KT <= 16 ? 4 : 2;
+}
+template <int MT, int KT>
+constexpr int frag_red()
+{
+  return frag_wb<MT, KT>() * MT * KT * 64;
+}
+
+// The end of a V'W kernel: acc holds the warp's tiles (SYM: those on and above
+// the diagonal); warps, then blocks are summed in fixed order and the block
+// with the totals writes C = alpha V'W + beta C.  red: frag_red<MT, KT>()
+// doubles, free on entry after a barrier.
+template <class T, int MT, int KT, bool SYM, bool VEC, int NTILE>
+__device__ __forceinline__ void frag_finish(const FragTnArgs<T>& a, const double (&acc)[NTILE][2], double* red)
+{
+  constexpr int NOUT = MT * KT * 64, WB = frag_wb<MT, KT>();
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  double acc[NTILE][2];
-#pragma unroll
-  for (int i = 0; i < NTILE; i++) acc[i][0] = acc[i][1] = 0.0;
-
-  auto step = [&](const T* v, const T* wv) {
-    int q = 0;
-#pragma unroll
-    for (int j = 0; j < KT; j++)
-#pragma unroll
-      for (int i = 0; i < (SYM ? j + 1 : MT); i++, q++)
-        dmma_884(acc[q][0], acc[q][1], (double)v[i], (double)(SYM ? v[j] : wv[j]));
-  };
-  const int64_t nch = a.n / (4 * U);
-  const int64_t gw = blockIdx.x * (int64_t)FRAG_NW + w, GW = gridDim.x * (int64_t)FRAG_NW;
-  for (int64_t c = gw; c < nch; c += GW) {
-    const int64_t r = c * (4 * U) + t;
-    const T* pv = a.V + r * a.ldv;
-    const T* pw = a.W + r * a.ldw;
-    T v[U][MT], wv[U][KT];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      frag_row<T, MT, VEC>(pv + 4 * u * a.ldv, a.m, g, v[u]);
-      if (!SYM) frag_row<T, KT, VEC>(pw + 4 * u * a.ldw, a.k, g, wv[u]);
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) step(v[u], wv[u]);
-  }
-  if (gw == nch % GW) {
-    // the last rows: steps past the block's end multiply zeros
-    for (int64_t r0 = nch * (4 * U); r0 < a.n; r0 += 4) {
-      const int64_t r = r0 + t;
-      T v[MT], wv[KT];
-#pragma unroll
-      for (int i = 0; i < MT; i++) v[i] = T(0);
-#pragma unroll
-      for (int j = 0; j < KT; j++) wv[j] = T(0);
-      if (r < a.n) {
-        frag_row<T, MT, VEC>(a.V + r * a.ldv, a.m, g, v);
-        if (!SYM) frag_row<T, KT, VEC>(a.W + r * a.ldw, a.k, g, wv);
-      }
-      step(v, wv);
-    }
-  }
   // the warps' sums in warp order, WB warps at a time through shared memory
   const int nout = a.m * a.k;
   constexpr int NQ = (NOUT + FRAG_BS - 1) / FRAG_BS;
@@ -283,6 +249,104 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_tn_frag(const __grid_constant__ 
   }
 }
 
+// C = alpha V'W + beta C.  Warps take chunks of 4U rows in grid-stride
+// order.  SYM: W is V, the fragments of V serve both operands and only the
+// tiles on and above the diagonal are formed.
+template <class T, int MT, int KT, bool SYM, bool VEC, int U>
+__global__ void __launch_bounds__(FRAG_BS, 2) k_tn_frag(const __grid_constant__ FragTnArgs<T> a)
+{
+  static_assert(!SYM || MT == KT, "a symmetric product is square");
+  constexpr int NTILE = SYM ? MT * (MT + 1) / 2 : MT * KT;
+  __shared__ double red[frag_red<MT, KT>()];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  double acc[NTILE][2];
+#pragma unroll
+  for (int i = 0; i < NTILE; i++) acc[i][0] = acc[i][1] = 0.0;
+
+  auto step = [&](const T* v, const T* wv) {
+    int q = 0;
+#pragma unroll
+    for (int j = 0; j < KT; j++)
+#pragma unroll
+      for (int i = 0; i < (SYM ? j + 1 : MT); i++, q++)
+        dmma_884(acc[q][0], acc[q][1], (double)v[i], (double)(SYM ? v[j] : wv[j]));
+  };
+  const int64_t nch = a.n / (4 * U);
+  const int64_t gw = blockIdx.x * (int64_t)FRAG_NW + w, GW = gridDim.x * (int64_t)FRAG_NW;
+  for (int64_t c = gw; c < nch; c += GW) {
+    const int64_t r = c * (4 * U) + t;
+    const T* pv = a.V + r * a.ldv;
+    const T* pw = a.W + r * a.ldw;
+    T v[U][MT], wv[U][KT];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      frag_row<T, MT, VEC>(pv + 4 * u * a.ldv, a.m, g, v[u]);
+      if (!SYM) frag_row<T, KT, VEC>(pw + 4 * u * a.ldw, a.k, g, wv[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) step(v[u], wv[u]);
+  }
+  if (gw == nch % GW) {
+    // the last rows: steps past the block's end multiply zeros
+    for (int64_t r0 = nch * (4 * U); r0 < a.n; r0 += 4) {
+      const int64_t r = r0 + t;
+      T v[MT], wv[KT];
+#pragma unroll
+      for (int i = 0; i < MT; i++) v[i] = T(0);
+#pragma unroll
+      for (int j = 0; j < KT; j++) wv[j] = T(0);
+      if (r < a.n) {
+        frag_row<T, MT, VEC>(a.V + r * a.ldv, a.m, g, v);
+        if (!SYM) frag_row<T, KT, VEC>(a.W + r * a.ldw, a.k, g, wv);
+      }
+      step(v, wv);
+    }
+  }
+  frag_finish<T, MT, KT, SYM, VEC>(a, acc, red);
+}
+
+// chunk ch of 8*RT rows: the fragments of V, and for beta != 0 the old W in
+// the layout of the result
+template <class T, int MC, int KT, bool VEC, int RT>
+__device__ __forceinline__ void frag_nn_load(const FragNnArgs<T>& a, int64_t ch, int g, int t, T (&v)[RT][2 * MC],
+                                             T (&wo)[RT][KT][2])
+{
+#pragma unroll
+  for (int r = 0; r < RT; r++) {
+    // rows past the end read the last row and are not stored
+    const int64_t row = min(ch * (8 * RT) + 8 * r + g, a.n - 1);
+    const T* pv = a.V + row * a.ldv;
+#pragma unroll
+    for (int q = 0; q < MC; q++) {
+      // columns past m must not meet the zero rows of C as infinities
+      const bool whole = q < MC - 1;
+      if (VEC) {
+        v[r][2 * q] = v[r][2 * q + 1] = T(0);
+        if (whole || 8 * q + 2 * t < a.m) frag_ld2(pv + 8 * q + 2 * t, v[r][2 * q], v[r][2 * q + 1]);
+      } else {
+        v[r][2 * q] = v[r][2 * q + 1] = T(0);
+        if (whole || 8 * q + t < a.m) frag_ld1(pv + 8 * q + t, v[r][2 * q]);
+        if (whole || 8 * q + 4 + t < a.m) frag_ld1(pv + 8 * q + 4 + t, v[r][2 * q + 1]);
+      }
+    }
+    if (a.beta != T(0)) {
+      const T* pw = a.W + row * a.ldw;
+#pragma unroll
+      for (int j = 0; j < KT; j++) {
+        const int c = 8 * j + 2 * t;
+        wo[r][j][0] = wo[r][j][1] = T(0);
+        if (VEC) {
+          if (c < a.k) frag_ld2(pw + c, wo[r][j][0], wo[r][j][1]);
+        } else {
+          if (c < a.k) frag_ld1(pw + c, wo[r][j][0]);
+          if (c + 1 < a.k) frag_ld1(pw + c + 1, wo[r][j][1]);
+        }
+      }
+    }
+  }
+}
+
 // W = alpha V C + beta W (V == W: in place).  A warp owns 8*RT rows: all its
 // fragments of V are in registers before the first store, so the update in
 // place needs no copy.  C sits in shared memory in fragment order.  WV: rows
@@ -306,39 +370,7 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_nn_frag(const __grid_constant__ 
   const int64_t GW = gridDim.x * (int64_t)FRAG_NW;
   for (int64_t ch = blockIdx.x * (int64_t)FRAG_NW + w; ch < nch; ch += GW) {
     T v[RT][KS], wo[RT][KT][2];
-#pragma unroll
-    for (int r = 0; r < RT; r++) {
-      // rows past the end read the last row and are not stored
-      const int64_t row = min(ch * (8 * RT) + 8 * r + g, a.n - 1);
-      const T* pv = a.V + row * a.ldv;
-#pragma unroll
-      for (int q = 0; q < MC; q++) {
-        // columns past m must not meet the zero rows of C as infinities
-        const bool whole = q < MC - 1;
-        if (VEC) {
-          v[r][2 * q] = v[r][2 * q + 1] = T(0);
-          if (whole || 8 * q + 2 * t < a.m) frag_ld2(pv + 8 * q + 2 * t, v[r][2 * q], v[r][2 * q + 1]);
-        } else {
-          v[r][2 * q] = v[r][2 * q + 1] = T(0);
-          if (whole || 8 * q + t < a.m) frag_ld1(pv + 8 * q + t, v[r][2 * q]);
-          if (whole || 8 * q + 4 + t < a.m) frag_ld1(pv + 8 * q + 4 + t, v[r][2 * q + 1]);
-        }
-      }
-      if (a.beta != T(0)) {
-        const T* pw = a.W + row * a.ldw;
-#pragma unroll
-        for (int j = 0; j < KT; j++) {
-          const int c = 8 * j + 2 * t;
-          wo[r][j][0] = wo[r][j][1] = T(0);
-          if (VEC) {
-            if (c < a.k) frag_ld2(pw + c, wo[r][j][0], wo[r][j][1]);
-          } else {
-            if (c < a.k) frag_ld1(pw + c, wo[r][j][0]);
-            if (c + 1 < a.k) frag_ld1(pw + c + 1, wo[r][j][1]);
-          }
-        }
-      }
-    }
+    frag_nn_load<T, MC, KT, VEC, RT>(a, ch, g, t, v, wo);
     double acc[RT][KT][2];
 #pragma unroll
     for (int r = 0; r < RT; r++)
@@ -377,6 +409,93 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_nn_frag(const __grid_constant__ 
   }
 }
 
+// W = alpha V C + beta W (or in place) and G = galpha W'W + gbeta G of the new
+// W in one pass (go.alpha, go.beta, go.C; go.m == go.k == a.k): the rows that
+// a warp has just formed go through its own shared-memory tile from the
+// result's fragment layout to the operands', and the tiles of W'W on and
+// above the diagonal are accumulated at once, so W is not read again.
+template <class T, int MC, int KT, bool VEC, int RT>
+__global__ void __launch_bounds__(FRAG_BS, (MC * KT > 6 ? 1 : 2))
+k_nn_gram_frag(const __grid_constant__ FragNnArgs<T> a, const __grid_constant__ FragTnArgs<T> go)
+{
+  constexpr int KS = 2 * MC, P = KT * 8 + 4;
+  constexpr int NC = KS * KT * 32, NTL = FRAG_NW * 8 * P, NRED = frag_red<KT, KT>();
+  constexpr int NTILE = KT * (KT + 1) / 2;
+  __shared__ double sm[NC + NTL > NRED ? NC + NTL : NRED];
+  double* sC = sm;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  double* tile = sm + NC + w * 8 * P;
+  for (int q = tid; q < NC; q += FRAG_BS) {
+    const int l = q & 31, j = (q >> 5) % KT, s = (q >> 5) / KT;
+    const int i = VEC ? 8 * (s / 2) + 2 * (l & 3) + (s & 1) : 4 * s + (l & 3), c = j * 8 + (l >> 2);
+    sC[q] = (i < a.m && c < a.k) ? (double)a.C[i + (int64_t)c * a.ldc] : 0.0;
+  }
+  __syncthreads();
+  double gacc[NTILE][2];
+#pragma unroll
+  for (int i = 0; i < NTILE; i++) gacc[i][0] = gacc[i][1] = 0.0;
+  const int64_t nch = (a.n + 8 * RT - 1) / (8 * RT);
+  const int64_t GW = gridDim.x * (int64_t)FRAG_NW;
+  for (int64_t ch = blockIdx.x * (int64_t)FRAG_NW + w; ch < nch; ch += GW) {
+    T v[RT][KS], wo[RT][KT][2];
+    frag_nn_load<T, MC, KT, VEC, RT>(a, ch, g, t, v, wo);
+    double acc[RT][KT][2];
+#pragma unroll
+    for (int r = 0; r < RT; r++)
+#pragma unroll
+      for (int j = 0; j < KT; j++) acc[r][j][0] = acc[r][j][1] = 0.0;
+#pragma unroll
+    for (int s = 0; s < KS; s++)
+#pragma unroll
+      for (int j = 0; j < KT; j++) {
+        const double b = sC[(s * KT + j) * 32 + lane];
+#pragma unroll
+        for (int r = 0; r < RT; r++) dmma_884(acc[r][j][0], acc[r][j][1], (double)v[r][s], b);
+      }
+#pragma unroll
+    for (int r = 0; r < RT; r++) {
+      const int64_t row = ch * (8 * RT) + 8 * r + g;
+      T* pw = a.W + row * a.ldw;
+#pragma unroll
+      for (int j = 0; j < KT; j++) {
+        const int c = 8 * j + 2 * t;
+        T o[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          double x = (double)a.alpha * acc[r][j][e];
+          if (a.beta != T(0)) x += (double)a.beta * (double)wo[r][j][e];
+          o[e] = row < a.n ? (T)x : T(0);
+        }
+        if (row < a.n) {
+          if (VEC) {
+            if (c < a.k) frag_st2(pw + c, o[0], o[1]);
+          } else {
+            if (c < a.k) pw[c] = o[0];
+            if (c + 1 < a.k) pw[c + 1] = o[1];
+          }
+        }
+        frag_st2(tile + g * P + c, (double)o[0], (double)o[1]);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        double f[KT];
+#pragma unroll
+        for (int j = 0; j < KT; j++) f[j] = tile[(4 * h + t) * P + 8 * j + g];
+        int q = 0;
+#pragma unroll
+        for (int j = 0; j < KT; j++)
+#pragma unroll
+          for (int i = 0; i <= j; i++, q++) dmma_884(gacc[q][0], gacc[q][1], f[i], f[j]);
+      }
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  frag_finish<T, KT, KT, true, false>(go, gacc, sm);
+}
+
 // C = alpha V'W + beta C / W = alpha V C + beta W with the kernels above;
 // false when the shape is not theirs (pb_frag.cu holds the rule).  mbox: C
 // also goes there, dense and column-major (mapped host memory), or NULL.
@@ -385,5 +504,9 @@ bool frag_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const
                 int64_t ldc, T* mbox);
 template <class T>
 bool frag_mvsd(const RowGemmArgs<T>& a);
+// the same with G = galpha W'W + gbeta G (a.Gd, a.ldg) of the new W in one
+// pass; mbox as above
+template <class T>
+bool frag_mvsd_gram(const RowGemmArgs<T>& a, T* mbox);
 
 }  // namespace pb
