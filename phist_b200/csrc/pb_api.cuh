@@ -148,8 +148,8 @@ template <class T>
 void copy_cols(const Mvec<T>* X, int xoff, Mvec<T>* Y, int yoff, int ncols)
 {
   if (X->nrows == 0 || ncols == 0) return;
-  k_copy<T, T><<<grid_for((int64_t)X->nrows * ncols), 256, 0, stream()>>>(
-      X->d() + xoff, X->lda, Y->d() + yoff, Y->lda, X->nrows, ncols);
+  launch_pdl(k_copy<T, T>, grid_for((int64_t)X->nrows * ncols), 256, 0, (const T*)(X->d() + xoff), X->lda,
+             Y->d() + yoff, Y->lda, (int64_t)X->nrows, ncols);
   PB_LAUNCH_CHECK();
 }
 
@@ -761,7 +761,7 @@ void launch_spmv_nv(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p, 
         static std::atomic<int> occ32{0};
         auto kern = pf_kernel<T, NV, TPR, NT, false, 32>();
         const int pgrid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rt().num_sms() * resident(kern, occ32)));
-        kern<<<pgrid, NT, 0, stream()>>>(S, p);
+        launch_pdl(kern, pgrid, NT, 0, S, p);
         PB_LAUNCH_CHECK();
         return;
       }
@@ -769,7 +769,7 @@ void launch_spmv_nv(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p, 
     static std::atomic<int> occ{0};
     auto kern = pf_kernel<T, NV, TPR, NT>();
     const int pgrid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rt().num_sms() * resident(kern, occ)));
-    kern<<<pgrid, NT, 0, stream()>>>(S, p);
+    launch_pdl(kern, pgrid, NT, 0, S, p);
     PB_LAUNCH_CHECK();
     return;
   }
@@ -782,12 +782,12 @@ void launch_spmv_nv(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p, 
     const int lgrid = (int)ceil_div(npad > 0 ? npad : 1, NT / TPR);
     if constexpr ((NV / TPR) * sizeof(T) >= 32) {
       if (v256) {
-        k_sell_spmmv_long<T, NV, TPR, NT, 32, false><<<lgrid, NT, 0, stream()>>>(S, p);
+        launch_pdl(k_sell_spmmv_long<T, NV, TPR, NT, 32, false>, lgrid, NT, 0, S, p);
         PB_LAUNCH_CHECK();
         return;
       }
     }
-    k_sell_spmmv_long<T, NV, TPR, NT, 16, false><<<lgrid, NT, 0, stream()>>>(S, p);
+    launch_pdl(k_sell_spmmv_long<T, NV, TPR, NT, 16, false>, lgrid, NT, 0, S, p);
     PB_LAUNCH_CHECK();
     return;
   }
@@ -821,9 +821,9 @@ void launch_spmv_any(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p)
     }
     const int64_t ntiles = ceil_div(A->nchunks, RPB / 32);
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rt().num_sms() * occ.load()));
-    kern<<<grid, NT, 0, stream()>>>(S, p);
+    launch_pdl(kern, grid, NT, 0, S, p);
   } else {
-    k_sell_spmmv_long<T, NV, TPR, NT, VB, true><<<(int)ceil_div(A->nchunks * 32, RPB), NT, 0, stream()>>>(S, p);
+    launch_pdl(k_sell_spmmv_long<T, NV, TPR, NT, VB, true>, (int)ceil_div(A->nchunks * 32, RPB), NT, 0, S, p);
   }
   PB_LAUNCH_CHECK();
 }
@@ -931,7 +931,7 @@ void launch_spmv_gram_nv(const SparseMat<T>* A, SpmvArgs<T>& p, SdMat<T>* Gw, Sd
   T* part = (T*)rt().scratch(sizeof(T) * 2 * (size_t)grid * NV * NV);
   p.gram_w = Gw ? part : nullptr;
   p.gram_v = Gv ? part + (size_t)grid * NV * NV : nullptr;
-  kern<<<grid, NT, 0, stream()>>>(sell_dev(A), p);
+  launch_pdl(kern, grid, NT, 0, sell_dev(A), p);
   PB_LAUNCH_CHECK();
   const int rb = (int)ceil_div(NV * NV, 32);
   if (Gw) {

@@ -105,6 +105,8 @@ template <class TI, class TO>
 __global__ void k_copy(const TI* __restrict__ x, int64_t ldx, TO* y, int64_t ldy, int64_t n,
                        int nvec)
 {
+  pdl_begin();
+  pdl_wait();
   PB_FOR_ELEMS(n, nvec, i, j) y[i * ldy + j] = TO(x[i * ldx + j]);
 }
 

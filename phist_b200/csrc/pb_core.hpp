@@ -257,6 +257,27 @@ inline cudaStream_t stream() { return rt().stream(); }
     PB_CUDA(cudaGetLastError());                 \
   } while (0)
 
+// Launch with a programmatic dependency on the previous kernel of the stream:
+// the blocks may start while that kernel drains, do what does not depend on
+// it and wait in pdl_wait() (pb_reduce.cuh) for its end and its memory.  Only
+// for kernels that call pdl_wait() before they touch anything a kernel writes.
+template <class... KA, class... A>
+inline void launch_pdl(void (*kern)(KA...), int grid, int block, size_t smem, const A&... args)
+{
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream();
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  PB_CUDA(cudaLaunchKernelEx(&cfg, kern, KA(args)...));
+}
+
 // ---------------------------------------------------------------- objects
 struct Comm {
   int rank = 0;

@@ -55,7 +55,7 @@ void tn_launch(FragTnArgs<T>& a)
   const int ngrp = (int)ceil_div(grid, a.gsz);
   a.part = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ngrp) * a.m * a.k);
   a.counters = rt().counters();
-  kern<<<grid, FRAG_BS, 0, stream()>>>(a);
+  launch_pdl(kern, grid, FRAG_BS, 0, a);
   PB_LAUNCH_CHECK();
 }
 
@@ -95,7 +95,7 @@ void nn_launch(const FragNnArgs<T>& a)
   static std::atomic<int> occ{0};
   const int64_t want = ceil_div(a.n, 8 * RT * FRAG_NW);
   const int grid = (int)std::min<int64_t>(want, (int64_t)rt().num_sms() * frag_occ(kern, occ));
-  kern<<<grid, FRAG_BS, 0, stream()>>>(a);
+  launch_pdl(kern, grid, FRAG_BS, 0, a);
   PB_LAUNCH_CHECK();
 }
 
@@ -126,7 +126,7 @@ void nn_gram_launch(const FragNnArgs<T>& a, FragTnArgs<T>& go)
   go.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
   go.part = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ceil_div(grid, go.gsz)) * a.k * a.k);
   go.counters = rt().counters();
-  kern<<<grid, FRAG_BS, 0, stream()>>>(a, go);
+  launch_pdl(kern, grid, FRAG_BS, 0, a, go);
   PB_LAUNCH_CHECK();
 }
 
@@ -150,7 +150,7 @@ void prec_launch(MvTmvPrecArgs& a)
   a.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
   a.part = (double*)rt().scratch(2 * sizeof(double) * (size_t)(grid + ceil_div(grid, a.gsz)) * a.m * a.k);
   a.counters = rt().counters();
-  k_mvTmv_prec<MT, TJ><<<grid, FRAG_BS, 0, stream()>>>(a);
+  launch_pdl(k_mvTmv_prec<MT, TJ>, grid, FRAG_BS, 0, a);
   PB_LAUNCH_CHECK();
 }
 

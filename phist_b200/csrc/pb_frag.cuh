@@ -255,6 +255,8 @@ __device__ __forceinline__ void frag_finish(const FragTnArgs<T>& a, const double
 template <class T, int MT, int KT, bool SYM, bool VEC, int U>
 __global__ void __launch_bounds__(FRAG_BS, 2) k_tn_frag(const __grid_constant__ FragTnArgs<T> a)
 {
+  pdl_begin();
+  pdl_wait();
   static_assert(!SYM || MT == KT, "a symmetric product is square");
   constexpr int NTILE = SYM ? MT * (MT + 1) / 2 : MT * KT;
   __shared__ double red[frag_red<MT, KT>()];
@@ -354,6 +356,8 @@ __device__ __forceinline__ void frag_nn_load(const FragNnArgs<T>& a, int64_t ch,
 template <class T, int MC, int KT, bool VEC, int RT>
 __global__ void __launch_bounds__(FRAG_BS, 2) k_nn_frag(const __grid_constant__ FragNnArgs<T> a)
 {
+  pdl_begin();
+  pdl_wait();
   constexpr int KS = 2 * MC;  // steps of 4 columns of V
   __shared__ double sC[KS * KT * 32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -418,6 +422,8 @@ template <class T, int MC, int KT, bool VEC, int RT>
 __global__ void __launch_bounds__(FRAG_BS, (MC * KT > 6 ? 1 : 2))
 k_nn_gram_frag(const __grid_constant__ FragNnArgs<T> a, const __grid_constant__ FragTnArgs<T> go)
 {
+  pdl_begin();
+  pdl_wait();
   constexpr int KS = 2 * MC, P = KT * 8 + 4;
   constexpr int NC = KS * KT * 32, NTL = FRAG_NW * 8 * P, NRED = frag_red<KT, KT>();
   constexpr int NTILE = KT * (KT + 1) / 2;

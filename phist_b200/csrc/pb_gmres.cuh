@@ -127,7 +127,7 @@ void kry_launch(KryArgs<T>& a)
   a.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
   a.part = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ceil_div(grid, a.gsz)) * KRY_MAXOUT);
   a.counters = rt().counters();
-  k_kry<T, MQ, MJ, UPD, DOTS><<<grid, FRAG_BS, 0, stream()>>>(a);
+  launch_pdl(k_kry<T, MQ, MJ, UPD, DOTS>, grid, FRAG_BS, 0, a);
   PB_LAUNCH_CHECK();
 }
 
@@ -290,7 +290,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
       a.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
       a.part = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ceil_div(grid, a.gsz)) * KRY_MAXOUT);
       a.counters = rt().counters();
-      k_kry_start<T><<<grid, FRAG_BS, 0, stream()>>>(a);
+      launch_pdl(k_kry_start<T>, grid, FRAG_BS, 0, a);
       PB_LAUNCH_CHECK();
     });
     hflags[1] = 0;

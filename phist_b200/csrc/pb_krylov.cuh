@@ -306,6 +306,8 @@ __device__ __forceinline__ void kry_finish(const KryArgs<T>& a, int nqo, int nbo
 template <class T, int MQ, int MJ, bool UPD, bool DOTS>
 __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryArgs<T> a)
 {
+  pdl_begin();
+  pdl_wait();
   if (a.skip && *a.skip == 0) return;
   constexpr int UB = MJ <= 2 ? 4 : MJ <= 8 ? 2 : 1;  // packed steps of loads in flight
   constexpr int MQ1 = MQ > 0 ? MQ : 1;
@@ -423,6 +425,8 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
 template <class T>
 __global__ void __launch_bounds__(FRAG_BS) k_kry_start(const __grid_constant__ KryArgs<T> a)
 {
+  pdl_begin();
+  pdl_wait();
   __shared__ double sm[KRY_RED];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int kc = a.kc, kp = a.kp, k = a.k;

@@ -130,6 +130,8 @@ __device__ __forceinline__ bool prec_tree_sum(double* part, int nout, int gsz, u
 template <int MT, int TJ>
 __global__ void __launch_bounds__(FRAG_BS, 2) k_mvTmv_prec(const __grid_constant__ MvTmvPrecArgs a)
 {
+  pdl_begin();
+  pdl_wait();
   constexpr int U = MT <= 2 ? 8 : MT <= 4 ? 4 : 2;  // rows of loads in flight
   constexpr int NO = MT * TJ * 32;                  // outputs, padded
   constexpr int NQ = (NO + FRAG_BS - 1) / FRAG_BS;

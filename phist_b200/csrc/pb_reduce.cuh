@@ -14,6 +14,12 @@
 
 namespace pb {
 
+// Programmatic dependencies (launch_pdl): pdl_begin() lets the next kernel of
+// the stream start its blocks once all blocks of this one run; pdl_wait()
+// waits for the previous kernel.  Both do nothing in an ordinary launch.
+__device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <class T>
 struct Acc;  // accumulation type
 template <>

@@ -279,8 +279,12 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
     }
   };
 
+  // the matrix is read before the wait for the previous kernel: nothing on
+  // the stream writes it
+  pdl_begin();
   int64_t t = blockIdx.x;
   if (t >= ntiles) {
+    pdl_wait();
     if constexpr (GRAM) gram.store(p, gys);
     return;
   }
@@ -294,6 +298,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
     __syncthreads();
     copy_entries(t, 0, 0);
     cp_async_commit();
+    pdl_wait();
     cp_async_wait<0>();
     __syncthreads();
   }
@@ -492,6 +497,7 @@ __global__ void __launch_bounds__(NT) k_sell_spmmv_long(SellDev<T> A, SpmvArgs<T
   constexpr int KB = VPT * (int)sizeof(T) <= 32 ? 8 : 4;
   static_assert(VPT % VW == 0, "bad column split");
   typedef typename Acc<T>::type AT;
+  pdl_begin();
   const int s = threadIdx.x % TPR;
   const int64_t r = blockIdx.x * (int64_t)RPB + threadIdx.x / TPR;  // SELL row
   if (r >= A.nchunks * (int64_t)CC) return;
@@ -519,6 +525,7 @@ __global__ void __launch_bounds__(NT) k_sell_spmmv_long(SellDev<T> A, SpmvArgs<T
 #pragma unroll
   for (int q = 0; q < VPT; q++) acc[q] = AT(0);
   if (len > 0) entries(0);
+  pdl_wait();  // the matrix does not depend on earlier kernels
   if (i >= 0 && p.has_shift) {
     T xs[VPT];
 #pragma unroll
