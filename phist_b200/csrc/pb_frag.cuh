@@ -107,34 +107,37 @@ __device__ __forceinline__ bool frag_tree_sum(double* part, int nout, int gsz, u
   const int nb = gridDim.x, tid = threadIdx.x;
   const int grp = blockIdx.x / gsz, ngrp = (nb + gsz - 1) / gsz;
   const int b0 = grp * gsz, cnt = min(gsz, nb - b0);
+  // one thread's fence after the barrier covers the block's writes
   auto arrive = [&](unsigned int* c, int total) {
-    __threadfence();
     __syncthreads();
     if (tid == 0) {
+      __threadfence();
       last = (atomicAdd(c, 1u) == (unsigned)total - 1);
       if (last) *c = 0u;  // ready for the next launch
+      __threadfence();
     }
     __syncthreads();
-    if (last) __threadfence();
     return last != 0;
   };
-  // all outputs of a thread together, 4 partials of each in flight
+  // all outputs of a thread together, B partials of each in flight (a level is
+  // 17 to 25 long: two rounds of loads)
+  constexpr int B = NQ == 1 ? 16 : NQ == 2 ? 12 : 4;
   auto sum = [&](const double* p, int count) {
 #pragma unroll
     for (int q = 0; q < NQ; q++) tot[q] = 0.0;
-    for (int b = 0; b < count; b += 4) {
-      double v[NQ][4];
+    for (int b = 0; b < count; b += B) {
+      double v[NQ][B];
 #pragma unroll
       for (int q = 0; q < NQ; q++)
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
+        for (int u = 0; u < B; u++) {
           const int o = tid + q * FRAG_BS;
           v[q][u] = (b + u < count && o < nout) ? __ldcg(p + (int64_t)(b + u) * nout + o) : 0.0;
         }
 #pragma unroll
       for (int q = 0; q < NQ; q++)
 #pragma unroll
-        for (int u = 0; u < 4; u++) tot[q] += v[q][u];
+        for (int u = 0; u < B; u++) tot[q] += v[q][u];
     }
   };
   if (!arrive(counters + 1 + grp, cnt)) return false;

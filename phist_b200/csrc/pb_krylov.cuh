@@ -295,7 +295,13 @@ __device__ __forceinline__ void kry_finish(const KryArgs<T>& a, int nqo, int nbo
       a.part[(int64_t)blockIdx.x * nout + o] = tot[q];
     }
   }
-  if (!frag_tree_sum<2>(a.part, nout, a.gsz, a.counters, tot)) return;
+  if (nout <= FRAG_BS) {
+    double one[1] = {tot[0]};
+    if (!frag_tree_sum<1>(a.part, nout, a.gsz, a.counters, one)) return;
+    tot[0] = one[0];
+  } else if (!frag_tree_sum<2>(a.part, nout, a.gsz, a.counters, tot)) {
+    return;
+  }
 #pragma unroll
   for (int q = 0; q < 2; q++)
     if (tid + q * FRAG_BS < nout) sm[tid + q * FRAG_BS] = tot[q];
@@ -309,9 +315,11 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
   pdl_begin();
   pdl_wait();
   if (a.skip && *a.skip == 0) return;
-  constexpr int UB = MJ <= 2 ? 4 : MJ <= 8 ? 2 : 1;  // packed steps of loads in flight
+  // packed steps, 4-row steps of Q'W and row tiles of Q cq with their loads in flight
+  constexpr int UB = MJ <= 2 ? 4 : sizeof(T) == 4 ? (MJ <= 8 ? 4 : 2) : (MJ <= 8 ? 2 : 1);
+  constexpr int QU = sizeof(T) == 4 ? 8 : 4;
   constexpr int MQ1 = MQ > 0 ? MQ : 1;
-  constexpr int RTB = MQ <= 2 ? 4 : 2;               // row tiles of Q in flight
+  constexpr int RTB = MQ <= 2 ? 4 : 2;
   __shared__ double sm[KRY_RED];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
   const int kc = a.kc, kp = a.kp, k = a.k, nb = a.nb, nq = a.nq;
@@ -341,13 +349,13 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
   for (int64_t ch = blockIdx.x * (int64_t)FRAG_NW + w; ch < nch; ch += GW) {
     const int64_t r0 = ch * 32;
     if (MQ > 0 && !UPD && DOTS) {
-      // Q'W: 4-row steps, half of the chunk's loads at a time
+      // Q'W: 4-row steps
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        T qv[4][MQ1], wv[4];
+      for (int h = 0; h < 8; h += QU) {
+        T qv[QU][MQ1], wv[QU];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int64_t row = r0 + 16 * h + 4 * u + t;
+        for (int u = 0; u < QU; u++) {
+          const int64_t row = r0 + 4 * (h + u) + t;
           const bool ok = row < a.n;
           const T* pq = a.Q + (ok ? row : 0) * a.ldq;
 #pragma unroll
@@ -355,7 +363,7 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
           kry_ldp(a.W + (ok ? row : 0) * k + min(g, kc - 1), ok, wv[u]);
         }
 #pragma unroll
-        for (int u = 0; u < 4; u++)
+        for (int u = 0; u < QU; u++)
 #pragma unroll
           for (int i = 0; i < MQ; i++) dmma_884(qa[i][0], qa[i][1], (double)qv[u][i], (double)wv[u]);
       }

@@ -82,25 +82,26 @@ __device__ __forceinline__ bool prec_tree_sum(double* part, int nout, int gsz, u
   const int grp = blockIdx.x / gsz, ngrp = (nb + gsz - 1) / gsz;
   const int b0 = grp * gsz, cnt = min(gsz, nb - b0);
   auto arrive = [&](unsigned int* ctr, int total) {
-    __threadfence();
     __syncthreads();
     if (tid == 0) {
+      __threadfence();
       last = (atomicAdd(ctr, 1u) == (unsigned)total - 1);
       if (last) *ctr = 0u;  // ready for the next launch
+      __threadfence();
     }
     __syncthreads();
-    if (last) __threadfence();
     return last != 0;
   };
+  constexpr int B = NQ == 1 ? 12 : 6;
   auto sum = [&](const double* p, int count) {
 #pragma unroll
     for (int q = 0; q < NQ; q++) s[q] = c[q] = 0.0;
-    for (int b = 0; b < count; b += 4) {
-      double2 v[NQ][4];
+    for (int b = 0; b < count; b += B) {
+      double2 v[NQ][B];
 #pragma unroll
       for (int q = 0; q < NQ; q++)
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
+        for (int u = 0; u < B; u++) {
           const int o = tid + q * FRAG_BS;
           v[q][u] = make_double2(0.0, 0.0);
           if (b + u < count && o < nout)
@@ -109,7 +110,7 @@ __device__ __forceinline__ bool prec_tree_sum(double* part, int nout, int gsz, u
 #pragma unroll
       for (int q = 0; q < NQ; q++)
 #pragma unroll
-        for (int u = 0; u < 4; u++) dd_add(s[q], c[q], v[q][u].x, v[q][u].y);
+        for (int u = 0; u < B; u++) dd_add(s[q], c[q], v[q][u].x, v[q][u].y);
     }
   };
   auto put = [&](int64_t slot) {
