@@ -280,7 +280,9 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_tn_frag(const __grid_constant__ 
   const int64_t nch = a.n / (4 * U);
   const int64_t gw = blockIdx.x * (int64_t)FRAG_NW + w, GW = gridDim.x * (int64_t)FRAG_NW;
   for (int64_t c = gw; c < nch; c += GW) {
-    const int64_t r = c * (4 * U) + t;
+    // from the last rows to the first: what the kernel before this one (rows
+    // in ascending order) touched last is still in the L2
+    const int64_t r = (nch - 1 - c) * (4 * U) + t;
     const T* pv = a.V + r * a.ldv;
     const T* pw = a.W + r * a.ldw;
     T v[U][MT], wv[U][KT];

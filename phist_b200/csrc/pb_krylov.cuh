@@ -347,7 +347,9 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
   for (int i = 0; i < MJ; i++) va[i] = T(0);
   const int64_t nch = (a.n + 31) / 32, GW = gridDim.x * (int64_t)FRAG_NW;
   for (int64_t ch = blockIdx.x * (int64_t)FRAG_NW + w; ch < nch; ch += GW) {
-    const int64_t r0 = ch * 32;
+    // dots go from the last rows to the first, updates the other way: each
+    // pass begins with the rows that the one before it left in the L2
+    const int64_t r0 = (UPD ? ch : nch - 1 - ch) * 32;
     if (MQ > 0 && !UPD && DOTS) {
       // Q'W: 4-row steps
 #pragma unroll

@@ -153,7 +153,8 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_mvTmv_prec(const __grid_constant
   for (int e = 0; e < TJ; e++) cj[e] = min(lj * TJ + e, a.k - 1);
   const int64_t nch = (a.n + U - 1) / U;
   const int64_t GW = gridDim.x * (int64_t)FRAG_NW;
-  for (int64_t ch = blockIdx.x * (int64_t)FRAG_NW + w; ch < nch; ch += GW) {
+  for (int64_t cc = blockIdx.x * (int64_t)FRAG_NW + w; cc < nch; cc += GW) {
+    const int64_t ch = nch - 1 - cc;  // descending, as k_tn_frag
     double x[U][MT], y[U][TJ];
 #pragma unroll
     for (int u = 0; u < U; u++) {
