@@ -140,6 +140,33 @@ __device__ __forceinline__ bool frag_tree_sum(double* part, int nout, int gsz, u
         for (int u = 0; u < B; u++) tot[q] += v[q][u];
     }
   };
+  if (nout <= FRAG_BS && nout * nb <= 20 * FRAG_BS) {
+    // few outputs: one level, the blocks of an output split over G threads
+    // whose sums meet in a fixed tree
+    if (!arrive(counters, nb)) return false;
+    __shared__ double red1[FRAG_BS];
+    const int G = FRAG_BS / nout, q = tid / nout, o = tid - q * nout;
+    double s = 0.0;
+    if (q < G)
+      for (int b = q; b < nb; b += 8 * G) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = b + u * G < nb ? __ldcg(part + (int64_t)(b + u * G) * nout + o) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; u++) s += v[u];
+      }
+    red1[tid] = s;
+    __syncthreads();
+    int P = 1;
+    while (2 * P <= G) P *= 2;
+    if (q < G - P) red1[tid] += red1[tid + P * nout];
+    for (int h = P / 2; h >= 1; h >>= 1) {
+      __syncthreads();
+      if (q < h) red1[tid] += red1[tid + h * nout];
+    }
+    tot[0] = red1[tid];  // nout <= FRAG_BS: outputs o < nout are in thread o
+    return true;
+  }
   if (!arrive(counters + 1 + grp, cnt)) return false;
   sum(part + (int64_t)b0 * nout, cnt);
 #pragma unroll

@@ -218,7 +218,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
   DBuf<int> conv(k), jcount(k), reorth(ngrp);
   std::vector<T> negsig(k);
   for (int s = 0; s < k; s++) negsig[s] = (T)(-sigma[s]);
-  volatile int* hflags = (volatile int*)rt().mailbox_host();
+  volatile unsigned long long* hflags = (volatile unsigned long long*)rt().mailbox_host();
   const int gw = grid_for(n * (int64_t)k);
   // a projection block of at most KRY_MAXQ columns goes with the passes over
   // the basis, a wider one in products of its own
@@ -246,7 +246,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
     e.F = F.p; e.cq = Cq.p; e.hv = hv.p; e.hv2 = hv2.p; e.finv = f.p;
     e.conv = conv.p; e.jcount = jcount.p;
     e.eps_abs = eps_abs;
-    e.flags = (int*)rt().mailbox_dev();
+    e.flags = (unsigned long long*)rt().mailbox_dev();
     for (int s = 0; s < k; s++) {
       base.idx.v[s] = resIndex ? resIndex[s] : s;
       e.tol.v[s] = tol[s];
@@ -293,8 +293,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
       launch_pdl(k_kry_start<T>, grid, FRAG_BS, 0, a);
       PB_LAUNCH_CHECK();
     });
-    hflags[1] = 0;
-    hflags[0] = -1;
+    *hflags = 0;
     int j = 0, steps = 0;
     const int jmax = std::min(m, maxIter - total);
     bool stop = false;
@@ -364,12 +363,12 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
       // stop launching once the device reports every system converged (a
       // look at the flags, no wait: the host never blocks inside a cycle,
       // so concurrent solves on other threads keep their cores)
-      if (hflags[0] >= 0 && hflags[1] >= k) stop = true;
+      if ((int)(*hflags >> 32) >= k) stop = true;
     }
     total += steps;
     // x += [V_0..V_{J-1}] y with J the largest step count of a system
     rt().sync();
-    nconv = hflags[1];
+    nconv = (int)(*hflags >> 32);
     const int J = steps;
     k_gm_solve<T><<<1, 32 * k, 0, stream()>>>(H.p, g.p, jcount.p, k, m, J, F.p, Y.p);
     PB_LAUNCH_CHECK();

@@ -69,7 +69,7 @@ struct KryEpi {
   int *conv, *jcount, *reorth;
   double eps_abs;
   GmTol tol;
-  volatile int* flags;        // mapped host memory: step, converged systems
+  volatile unsigned long long* flags;  // mapped host memory: converged systems << 32 | steps done
 };
 
 template <class T>
@@ -113,6 +113,14 @@ __device__ __forceinline__ void kry_step(const KryEpi<T>& e, int kc, const doubl
   double* sh = sm;
   double* sc = sm + 64 * KRY_MAXC;
   double* ss = sc + 64 * KRY_MAXC;
+  // what the chain of a system needs beside the rotations, loaded with them
+  double gj = 0.0, bn = 0.0;
+  int done = 0;
+  if (tid < kc) {
+    gj = __ldcg(&e.g[j * k + e.c0 + tid]);
+    bn = __ldcg(&e.bnorm[e.c0 + tid]);
+    done = __ldcg(&e.conv[e.c0 + tid]);
+  }
   __syncthreads();
   for (int q = tid; q < (j + 1 - lo) * kc; q += FRAG_BS) {
     const int i = lo + q / kc, c = q % kc, s = e.c0 + c;
@@ -141,29 +149,27 @@ __device__ __forceinline__ void kry_step(const KryEpi<T>& e, int kc, const doubl
     sh[j * kc + c] = r;
     e.cs[j * k + s] = co;
     e.sn[j * k + s] = si;
-    const double gj = e.g[j * k + s];
     const double gn = -si * gj;
     e.g[j * k + s] = co * gj;
     e.g[(j + 1) * k + s] = gn;
-    if (!e.conv[s]) {
+    if (!done) {
       e.jcount[s] = j + 1;
       const double res = fabs(gn);
-      if (res < e.eps_abs || (e.bnorm[s] > 0.0 && res / e.bnorm[s] < e.tol.v[s])) e.conv[s] = 1;
+      if (res < e.eps_abs || (bn > 0.0 && res / bn < e.tol.v[s])) e.conv[s] = done = 1;
     }
     e.nf[s] = n2;
     e.F[(j + 1) * k + s] = (hn > 0.0) ? (T)(1.0 / hn) : T(0);
   }
-  __syncthreads();
+  int nconv = __syncthreads_count(tid < kc && done);
   for (int q = tid; q < (j + 1 - lo) * kc; q += FRAG_BS) {
     const int i = lo + q / kc, c = q % kc;
     e.H[((int64_t)i * m + j) * k + e.c0 + c] = sh[i * kc + c];
   }
   if (tid == 0 && e.last) {
-    int nconv = 0;
-    for (int s = 0; s < k; s++) nconv += e.conv[s] ? 1 : 0;
-    e.flags[1] = nconv;
-    __threadfence_system();
-    e.flags[0] = j;
+    for (int s = 0; s < k; s++)
+      if (s < e.c0 || s >= e.c0 + kc) nconv += __ldcg(&e.conv[s]) ? 1 : 0;
+    // step and count in one store: the host reads them together
+    *e.flags = ((unsigned long long)(unsigned)nconv << 32) | (unsigned)(j + 1);
   }
 }
 
