@@ -45,6 +45,7 @@
 
 #include "pb_api.cuh"
 #include "pb_krylov.cuh"
+#include "pb_spmmv_lz.cuh"
 
 namespace pb {
 namespace {
@@ -161,6 +162,54 @@ void kry_update(KryArgs<T>& a)
   } else if (a.nb <= 8) kry_launch<T, 0, 8, true, false>(a);
   else if (a.nb <= 16) kry_launch<T, 0, 16, true, false>(a);
   else kry_launch<T, 0, KRY_MAXJ, true, false>(a);
+}
+
+// W = (A - sigma I) V_j F_j with Q'W and V_j'W (pb_spmmv_lz.cuh): 4 or 8
+// systems whose rows are one 16- or 32-byte vector a thread, rows of at most 8
+// entries, at most 16 projection columns.  False otherwise.
+template <class T, int NV>
+bool spmv_lanczos_nv(const SparseMat<T>* A, const T* negsig, const Mvec<T>* X, Mvec<T>* W, const T* cscale,
+                     KryArgs<T>& a)
+{
+  constexpr int TPR = 2, VB = NV / TPR * (int)sizeof(T);
+  if (((uintptr_t)X->d() | (uintptr_t)W->d()) % VB != 0) return false;
+  SpmvArgs<T> p;
+  memset(&p, 0, sizeof(p));
+  p.alpha = T(1);
+  p.x = X->d();
+  p.ldx = X->lda;
+  p.y = W->d();
+  p.ldy = W->lda;
+  p.nvec = NV;
+  p.cscale = cscale;
+  p.has_shift = 1;
+  for (int s = 0; s < NV; s++) p.sh[s] = negsig[s];
+  auto kern = k_sell_spmmv_lz<T, NV, TPR, VB>;
+  static std::atomic<int> occ{0};
+  int o = occ.load();
+  if (o == 0) {
+    PB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, LZ_NT, 0));
+    o = std::max(1, o);
+    occ.store(o);
+  }
+  const int grid = (int)std::min<int64_t>(ceil_div(A->nchunks, LZ_NT / TPR / 32), (int64_t)rt().num_sms() * o);
+  a.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
+  a.part = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ceil_div(grid, a.gsz)) * KRY_MAXOUT);
+  a.counters = rt().counters();
+  launch_pdl(kern, grid, LZ_NT, 0, sell_dev(A), p, a);
+  PB_LAUNCH_CHECK();
+  return true;
+}
+
+template <class T>
+bool spmv_lanczos(const SparseMat<T>* A, const T* negsig, const Mvec<T>* X, Mvec<T>* W, const T* cscale,
+                  KryArgs<T>& a)
+{
+  if (!rt().spmv_pf || !rt().spmv_v256 || A->C != 32 || A->max_row_len > 8 || A->nnz == 0) return false;
+  if (a.nq < 1 || a.nq > LZ_MAXQ) return false;
+  if (a.k == 8) return spmv_lanczos_nv<T, 8>(A, negsig, X, W, cscale, a);
+  if (a.k == 4) return spmv_lanczos_nv<T, 4>(A, negsig, X, W, cscale, a);
+  return false;
 }
 
 }  // namespace
@@ -302,8 +351,18 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
       T* Wj = V.p + (int64_t)(j + 1) * nk;
       raw_view(mVj, V.p + (int64_t)j * nk, n, k, k);
       raw_view(mW, Wj, n, k, k);
-      spmv_general<T>(T(1), A, negsig.data(), &mVj, T(0), &mW, nullptr, nullptr, T(0), T(0), nullptr,
-                      F.p + (int64_t)j * k);
+      bool dotted = false;  // Q'W and V_j'W came with the SpMMV
+      if (lanczos && fuse && ngrp == 1) {
+        for_groups([&](KryArgs<T>& a, int) {
+          a.nq = nq;
+          a.e.j = j;
+          a.e.kind = KE_LZ;
+          dotted = spmv_lanczos<T>(A, negsig.data(), &mVj, &mW, F.p + (int64_t)j * k, a);
+        });
+      }
+      if (!dotted)
+        spmv_general<T>(T(1), A, negsig.data(), &mVj, T(0), &mW, nullptr, nullptr, T(0), T(0), nullptr,
+                        F.p + (int64_t)j * k);
       if (!fuse) project(Wj);
       const int J = j + 1;
       for_groups([&](KryArgs<T>& a0, int c0) {
@@ -333,7 +392,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
           // [Q V_j]'W; W -= Q (Q'W) + v_j alpha + v_{j-1} beta and its norm
           // (alpha = v_j'W equals v_j'(P W) because V_j is orthogonal to Q;
           // PHIST's order: projection, then the Lanczos terms)
-          pass(false, true, j, 1, true, nullptr, KE_LZ, true, nullptr);
+          if (!dotted) pass(false, true, j, 1, true, nullptr, KE_LZ, true, nullptr);
           pass(true, false, j, j > 0 ? 2 : 1, true, hv.p, KE_STEP, lastg, nullptr);
           return;
         }

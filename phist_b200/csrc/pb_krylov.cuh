@@ -254,15 +254,47 @@ constexpr int KRY_SH = KRY_SC + 2 * (KRY_MAXQ / 8) * 32;        // coefficients 
 static_assert(KRY_SH + KRY_MAXJ * KRY_MAXC <= KRY_RED, "tiles fit the reduction buffer");
 static_assert(KRY_MAXOUT + 3 * 64 * KRY_MAXC <= KRY_RED, "epilogue scratch fits the reduction buffer");
 
-// after the row loop: the lanes' sums to the block's, the blocks' to the
-// totals, and the epilogue in the block that holds them
+// red: the warps' sums, stride apart; from there the
+// block's, the blocks' and, in the block that holds the totals, the epilogue
+// (sm: shared scratch for it, may be red)
+template <class T>
+__device__ __forceinline__ void kry_totals(const KryArgs<T>& a, int nqo, int nbo, const double* red, int stride,
+                                           double* sm)
+{
+  const int tid = threadIdx.x, nout = (nqo + nbo + 1) * a.kc;
+  __syncthreads();
+  double tot[2];
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int o = tid + q * FRAG_BS;
+    tot[q] = 0.0;
+    if (o < nout) {
+#pragma unroll
+      for (int b = 0; b < FRAG_NW; b++) tot[q] += red[b * stride + o];
+      a.part[(int64_t)blockIdx.x * nout + o] = tot[q];
+    }
+  }
+  if (nout <= FRAG_BS) {
+    double one[1] = {tot[0]};
+    if (!frag_tree_sum<1>(a.part, nout, a.gsz, a.counters, one)) return;
+    tot[0] = one[0];
+  } else if (!frag_tree_sum<2>(a.part, nout, a.gsz, a.counters, tot)) {
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < 2; q++)
+    if (tid + q * FRAG_BS < nout) sm[tid + q * FRAG_BS] = tot[q];
+  __syncthreads();
+  kry_epilogue<T>(a, nqo, nbo, sm, sm + KRY_MAXOUT);
+}
+
+// after the row loop: the lanes' sums to the warps'
 template <class T, int MQ, int MJ>
 __device__ __forceinline__ void kry_finish(const KryArgs<T>& a, int nqo, int nbo, double (&qa)[MQ > 0 ? MQ : 1][2],
                                            T (&va)[MJ], T na, double* sm)
 {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
   const int kc = a.kc, kp = a.kp, s = lane & (kp - 1);
-  const int nout = (nqo + nbo + 1) * kc;
   double nd = (double)na, vd[MJ];
 #pragma unroll
   for (int i = 0; i < MJ; i++) vd[i] = i < nbo ? (double)va[i] : 0.0;
@@ -289,30 +321,7 @@ __device__ __forceinline__ void kry_finish(const KryArgs<T>& a, int nqo, int nbo
       if (i < nbo) red[(nqo + i) * kc + s] = vd[i];
     red[(nqo + nbo) * kc + s] = nd;
   }
-  __syncthreads();
-  double tot[2];
-#pragma unroll
-  for (int q = 0; q < 2; q++) {
-    const int o = tid + q * FRAG_BS;
-    tot[q] = 0.0;
-    if (o < nout) {
-#pragma unroll
-      for (int b = 0; b < FRAG_NW; b++) tot[q] += sm[b * KRY_MAXOUT + o];
-      a.part[(int64_t)blockIdx.x * nout + o] = tot[q];
-    }
-  }
-  if (nout <= FRAG_BS) {
-    double one[1] = {tot[0]};
-    if (!frag_tree_sum<1>(a.part, nout, a.gsz, a.counters, one)) return;
-    tot[0] = one[0];
-  } else if (!frag_tree_sum<2>(a.part, nout, a.gsz, a.counters, tot)) {
-    return;
-  }
-#pragma unroll
-  for (int q = 0; q < 2; q++)
-    if (tid + q * FRAG_BS < nout) sm[tid + q * FRAG_BS] = tot[q];
-  __syncthreads();
-  kry_epilogue<T>(a, nqo, nbo, sm, sm + KRY_MAXOUT);
+  kry_totals<T>(a, nqo, nbo, sm, KRY_MAXOUT, sm);
 }
 
 template <class T, int MQ, int MJ, bool UPD, bool DOTS>

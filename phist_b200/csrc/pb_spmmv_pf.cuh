@@ -200,6 +200,12 @@ struct GramNone {
   __device__ __forceinline__ void init() {}
 };
 
+// What else a kernel does with the rows it forms (pb_spmmv_lz.cuh); this one
+// nothing.
+struct EpiNone {
+  static constexpr bool on = false;
+};
+
 template <class T, int NV, int NT, int RPB>
 struct GramPick {
   typedef GramScalar<T, NV, NT, RPB> type;
@@ -216,8 +222,8 @@ struct GramPick<double, NV, NT, RPB> {
 // ANY: p.nvec <= NV columns of any alignment that VB allows; a thread's
 // vectors past the last column read that column again (no predicate between
 // the gathers) and are not stored
-template <class T, int NV, int TPR, int NT, bool GRAM, int VB, bool ANY>
-__device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArgs<T>& p)
+template <class T, int NV, int TPR, int NT, bool GRAM, int VB, bool ANY, class Epi>
+__device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArgs<T>& p, Epi& epi)
 {
   constexpr int KMAX = 8, CC = 32;
   constexpr int VPT = NV / TPR;
@@ -286,6 +292,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
   if (t >= ntiles) {
     pdl_wait();
     if constexpr (GRAM) gram.store(p, gys);
+    if constexpr (Epi::on) epi.finish();
     return;
   }
   {
@@ -320,6 +327,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
           gxs[lr * PY + spmv_col<TPR, VW>(s, v, w)] = T(0);
         }
     }
+    if constexpr (Epi::on) epi.clear(lr);
     if (r < nch * (int64_t)CC) {
       const int64_t i = (r < A.nrows) ? (A.perm ? (int64_t)A.perm[r] : r) : -1;
       AT acc[VPT];
@@ -343,13 +351,12 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
         }
       } else {
         if (i >= 0 && p.has_shift) {
-          T xs[VPT];
 #pragma unroll
-          for (int v = 0; v < NVV; v++) Vec<T, VW>::ld(x + i * p.ldx + lcol(v), &xs[v * VW]);
+          for (int v = 0; v < NVV; v++) Vec<T, VW>::ld(x + i * p.ldx + lcol(v), &xi[v * VW]);
 #pragma unroll
           for (int v = 0; v < NVV; v++)
 #pragma unroll
-            for (int w = 0; w < VW; w++) acc[v * VW + w] = AT(p.sh[lcol(v) + w]) * AT(xs[v * VW + w]);
+            for (int w = 0; w < VW; w++) acc[v * VW + w] = AT(p.sh[lcol(v) + w]) * AT(xi[v * VW + w]);
         }
       }
       const int lc = lr / CC, l = lr % CC;
@@ -402,6 +409,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
             for (int w = 0; w < VW; w++) yv[w] = T(AT(p.alpha) * acc[v * VW + w]);
           }
           if (!GRAM || !p.no_store) Vec<T, VW>::st(yr + c, yv);
+          if constexpr (Epi::on) epi.template put<VW>(lr, i, v, c, yv, &xi[v * VW]);
           if constexpr (GRAM) {
 #pragma unroll
             for (int w = 0; w < VW; w++) {
@@ -417,11 +425,16 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
       __syncthreads();
       gram.add_tile(gys, gxs);
     }
+    if constexpr (Epi::on) {
+      __syncthreads();
+      epi.tile();
+    }
     cp_async_wait<0>();
     if (tid <= NCH) smeta[mbnn][tid] = mnext;
     __syncthreads();
   }
   if constexpr (GRAM) gram.store(p, gys);
+  if constexpr (Epi::on) epi.finish();
 }
 
 // The kernel comes in two entry points around the same body: with a minimum
@@ -445,13 +458,15 @@ constexpr int pf_min_blocks()
 template <class T, int NV, int TPR, int NT, bool GRAM = false, int VB = 16>
 __global__ void __launch_bounds__(NT) k_sell_spmmv_pf(SellDev<T> A, SpmvArgs<T> p)
 {
-  sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB, false>(A, p);
+  EpiNone none;
+  sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB, false>(A, p, none);
 }
 
 template <class T, int NV, int TPR, int NT, bool GRAM, int VB, int MB>
 __global__ void __launch_bounds__(NT, MB) k_sell_spmmv_pf_mb(SellDev<T> A, SpmvArgs<T> p)
 {
-  sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB, false>(A, p);
+  EpiNone none;
+  sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB, false>(A, p, none);
 }
 
 // Any width and alignment: NV >= p.nvec columns, TPR threads a row, vectors
@@ -465,7 +480,8 @@ constexpr int pf_any_blocks()
 template <class T, int NV, int TPR, int NT, int VB>
 __global__ void __launch_bounds__(NT, (pf_any_blocks<T, NV / TPR, NT>())) k_sell_spmmv_pf_any(SellDev<T> A, SpmvArgs<T> p)
 {
-  sell_spmmv_pf<T, NV, TPR, NT, false, VB, true>(A, p);
+  EpiNone none;
+  sell_spmmv_pf<T, NV, TPR, NT, false, VB, true>(A, p, none);
 }
 
 // the entry point of a form
