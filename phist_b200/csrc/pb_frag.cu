@@ -118,8 +118,8 @@ bool nn_mc(const FragNnArgs<T>& a)
 template <class T, int MC, int KT, bool VEC>
 void nn_gram_launch(const FragNnArgs<T>& a, FragTnArgs<T>& go)
 {
-  constexpr int RT = 2;
-  auto kern = k_nn_gram_frag<T, MC, KT, VEC, RT>;
+  constexpr int RT = nn_gram_rt<KT>();
+  auto kern = k_nn_gram_frag<T, MC, KT, VEC>;
   static std::atomic<int> occ{0};
   const int64_t want = ceil_div(a.n, 8 * RT * FRAG_NW);
   const int grid = (int)std::min<int64_t>(want, (int64_t)rt().num_sms() * std::min(3, frag_occ(kern, occ)));
@@ -201,8 +201,11 @@ void launch_mvTmv_prec(int64_t n, int m, int k, double alpha, const double* V, i
 }
 
 // Which products go here (us at n = 2,097,152, fragment | other kernel):
-//   * thin ones (at most 4 columns against 4, FP32 8) stay with the register
-//     kernel, one row per thread: FP32 3 x 3 36 | 25, FP64 4 x 4 45 | 39;
+//   * thin ones (at most 4 columns against 4, FP32 8) of many rows stay with
+//     the register kernel, one row per thread: FP32 3 x 3 33 | 25, FP64 4 x 4
+//     43 | 39; up to 2^20 rows the shorter cross-block sum decides (n =
+//     262,144, W'W of 4 columns 12.3 | 16.4), and for W'W of 2 to 4 FP64
+//     columns always (26.7 | 28.7);
 //   * W'W up to 32 columns: half the tiles, one read (see pb_frag.cuh);
 //   * blocks on 16-byte rows keep the TMA-staged kernels where those share
 //     every row among many tiles: 64 x 8 207 | 202, 64 x 16 269 | 222,
@@ -213,10 +216,11 @@ template <class T>
 bool frag_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const T* W, int64_t ldw, T beta, T* C,
                 int64_t ldc, T* mbox)
 {
-  if (n < 1 || m < 1 || k < 1 || m > 64 || k > 64) return false;
+  if (n < 0 || m < 1 || k < 1 || m > 64 || k > 64) return false;
   const bool sym = V == W && ldv == ldw && m == k;
   const int big = std::max(m, k), small = std::min(m, k);
-  if (small <= 4 && big <= (sizeof(T) == 4 ? 8 : 4)) return false;
+  const bool thin = small <= 4 && big <= (sizeof(T) == 4 ? 8 : 4);
+  if (thin && n > (1 << 20) && !(sym && sizeof(T) == 8 && m >= 2)) return false;
   const bool staged = rows16(V, ldv, m) && rows16(W, ldw, k);
   if (staged && (sym ? m > 32 : small > 8 ? big > 16 : big > 40)) return false;
   FragTnArgs<T> a;

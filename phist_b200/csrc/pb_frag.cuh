@@ -99,8 +99,8 @@ __device__ __forceinline__ void frag_st2(float* p, float a, float b)
 // group order.  Both levels are about sqrt(blocks) long, so two short rounds
 // of independent loads replace one long one (a single last block) or a
 // second launch.  True in the block that holds the totals: thread o (in
-// steps of the block size) has output o in tot[o / FRAG_BS].
-template <int NQ>
+// steps of the block size NTH) has output o in tot[o / NTH].
+template <int NQ, int NTH = FRAG_BS>
 __device__ __forceinline__ bool frag_tree_sum(double* part, int nout, int gsz, unsigned int* counters, double (&tot)[NQ])
 {
   __shared__ int last;
@@ -131,7 +131,7 @@ __device__ __forceinline__ bool frag_tree_sum(double* part, int nout, int gsz, u
       for (int q = 0; q < NQ; q++)
 #pragma unroll
         for (int u = 0; u < B; u++) {
-          const int o = tid + q * FRAG_BS;
+          const int o = tid + q * NTH;
           v[q][u] = (b + u < count && o < nout) ? __ldcg(p + (int64_t)(b + u) * nout + o) : 0.0;
         }
 #pragma unroll
@@ -140,12 +140,12 @@ __device__ __forceinline__ bool frag_tree_sum(double* part, int nout, int gsz, u
         for (int u = 0; u < B; u++) tot[q] += v[q][u];
     }
   };
-  if (nout <= FRAG_BS && nout * nb <= 20 * FRAG_BS) {
+  if (nout <= NTH && nout * nb <= 20 * NTH) {
     // few outputs: one level, the blocks of an output split over G threads
     // whose sums meet in a fixed tree
     if (!arrive(counters, nb)) return false;
-    __shared__ double red1[FRAG_BS];
-    const int G = FRAG_BS / nout, q = tid / nout, o = tid - q * nout;
+    __shared__ double red1[NTH];
+    const int G = NTH / nout, q = tid / nout, o = tid - q * nout;
     double s = 0.0;
     if (q < G)
       for (int b = q; b < nb; b += 8 * G) {
@@ -164,14 +164,14 @@ __device__ __forceinline__ bool frag_tree_sum(double* part, int nout, int gsz, u
       __syncthreads();
       if (q < h) red1[tid] += red1[tid + h * nout];
     }
-    tot[0] = red1[tid];  // nout <= FRAG_BS: outputs o < nout are in thread o
+    tot[0] = red1[tid];  // nout <= NTH: outputs o < nout are in thread o
     return true;
   }
   if (!arrive(counters + 1 + grp, cnt)) return false;
   sum(part + (int64_t)b0 * nout, cnt);
 #pragma unroll
   for (int q = 0; q < NQ; q++)
-    if (tid + q * FRAG_BS < nout) part[(int64_t)(nb + grp) * nout + tid + q * FRAG_BS] = tot[q];
+    if (tid + q * NTH < nout) part[(int64_t)(nb + grp) * nout + tid + q * NTH] = tot[q];
   if (!arrive(counters, ngrp)) return false;
   sum(part + (int64_t)nb * nout, ngrp);
   return true;
@@ -450,12 +450,22 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_nn_frag(const __grid_constant__ 
 // a warp has just formed go through its own shared-memory tile from the
 // result's fragment layout to the operands', and the tiles of W'W on and
 // above the diagonal are accumulated at once, so W is not read again.
-template <class T, int MC, int KT, bool VEC, int RT>
-__global__ void __launch_bounds__(FRAG_BS, (MC * KT > 6 ? 1 : 2))
+// RT row tiles in flight: 3 and one block per SM up to 16 columns, beyond (the
+// accumulators of W'W take the registers) 1 and two blocks (n = 2,097,152, us:
+// RT 1 / 2 / 3 at 8 columns 94 / 69 / 66, at 16 129 / 111 / 109, at 24 188 /
+// 210 / 213, at 32 266 / 278 / 270)
+template <int KT>
+constexpr int nn_gram_rt()
+{
+  return KT <= 2 ? 3 : 1;
+}
+template <class T, int MC, int KT, bool VEC>
+__global__ void __launch_bounds__(FRAG_BS, (KT <= 2 ? 1 : 2))
 k_nn_gram_frag(const __grid_constant__ FragNnArgs<T> a, const __grid_constant__ FragTnArgs<T> go)
 {
   pdl_begin();
   pdl_wait();
+  constexpr int RT = nn_gram_rt<KT>();
   constexpr int KS = 2 * MC, P = KT * 8 + 4;
   constexpr int NC = KS * KT * 32, NTL = FRAG_NW * 8 * P, NRED = frag_red<KT, KT>();
   constexpr int NTILE = KT * (KT + 1) / 2;

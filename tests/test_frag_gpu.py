@@ -62,6 +62,23 @@ def test_products(session, n, m, k, vo, vld, wo, wld, dtype):
         o.delete()
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("m,k", [(2, 3), (5, 4), (16, 16), (20, 17), (33, 33), (48, 8), (64, 64)])
+def test_no_rows(session, m, k, dtype):
+    """blocks without rows: the sum is empty, C = beta C"""
+    from phist_b200 import kernels as K
+    from phist_b200.objects import Map, Mvec, SdMat, fn
+    mp = Map(0)
+    V, W = Mvec(mp.h, m, dtype), Mvec(mp.h, k, dtype)
+    c0 = np.arange(m * k, dtype=dtype).reshape(m, k)
+    C = SdMat(m, k, dtype).set(c0)
+    K.chk(fn(dtype, "mvecT_times_mvec"), 1.0, V.h, W.h, 2.0, C.h)
+    assert np.array_equal(C.get(), 2 * c0)
+    K.chk(fn(dtype, "mvec_times_sdMat"), 1.0, V.h, C.h, 2.0, W.h)
+    for o in (V, W, C, mp):
+        o.delete()
+
+
 def test_infinity_stays_in_its_row(session):
     """an infinite entry in the last column meets no zero padding"""
     from phist_b200 import kernels as K
@@ -77,4 +94,33 @@ def test_infinity_stays_in_its_row(session):
     got = Wb.get()
     assert np.isposinf(got[7]).all() and np.isfinite(np.delete(got, 7, axis=0)).all()
     for o in (V, W, C, Vb, Wb, mp, mq):
+        o.delete()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("m,k,ld", [(5, 5, 5), (8, 8, 8), (13, 7, 17), (16, 16, 16), (24, 20, 24), (31, 31, 33), (32, 32, 32)])
+@pytest.mark.parametrize("n", [1, 130, 5003])
+def test_product_with_gram(session, n, m, k, ld, dtype):
+    """W = a V C + b W with W'W, and W = W C in place with W'W"""
+    from phist_b200 import kernels as K
+    from phist_b200.objects import SdMat, fn
+    rng = np.random.default_rng(n + m)
+    eps = np.finfo(dtype).eps
+    mp, Vb, V, v = _block(n, ld, 0, m, rng, dtype)
+    mq, Wb, W, w = _block(n, k, 0, k, rng, dtype)
+    c = (rng.uniform(-1, 1, (m, k)) / m).astype(dtype)
+    C, G = SdMat(m, k, dtype).set(c), SdMat(k, k, dtype)
+    K.chk(fn(dtype, "fused_mvsd_mvTmv"), 0.5, V.h, C.h, -0.5, W.h, G.h)
+    new = W.get().astype(np.float64)
+    assert np.abs(new - (0.5 * (v @ c.astype(np.float64)) - 0.5 * w)).max() <= (m + 3) * 2 * eps
+    g = G.get()
+    assert np.abs(g - new.T @ new).max() <= (n + 3) * (n * np.finfo(np.float64).eps + eps)
+    assert np.array_equal(g, g.T) and np.array_equal(G.host(), g)
+    X = Vb.view(0, k - 1)
+    D = SdMat(k, k, dtype).set(np.eye(k))
+    K.chk(fn(dtype, "fused_mvsdi_mvTmv"), 2.0, X.h, V.h, C.h, 1.0, D.h)
+    new = X.get().astype(np.float64)
+    assert np.abs(new - v @ c.astype(np.float64)).max() <= (m + 3) * 2 * eps
+    assert np.abs(D.get() - (2.0 * new.T @ new + np.eye(k))).max() <= 2 * (n + 3) * (n * np.finfo(np.float64).eps + eps)
+    for o in (X, D, V, W, C, G, Vb, Wb, mp, mq):
         o.delete()
