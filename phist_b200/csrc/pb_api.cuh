@@ -1187,15 +1187,24 @@ void mvtmv_async_launch(MvTmvArgs<T>& a, int64_t n)
   }
 }
 
+// the padded shapes that frag_mvTmv leaves to the staged kernels
+template <class T, int BM, int BK>
+void mvtmv_async_shape(MvTmvArgs<T>& a, int64_t n)
+{
+  constexpr int lo = BM < BK ? BM : BK, hi = BM < BK ? BK : BM;
+  if constexpr (hi == 64 || (hi == 32 && lo >= 16)) mvtmv_async_launch<T, BM, BK>(a, n);
+  else PB_REQUIRE(false, PB_NOT_IMPLEMENTED, "no staged product of %d x %d columns", a.m, a.k);
+}
+
 template <class T, int BM>
 void mvtmv_async_bk(MvTmvArgs<T>& a, int64_t n, int BK)
 {
   switch (BK) {
-    case 4: mvtmv_async_launch<T, BM, 4>(a, n); break;
-    case 8: mvtmv_async_launch<T, BM, 8>(a, n); break;
-    case 16: mvtmv_async_launch<T, BM, 16>(a, n); break;
-    case 32: mvtmv_async_launch<T, BM, 32>(a, n); break;
-    default: mvtmv_async_launch<T, BM, 64>(a, n); break;
+    case 4: mvtmv_async_shape<T, BM, 4>(a, n); break;
+    case 8: mvtmv_async_shape<T, BM, 8>(a, n); break;
+    case 16: mvtmv_async_shape<T, BM, 16>(a, n); break;
+    case 32: mvtmv_async_shape<T, BM, 32>(a, n); break;
+    default: mvtmv_async_shape<T, BM, 64>(a, n); break;
   }
 }
 
@@ -1329,28 +1338,24 @@ void gram_to_sdmat(const Mvec<T>* V, const Mvec<T>* W, int k, T alpha, T beta, S
 }
 
 // fused V*C + Gram on the tensor cores (FP64, widths 8..64 in steps of 8)
-template <int BM, int BK, int MV, int GM>
+template <int BM, int BK, int MV>
 bool mvsd_gram_dmma_launch(RowGemmArgs<double>& a)
 {
   constexpr int R = (BK >= 32 || MV >= 32) ? 64 : 128;
   constexpr int AP = BM + 4, CP = BK + 4, PT = BK + 4, PVG = MV + 4;
   constexpr int CSZ = (BM * CP * 8 + 127) / 128 * 128 / 8;
-  constexpr int VSZ = (GM == GM_VW) ? R * PVG : 0;
+  constexpr int VSZ = R * PVG;
   constexpr size_t BYTES3 = 8 * ((size_t)CSZ + 3 * (size_t)R * AP + 3 * (size_t)VSZ + (size_t)R * PT) + 24;
   constexpr int S = BYTES3 <= 200 * 1024 ? 3 : 2;
   const double* A = (a.mode == RM_MVSDI) ? (const double*)a.W : a.V;
   const int64_t lda = (a.mode == RM_MVSDI) ? a.ldw : a.ldv;
   CUtensorMap mA, mV;
   if (!make_rows_tmap<double>(&mA, A, a.n, a.m, lda, AP, R)) return false;
-  if (GM == GM_VW) {
-    if (!make_rows_tmap<double>(&mV, a.Vg, a.n, a.mv, a.ldvg, PVG, R)) return false;
-  } else {
-    mV = mA;
-  }
+  if (!make_rows_tmap<double>(&mV, a.Vg, a.n, a.mv, a.ldvg, PVG, R)) return false;
   const size_t smem = 8 * ((size_t)CSZ + (size_t)S * R * AP + (size_t)S * VSZ + (size_t)R * PT) + 8 * S;
   // one wave of as many blocks as fit an SM (shared memory allows 4 at
   // width 8, 2 from width 16 on)
-  auto kern = k_mvsd_gram_dmma<BM, BK, MV, R, S, GM>;
+  auto kern = k_mvsd_gram_dmma<BM, BK, MV, R, S>;
   set_smem(kern, smem);
   static std::atomic<int> occ{0};
   if (occ.load() == 0) {
@@ -1359,7 +1364,7 @@ bool mvsd_gram_dmma_launch(RowGemmArgs<double>& a)
     occ.store(std::max(1, o));
   }
   const int grid = (int)std::min<int64_t>(ceil_div(a.n, R), (int64_t)rt().num_sms() * occ.load());
-  const int gm = (GM == GM_WW) ? a.k : a.mv;
+  const int gm = a.mv;
   const int nout = gm * a.k;
   a.part = (double*)rt().scratch(sizeof(double) * (size_t)grid * nout);
   a.counter = rt().counters();
@@ -1375,14 +1380,14 @@ bool mvsd_gram_dmma_launch(RowGemmArgs<double>& a)
   return true;
 }
 
-template <int BM, int BK, int GM>
+template <int BM, int BK>
 bool mvsd_gram_dmma_mv(RowGemmArgs<double>& a, int MV)
 {
   switch (MV) {
-    case 8: return mvsd_gram_dmma_launch<BM, BK, 8, GM>(a);
-    case 16: return mvsd_gram_dmma_launch<BM, BK, 16, GM>(a);
-    case 32: return mvsd_gram_dmma_launch<BM, BK, 32, GM>(a);
-    default: return mvsd_gram_dmma_launch<BM, BK, 64, GM>(a);
+    case 8: return mvsd_gram_dmma_launch<BM, BK, 8>(a);
+    case 16: return mvsd_gram_dmma_launch<BM, BK, 16>(a);
+    case 32: return mvsd_gram_dmma_launch<BM, BK, 32>(a);
+    default: return mvsd_gram_dmma_launch<BM, BK, 64>(a);
   }
 }
 
@@ -1398,7 +1403,7 @@ inline bool mvsd_gram_dmma(RowGemmArgs<double>& a)
   const int BM = pad_width5(a.m), BK = pad_width5(a.k);
   if (a.mv < 5 || a.mv > 64 || BM != BK) return false;  // square blocks only
   const int MV = pad_width5(a.mv);
-  return BM == 8 ? mvsd_gram_dmma_mv<8, 8, GM_VW>(a, MV) : mvsd_gram_dmma_mv<16, 16, GM_VW>(a, MV);
+  return BM == 8 ? mvsd_gram_dmma_mv<8, 8>(a, MV) : mvsd_gram_dmma_mv<16, 16>(a, MV);
 }
 inline bool mvsd_gram_dmma(RowGemmArgs<float>&) { return false; }
 

@@ -140,34 +140,33 @@ __global__ void __launch_bounds__(256) k_mvtmv_dmma(MvTmvArgs<double> a, const _
 }
 
 // ------------------------------------------------------- V*C fused with a Gram
-// One pass for PHIST's fused_mvsd_mvTmv and fused_mvsdi_mvTmv
-// (phist_kernels_fused_decl.h:84,92): warp w forms the rows [w*R/8, ...) of
+// One pass for PHIST's fused_mvsdi_mvTmv with V another block than W
+// (phist_kernels_fused_decl.h:84): warp w forms the rows [w*R/8, ...) of
 // the new W tile from the staged rows of V and C in shared memory (pitch
 // BK + 4, zero-padded), writes them to global memory and keeps them in shared
 // memory (pitch PT = BK + 4), and the Gram product of the tile is accumulated
 // right away
-//   GM == GM_WW : G  = W'W              (GMR = BK rows)
-//   GM == GM_VW : D  = galpha V'W + gbeta D, V staged by TMA with A (GMR = MV)
+//   D = galpha V'W + gbeta D, V staged by TMA with A
 // with the warp split and fixed-order reduction of k_mvtmv_dmma.  W is not
 // read back from HBM.
-template <int BM, int BK, int MV, int R, int S, int GM>
+template <int BM, int BK, int MV, int R, int S>
 __global__ void __launch_bounds__(256) k_mvsd_gram_dmma(RowGemmArgs<double> a,
                                                         const __grid_constant__ CUtensorMap mapA,
                                                         const __grid_constant__ CUtensorMap mapV, int* err)
 {
   constexpr int NT = BK / 8, RW = R / 8, RT8 = RW / 8;
   constexpr int AP = BM + 4, CP = BK + 4, PT = BK + 4, PVG = MV + 4;
-  constexpr int GMR = (GM == GM_WW) ? BK : MV;
+  constexpr int GMR = MV;
   constexpr int MTG = GMR / 8, NTG = BK / 8;
   constexpr int WS = (MTG * NTG > 32) ? 2 : 1, MTW = MTG / WS, WQ = 8 / WS, KSTEPS = R / 4;
   constexpr int CSZ = (BM * CP * 8 + 127) / 128 * 128 / 8;
-  constexpr int VSZ = (GM == GM_VW) ? R * PVG : 0;
+  constexpr int VSZ = R * PVG;
   constexpr unsigned STAGE_BYTES = (unsigned)((R * AP + VSZ) * sizeof(double));
   static_assert(BM % 8 == 0 && BK % 8 == 0 && MV % 8 == 0 && R % 64 == 0 && R <= 256 && S >= 2, "bad shape");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double* sC = reinterpret_cast<double*>(smem_raw);  // [BM][CP]
   double* sA = sC + CSZ;                              // [S][R][AP]
-  double* sV = sA + S * R * AP;                       // [S][R][PVG] (GM_VW)
+  double* sV = sA + S * R * AP;                       // [S][R][PVG]
   double* sT = sV + S * VSZ;                          // [R][PT] new W tile
   uint64_t* bar = reinterpret_cast<uint64_t*>(sT + R * PT);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -180,7 +179,7 @@ __global__ void __launch_bounds__(256) k_mvsd_gram_dmma(RowGemmArgs<double> a,
     for (int st = 0; st < S; st++) mbar_init(&bar[st], 1);
     mbar_fence_init();
     tma_prefetch_desc(&mapA);
-    if (GM == GM_VW) tma_prefetch_desc(&mapV);
+    tma_prefetch_desc(&mapV);
   }
   for (int q = tid; q < BM * CP; q += blockDim.x) {
     const int i = q / CP, j = q - i * CP;
@@ -190,7 +189,7 @@ __global__ void __launch_bounds__(256) k_mvsd_gram_dmma(RowGemmArgs<double> a,
   auto issue = [&](int st, int64_t tl) {
     mbar_arrive_expect_tx(&bar[st], STAGE_BYTES);
     tma_load_2d(sA + st * R * AP, &mapA, 0, (int)(tl * R), &bar[st]);
-    if (GM == GM_VW) tma_load_2d(sV + st * VSZ, &mapV, 0, (int)(tl * R), &bar[st]);
+    tma_load_2d(sV + st * VSZ, &mapV, 0, (int)(tl * R), &bar[st]);
   };
   if (tid == 0)
     for (int st = 0; st < S - 1; st++) {
@@ -257,9 +256,9 @@ __global__ void __launch_bounds__(256) k_mvsd_gram_dmma(RowGemmArgs<double> a,
     }
     __syncthreads();  // sT complete
     if (ok) {
-      // ---- Gram of the tile: A operand rows from sT (W'W) or the V tile (V'W)
-      const double* gl = (GM == GM_WW) ? sT : sV + stage * VSZ;
-      constexpr int GP = (GM == GM_WW) ? PT : PVG;
+      // ---- V'W of the tile: A operand rows from the V tile
+      const double* gl = sV + stage * VSZ;
+      constexpr int GP = PVG;
 #pragma unroll 2
       for (int ks = wq; ks < KSTEPS; ks += WQ) {
         const int r = ks * 4 + t;
@@ -294,7 +293,7 @@ __global__ void __launch_bounds__(256) k_mvsd_gram_dmma(RowGemmArgs<double> a,
     }
     __syncthreads();
   }
-  const int gm = (GM == GM_WW) ? a.k : a.mv;
+  const int gm = a.mv;
   const int nout = gm * a.k;
   double* part = a.part + (int64_t)blockIdx.x * nout;
   for (int o = tid; o < nout; o += blockDim.x) part[o] = red[(o % gm) + (o / gm) * GMR];
