@@ -736,7 +736,9 @@ void launch_spmv_nv(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p, 
       return;
     }
   }
-  if (fast && !dots && !p.u && rt().spmv_pf && (vec || (NV == 1 && p.nvec == 1))) {
+  // column factors only in the default split (the device solvers' calls)
+  constexpr bool deftpr = TPR == (NV <= 4 ? 1 : NV == 8 ? 2 : 4);
+  if (fast && !dots && !p.u && rt().spmv_pf && (vec || (NV == 1 && p.nvec == 1)) && (deftpr || !p.cscale)) {
     // resident grid, next tile's entries prefetched into shared memory
     constexpr int NT = TPR == 1 ? 128 : (TPR == 16 ? 512 : 256);
     constexpr int RPBp = NT / TPR;
@@ -758,19 +760,35 @@ void launch_spmv_nv(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p, 
                       p.ldx % V32 == 0 && p.ldy % V32 == 0;
     if constexpr ((NV / TPR) * sizeof(T) >= 32) {
       if (v256) {
-        static std::atomic<int> occ32{0};
-        auto kern = pf_kernel<T, NV, TPR, NT, false, 32>();
-        const int pgrid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rt().num_sms() * resident(kern, occ32)));
-        launch_pdl(kern, pgrid, NT, 0, S, p);
-        PB_LAUNCH_CHECK();
+        auto go32 = [&](auto kern, std::atomic<int>& o) {
+          const int pgrid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rt().num_sms() * resident(kern, o)));
+          launch_pdl(kern, pgrid, NT, 0, S, p);
+          PB_LAUNCH_CHECK();
+        };
+        static std::atomic<int> occ32[2];
+        if constexpr (deftpr) {
+          if (p.cscale) {
+            go32(pf_kernel<T, NV, TPR, NT, false, 32, EpiScale>(), occ32[1]);
+            return;
+          }
+        }
+        go32(pf_kernel<T, NV, TPR, NT, false, 32>(), occ32[0]);
         return;
       }
     }
-    static std::atomic<int> occ{0};
-    auto kern = pf_kernel<T, NV, TPR, NT>();
-    const int pgrid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rt().num_sms() * resident(kern, occ)));
-    launch_pdl(kern, pgrid, NT, 0, S, p);
-    PB_LAUNCH_CHECK();
+    auto go = [&](auto kern, std::atomic<int>& o) {
+      const int pgrid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rt().num_sms() * resident(kern, o)));
+      launch_pdl(kern, pgrid, NT, 0, S, p);
+      PB_LAUNCH_CHECK();
+    };
+    static std::atomic<int> occ[2];
+    if constexpr (deftpr) {
+      if (p.cscale) {
+        go(pf_kernel<T, NV, TPR, NT, false, 16, EpiScale>(), occ[1]);
+        return;
+      }
+    }
+    go(pf_kernel<T, NV, TPR, NT>(), occ[0]);
     return;
   }
   if (unroll && A->C == 32 && !fast && !dots && !p.u && rt().spmv_pf && (vec || (NV == 1 && p.nvec == 1)) &&
@@ -811,6 +829,24 @@ template <class T, int VW, int TPR, int UPT>
 void launch_spmv_any(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p)
 {
   constexpr int NV = VW * TPR * UPT, NT = TPR == 1 ? 128 : 256, RPB = NT / TPR, VB = VW * (int)sizeof(T);
+  if (p.want_wdw || p.want_vdw) {
+    auto kern = k_sell_spmmv_pf_dots<T, NV, TPR, NT, VB>;
+    static std::atomic<int> occd{0};
+    if (occd.load() == 0) {
+      int o = 0;
+      PB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, NT, 0));
+      occd.store(std::max(1, o));
+    }
+    const int64_t ntiles = ceil_div(A->nchunks, RPB / 32);
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rt().num_sms() * occd.load()));
+    p.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
+    p.dpart = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ceil_div(grid, p.gsz)) * 2 * NV);
+    p.counter = rt().counters();
+    p.dots_nv = NV;
+    launch_pdl(kern, grid, NT, 0, S, p);
+    PB_LAUNCH_CHECK();
+    return;
+  }
   if (A->max_row_len <= 8) {
     auto kern = k_sell_spmmv_pf_any<T, NV, TPR, NT, VB>;
     static std::atomic<int> occ{0};
@@ -879,8 +915,14 @@ void spmv_tile(const SparseMat<T>* A, SpmvArgs<T>& p, int nv)
   const int tpr = A->tune_tpr[lg] > 0 ? A->tune_tpr[lg] : rt().spmv_tpr[lg];
   // widths that are no power of two, rows that start on no vector boundary
   const bool unroll = A->tune_unroll[lg] >= 0 ? A->tune_unroll[lg] != 0 : rt().spmv_unroll;
-  const bool plain = A->C == 32 && rt().spmv_pf && unroll && !p.want_wdw && !p.want_vdw && !p.u;
-  if (plain && !vec && NV > 1) {
+  const bool dots = p.want_wdw || p.want_vdw;
+  const bool plain = A->C == 32 && rt().spmv_pf && unroll && !p.u;
+  p.dots_nv = NV;
+  // The widths and alignments that the vector kernels do not take; with column
+  // dots on short rows and from 3 columns on (128^3 rows, us, one-tile kernel
+  // -> this: FP64 3 columns 171 -> 85, 5 319 -> 123, 13 641 -> 419; FP32 2
+  // columns 50 -> 54; on vector boundaries FP64 8 columns 174 -> 273)
+  if (plain && !vec && (dots ? A->max_row_len <= 8 && NV > 2 : NV > 1)) {
     spmv_any<T>(A, S, p);
     return;
   }
@@ -1052,11 +1094,10 @@ void spmv_general(T alpha, const SparseMat<T>* A, const T* shifts, const Mvec<T>
     }
     spmv_tile<T>(A, p, nv);
     if (dots_dev) {
-      const int NV = nv <= 1 ? 1 : nv <= 2 ? 2 : nv <= 4 ? 4 : nv <= 8 ? 8 : nv <= 16 ? 16 : 32;
       rt().sync();
       for (int j = 0; j < nv; j++) {
         if (WdotW) WdotW[c0 + j] = hd[j];
-        if (VdotW) VdotW[c0 + j] = hd[NV + j];
+        if (VdotW) VdotW[c0 + j] = hd[p.dots_nv + j];
       }
     }
   }

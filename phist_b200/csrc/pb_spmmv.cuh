@@ -50,6 +50,9 @@ struct SpmvArgs {
   T* part;                       // per-block partials [grid][2*NV]
   unsigned int* counter;
   T* dots_out;                   // device [2*NV]: WdotW then VdotW
+  int dots_nv;                   // NV of the kernel that ran (host)
+  double* dpart;                 // partials and group size of the resident kernel's dots
+  int gsz;
   T gamma, delta;
   T* u;
   int64_t ldu;

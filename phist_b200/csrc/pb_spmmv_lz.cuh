@@ -21,7 +21,7 @@ constexpr int LZ_MB = 3;
 
 template <class T, int NV, int TPR>
 struct EpiLanczos {
-  static constexpr bool on = true;
+  static constexpr bool on = true, scale = true;
   static constexpr int RPB = LZ_NT / TPR, PY = NV + 1, VPT = NV / TPR;
   static constexpr int MQ = LZ_MAXQ / 8;
   static constexpr int STEPS = RPB / 4 / FRAG_NW;  // 4-row steps of a warp in a tile
@@ -62,6 +62,7 @@ struct EpiLanczos {
   }
   __device__ __forceinline__ void tile()
   {
+    __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     T qv[STEPS][MQ];
 #pragma unroll

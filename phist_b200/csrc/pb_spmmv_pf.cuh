@@ -37,6 +37,7 @@
 #include "pb_spmmv.cuh"
 #include "pb_tile.cuh"
 #include "pb_dmma.cuh"
+#include "pb_frag.cuh"
 #include <type_traits>
 
 namespace pb {
@@ -200,10 +201,14 @@ struct GramNone {
   __device__ __forceinline__ void init() {}
 };
 
-// What else a kernel does with the rows it forms (pb_spmmv_lz.cuh); this one
-// nothing.
+// What else a kernel does with the rows it forms (EpiDots below,
+// pb_spmmv_lz.cuh).  `scale`: p.cscale may be given; compiled out of the plain
+// form, where its branch alone cost 5 % at width 32.
 struct EpiNone {
-  static constexpr bool on = false;
+  static constexpr bool on = false, scale = false;
+};
+struct EpiScale {
+  static constexpr bool on = false, scale = true;
 };
 
 template <class T, int NV, int NT, int RPB>
@@ -350,13 +355,27 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
             }
         }
       } else {
-        if (i >= 0 && p.has_shift) {
+        if constexpr (Epi::on) {
+          if (i >= 0) {
 #pragma unroll
-          for (int v = 0; v < NVV; v++) Vec<T, VW>::ld(x + i * p.ldx + lcol(v), &xi[v * VW]);
+            for (int v = 0; v < NVV; v++) Vec<T, VW>::ld(x + i * p.ldx + lcol(v), &xi[v * VW]);
+          }
+        }
+        if (i >= 0 && p.has_shift) {
+          T xs[VPT];
+#pragma unroll
+          for (int v = 0; v < NVV; v++) {
+            if constexpr (Epi::on) {
+#pragma unroll
+              for (int w = 0; w < VW; w++) xs[v * VW + w] = xi[v * VW + w];
+            } else {
+              Vec<T, VW>::ld(x + i * p.ldx + lcol(v), &xs[v * VW]);
+            }
+          }
 #pragma unroll
           for (int v = 0; v < NVV; v++)
 #pragma unroll
-            for (int w = 0; w < VW; w++) acc[v * VW + w] = AT(p.sh[lcol(v) + w]) * AT(xi[v * VW + w]);
+            for (int w = 0; w < VW; w++) acc[v * VW + w] = AT(p.sh[lcol(v) + w]) * AT(xs[v * VW + w]);
         }
       }
       const int lc = lr / CC, l = lr % CC;
@@ -398,7 +417,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
         for (int v = 0; v < NVV; v++) {
           const int c = spmv_col<TPR, VW>(s, v, 0);
           if (ANY && c >= p.nvec) continue;
-          spmv_cscale<VW>(p, c, &acc[v * VW]);
+          if constexpr (ANY || Epi::scale) spmv_cscale<VW>(p, c, &acc[v * VW]);
           T yv[VW];
           if (p.beta != T(0)) {
             Vec<T, VW>::ld_plain(yr + c, yv);
@@ -425,10 +444,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
       __syncthreads();
       gram.add_tile(gys, gxs);
     }
-    if constexpr (Epi::on) {
-      __syncthreads();
-      epi.tile();
-    }
+    if constexpr (Epi::on) epi.tile();
     cp_async_wait<0>();
     if (tid <= NCH) smeta[mbnn][tid] = mnext;
     __syncthreads();
@@ -436,6 +452,63 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
   if constexpr (GRAM) gram.store(p, gys);
   if constexpr (Epi::on) epi.finish();
 }
+
+// The column dots of fused_spmv_mvdot: W_j'W_j and V_j'W_j of the new rows
+// from the registers that hold them, the blocks' sums in the two-level tree of
+// pb_frag.cuh, the result straight into p.dots_out (mapped host memory): W'W
+// at [0, NV), V'W at [NV, 2 NV).
+template <class T, int NV, int TPR, int NT, int VW>
+struct EpiDots {
+  static constexpr bool on = true, scale = false;
+  static constexpr int VPT = NV / TPR, NVV = VPT / VW, NW = NT / 32;
+  const SpmvArgs<T>& p;
+  double* red;  // [NW][2 NV]
+  T wdw[VPT], vdw[VPT];
+  __device__ __forceinline__ EpiDots(const SpmvArgs<T>& args, double* r) : p(args), red(r)
+  {
+#pragma unroll
+    for (int q = 0; q < VPT; q++) wdw[q] = vdw[q] = T(0);
+  }
+  __device__ __forceinline__ void clear(int) {}
+  template <int W>
+  __device__ __forceinline__ void put(int, int64_t, int v, int, const T* y, const T* x)
+  {
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+      wdw[v * W + w] += y[w] * y[w];
+      vdw[v * W + w] += x[w] * y[w];
+    }
+  }
+  __device__ __forceinline__ void tile() {}
+  __device__ __forceinline__ void finish()
+  {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+    for (int v = 0; v < NVV; v++)
+#pragma unroll
+      for (int w = 0; w < VW; w++) {
+        double a = (double)wdw[v * VW + w], b = (double)vdw[v * VW + w];
+#pragma unroll
+        for (int off = 16; off >= TPR; off >>= 1) {
+          a += __shfl_xor_sync(0xffffffffu, a, off);
+          b += __shfl_xor_sync(0xffffffffu, b, off);
+        }
+        if (lane < TPR) {
+          red[warp * 2 * NV + spmv_col<TPR, VW>(lane, v, w)] = a;
+          red[warp * 2 * NV + NV + spmv_col<TPR, VW>(lane, v, w)] = b;
+        }
+      }
+    __syncthreads();
+    double tot[1] = {0.0};
+    if (tid < 2 * NV) {
+#pragma unroll
+      for (int k = 0; k < NW; k++) tot[0] += red[k * 2 * NV + tid];
+      p.dpart[(int64_t)blockIdx.x * 2 * NV + tid] = tot[0];
+    }
+    if (!frag_tree_sum<1, NT>(p.dpart, 2 * NV, p.gsz, p.counter, tot)) return;
+    if (tid < 2 * NV) p.dots_out[tid] = (T)tot[0];
+  }
+};
 
 // The kernel comes in two entry points around the same body: with a minimum
 // of resident blocks per SM handed to ptxas, which changes how it allocates
@@ -455,17 +528,17 @@ constexpr int pf_min_blocks()
   return NV == 2 ? 4 : NV == 8 ? 3 : NV == 16 ? 4 : 0;
 }
 
-template <class T, int NV, int TPR, int NT, bool GRAM = false, int VB = 16>
+template <class T, int NV, int TPR, int NT, bool GRAM = false, int VB = 16, class Epi = EpiNone>
 __global__ void __launch_bounds__(NT) k_sell_spmmv_pf(SellDev<T> A, SpmvArgs<T> p)
 {
-  EpiNone none;
+  Epi none;
   sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB, false>(A, p, none);
 }
 
-template <class T, int NV, int TPR, int NT, bool GRAM, int VB, int MB>
+template <class T, int NV, int TPR, int NT, bool GRAM, int VB, int MB, class Epi = EpiNone>
 __global__ void __launch_bounds__(NT, MB) k_sell_spmmv_pf_mb(SellDev<T> A, SpmvArgs<T> p)
 {
-  EpiNone none;
+  Epi none;
   sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB, false>(A, p, none);
 }
 
@@ -484,15 +557,25 @@ __global__ void __launch_bounds__(NT, (pf_any_blocks<T, NV / TPR, NT>())) k_sell
   sell_spmmv_pf<T, NV, TPR, NT, false, VB, true>(A, p, none);
 }
 
+// with the column dots; the split and the register budget of the any-width form
+template <class T, int NV, int TPR, int NT, int VB>
+__global__ void __launch_bounds__(NT, (pf_any_blocks<T, NV / TPR, NT>())) k_sell_spmmv_pf_dots(SellDev<T> A, SpmvArgs<T> p)
+{
+  typedef EpiDots<T, NV, TPR, NT, VB / (int)sizeof(T)> Epi;
+  __shared__ double red[Epi::NW * 2 * NV];
+  Epi epi(p, red);
+  sell_spmmv_pf<T, NV, TPR, NT, false, VB, true>(A, p, epi);
+}
+
 // the entry point of a form
-template <class T, int NV, int TPR, int NT, bool GRAM = false, int VB = 16>
+template <class T, int NV, int TPR, int NT, bool GRAM = false, int VB = 16, class Epi = EpiNone>
 constexpr auto pf_kernel()
 {
   constexpr int mb = pf_min_blocks<T, NV, TPR, NT, GRAM>();
   if constexpr (mb > 0)
-    return &k_sell_spmmv_pf_mb<T, NV, TPR, NT, GRAM, VB, mb>;
+    return &k_sell_spmmv_pf_mb<T, NV, TPR, NT, GRAM, VB, mb, Epi>;
   else
-    return &k_sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB>;
+    return &k_sell_spmmv_pf<T, NV, TPR, NT, GRAM, VB, Epi>;
 }
 
 // ------------------------------------------------------------ longer rows
