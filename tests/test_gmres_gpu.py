@@ -1,5 +1,5 @@
 """Device-resident GMRES and MINRES for the Jacobi-Davidson correction
-equations (phist_b200_{D,S}jadaCorrection_{gmres,minres}, csrc/pb_gmres.cu)
+equations (phist_b200_{D,S}jadaCorrection_{gmres,minres}, csrc/pb_gmres.cuh)
 against the numpy restatements of PHIST's GMRES and MINRES in the oracle: the
 iterate after a given number of steps is unique (the residual minimiser over
 the Krylov space), so cut-off runs, restarted runs and converged runs must
