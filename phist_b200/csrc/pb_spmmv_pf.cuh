@@ -31,8 +31,8 @@
 // each block leaves its partial sums for a fixed-order second pass.
 //
 // Preconditions (checked by the launcher): SELL chunk height 32, at most 8
-// entries per row, no fused dot / axpby epilogue, the whole block vector as
-// the column tile when GRAM is set.
+// entries per row, no axpby epilogue, the whole block vector as the column
+// tile when GRAM is set; column dots are a form of their own (EpiDots).
 #pragma once
 #include "pb_spmmv.cuh"
 #include "pb_tile.cuh"
