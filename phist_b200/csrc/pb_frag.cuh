@@ -469,7 +469,9 @@ k_nn_gram_frag(const __grid_constant__ FragNnArgs<T> a, const __grid_constant__ 
   constexpr int KS = 2 * MC, P = KT * 8 + 4;
   constexpr int NC = KS * KT * 32, NTL = FRAG_NW * 8 * P, NRED = frag_red<KT, KT>();
   constexpr int NTILE = KT * (KT + 1) / 2;
-  __shared__ double sm[NC + NTL > NRED ? NC + NTL : NRED];
+  // the tile's pairs are stored 16 bytes at a time
+  __shared__ __align__(16) double sm[NC + NTL > NRED ? NC + NTL : NRED];
+  static_assert(NC % 2 == 0 && P % 2 == 0, "pairs of a tile start on 16 bytes");
   double* sC = sm;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
