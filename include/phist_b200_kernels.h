@@ -402,12 +402,14 @@ void phist_b200_DcarpCG_tune_block(phist_Dconst_sparseMat_ptr A, int nsys, int m
  *   (I - Q Q')(A - sigma_j I) t_j = res(:, resIndex[j]),  j < k <= 32
  * (the task of PHIST's jadaCorrectionSolver_run with GMRES,
  * src/jada/phist_jadaCorrectionSolver_def.hpp:141-583).  Q (n x nq, may be
- * NULL) has orthonormal columns; resIndex may be NULL (identity).  x_0 = 0;
+ * NULL) has orthonormal columns, to which the columns of res need not be
+ * orthogonal; resIndex may be NULL (identity).  x_0 = 0;
  * restarted after maxBas steps (<= 63), at most maxIter steps; system j is
  * converged when its GMRES residual is below 1000 eps absolute or tol[j]
  * relative to ||res_j|| (phist_blockedgmres_def.hpp:604-606).  The
  * Hessenberg matrices, rotations and all dot products stay on the device;
- * Gram-Schmidt is classical, done twice, as block products.  t (n x k)
+ * Gram-Schmidt is classical, with a second subtraction where the first one
+ * cancels or leaves more than rounding along the basis.  t (n x k)
  * receives the solutions scaled to unit norm (as PHIST returns them);
  * *iflag >= 0 is the number of systems that did not converge.  The S form
  * runs in FP32 (the small dense part in FP64). */

@@ -264,7 +264,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
   DBuf<double> H((size_t)(m + 1) * m * k), cs((size_t)m * k), sn((size_t)m * k), g((size_t)(m + 1) * k), bnorm(k);
   DBuf<double> h1((size_t)(m + 1) * k), h2((size_t)(m + 1) * k), nrm0(k), nf(k);
   const int ngrp = (int)ceil_div(k, KRY_MAXC);
-  DBuf<int> conv(k), jcount(k), reorth(ngrp);
+  DBuf<int> conv(k), jcount(k), reorth(ngrp), gflag(ngrp);
   std::vector<T> negsig(k);
   for (int s = 0; s < k; s++) negsig[s] = (T)(-sigma[s]);
   volatile unsigned long long* hflags = (volatile unsigned long long*)rt().mailbox_host();
@@ -272,6 +272,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
   // a projection block of at most KRY_MAXQ columns goes with the passes over
   // the basis, a wider one in products of its own
   const bool fuse = nq > 0 && nq <= KRY_MAXQ;
+  DBuf<double> gq((size_t)(fuse ? nq + m + 2 : 0) * k);  // g0, gam, dq
 
   Mvec<T> mX, mW, mVj;
   raw_view(mX, X.p, n, k, k);
@@ -295,6 +296,11 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
     e.F = F.p; e.cq = Cq.p; e.hv = hv.p; e.hv2 = hv2.p; e.finv = f.p;
     e.conv = conv.p; e.jcount = jcount.p;
     e.eps_abs = eps_abs;
+    // 100 eps of the new direction: dots of a pass that left nothing but
+    // rounding stay below it
+    const double lim = 100.0 * std::numeric_limits<T>::epsilon();
+    e.h2_lim = lim * lim;
+    e.g0 = gq.p; e.gam = gq.p + (size_t)nq * k; e.dq = e.gam + (size_t)(m + 1) * k;
     e.flags = (unsigned long long*)rt().mailbox_dev();
     for (int s = 0; s < k; s++) {
       base.idx.v[s] = resIndex ? resIndex[s] : s;
@@ -312,6 +318,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
       a.e.c0 = c0;
       a.e.last = q == ngrp - 1;
       a.e.reorth = reorth.p + q;
+      a.e.gflag = fuse ? gflag.p + q : nullptr;
       pass(a, c0);
     }
   };
@@ -334,13 +341,21 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
       a.W = V.p + c0;
       a.restart = cycle > 0 ? 1 : 0;
       a.e.first = cycle == 0 ? 1 : 0;
-      a.e.kind = KE_START;
+      a.e.kind = fuse ? KE_NONE : KE_START;
       const int grid = (int)std::min<int64_t>(ceil_div(n * a.kp, 4 * FRAG_BS), 4 * (int64_t)rt().num_sms());
       a.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
       a.part = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ceil_div(grid, a.gsz)) * KRY_MAXOUT);
       a.counters = rt().counters();
       launch_pdl(k_kry_start<T>, grid, FRAG_BS, 0, a);
       PB_LAUNCH_CHECK();
+      if (fuse) {
+        // the norms together with Q'V_0
+        a.nq = nq;
+        a.V = a.W;
+        a.Win = a.W;
+        a.e.kind = KE_START;
+        kry_dots<T, false>(a);
+      }
     });
     *hflags = 0;
     int j = 0, steps = 0;
@@ -390,15 +405,15 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
         const bool lastg = a0.e.last;
         if (lanczos) {
           // [Q V_j]'W; W -= Q (Q'W) + v_j alpha + v_{j-1} beta and its norm
-          // (alpha = v_j'W equals v_j'(P W) because V_j is orthogonal to Q;
-          // PHIST's order: projection, then the Lanczos terms)
+          // (alpha = v_j'(P W) from both dots; PHIST's order: projection,
+          // then the Lanczos terms)
           if (!dotted) pass(false, true, j, 1, true, nullptr, KE_LZ, true, nullptr);
           pass(true, false, j, j > 0 ? 2 : 1, true, hv.p, KE_STEP, lastg, nullptr);
           return;
         }
-        // Gram-Schmidt against Q and V_0..V_j: h1 = V'W; W -= Q (Q'W) + V h1
-        // and h2 = V'W of the result; a second subtraction only where a norm
-        // fell below 1/sqrt(2) of its value before (a device flag)
+        // Gram-Schmidt against Q and V_0..V_j: h1 = V'(P W) from V'W and Q'W
+        // (kry_epilogue); W -= Q (Q'W) + V h1 and h2 = V'W of the result; a
+        // second subtraction only where that is needed (a device flag)
         if (J <= KRY_MAXJ) {
           pass(false, true, 0, J, true, nullptr, KE_GS, true, nullptr);
           pass(true, true, 0, J, true, hv.p, KE_GS2, true, nullptr);

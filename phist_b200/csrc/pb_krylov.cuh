@@ -45,7 +45,7 @@ struct GmIndex {
 // what the block holding the sums does
 enum KryKind {
   KE_NONE = 0,    // nothing (the update alone)
-  KE_START,       // beta = ||W||, g = beta e_1, F_0
+  KE_START,       // beta = ||W||, g = beta e_1, F_0, g0
   KE_LZ,          // Lanczos coefficients of step j
   KE_GS,          // first Gram-Schmidt coefficients (blocks i0..), ||W|| before
   KE_GS2,         // second coefficients; with last also the decision on a second pass
@@ -67,8 +67,11 @@ struct KryEpi {
   T *cq, *hv, *hv2;           // coefficients for the update passes
   T *finv;
   int *conv, *jcount, *reorth;
-  double eps_abs;
+  double eps_abs, h2_lim;
   GmTol tol;
+  // Q'V_i = gam[i*k + s] g0 (nq values g0[l*k + s]); used while *gflag != 0
+  double *g0, *gam, *dq;
+  int* gflag;                 // NULL: no projection in the passes
   volatile unsigned long long* flags;  // mapped host memory: converged systems << 32 | steps done
 };
 
@@ -173,15 +176,58 @@ __device__ __forceinline__ void kry_step(const KryEpi<T>& e, int kc, const doubl
   }
 }
 
-// out: the sums in shared memory, [Q'W | V'W | ||W||^2] as nqo + nb + 1 rows
-// of kc; sm: further shared scratch
+// The dots of a pass see W before the projection: V_i'W, where the step wants
+// V_i'(P W) = V_i'W - (Q'V_i)'c with c = Q'W.  Q'V_i is rounding where the
+// right-hand side is orthogonal to Q, but nothing demands that.  All vectors
+// but V_0 come from the range of P, so Q'V_i is a multiple gam_i of g0 =
+// Q'V_0, with V_{j+1} = P W - sum_i V_i hv_i: gam_{j+1} = -sum_i gam_i hv_i.
+// The start takes g0 with the norms and sets *gflag where an entry is above
+// rounding; the first coefficients then are F_i (V_i'W - gam_i d), d = g0'c.
+
+// Warp w < kc: d of system w in all lanes, for the c that the update subtracts
 template <class T>
-__device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int nbo, const double* out, double* sm)
+__device__ __forceinline__ double kry_proj_sum(const KryArgs<T>& a, int nqo, const double* out)
+{
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool on = w < a.kc && lane < nqo;
+  const double c = on ? (double)(T)out[lane * a.kc + w] : 0.0;
+  double d = on ? __ldcg(&a.e.g0[lane * a.e.k + a.e.c0 + w]) * c : 0.0;
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
+  return d;
+}
+
+// The kinds that a kernel can be asked for, as bits.  The last block runs this
+// code once, from a cold instruction cache: with the kinds of all kernels in
+// every kernel a pass of 20 us took 0.7 us more.
+constexpr int kry_kinds(bool upd, bool dots)
+{
+  return upd ? (dots ? 1 << KE_GS2 : 1 << KE_STEP | 1 << KE_NORM) : 1 << KE_START | 1 << KE_LZ | 1 << KE_GS | 1 << KE_GS2;
+}
+
+// out: the sums in shared memory, [Q'W | V'W | ||W||^2] as nqo + nb + 1 rows
+// of kc; sm: further shared scratch; flagged: *gflag
+template <class T, int KINDS>
+__device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int nbo, const double* out, double* sm,
+                                             bool flagged)
 {
   const KryEpi<T>& e = a.e;
   const int tid = threadIdx.x, kc = a.kc, k = e.k, j = e.j, m = e.m;
   const double* nrm = out + (nqo + nbo) * kc;
-  if (e.kind == KE_START) {
+  auto is = [&](int kind) { return ((KINDS >> kind) & 1) && e.kind == kind; };
+  if (is(KE_START)) {
+    if (e.gflag) {
+      int big = 0;
+      for (int q = tid; q < nqo * kc; q += FRAG_BS) {
+        const double v = out[q];
+        const double eps = sizeof(T) == 8 ? 2.3e-16 : 1.2e-7;
+        e.g0[(q / kc) * k + e.c0 + q % kc] = v;
+        big |= v * v > 256.0 * eps * eps * nrm[q % kc];
+      }
+      big = __syncthreads_or(big);
+      if (tid == 0) *e.gflag = big;
+      if (tid < kc) e.gam[e.c0 + tid] = 1.0;
+    }
     if (tid < kc) {
       const int s = e.c0 + tid;
       const double beta = sqrt(fmax(nrm[tid], 0.0));
@@ -194,42 +240,75 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
       e.g[s] = e.conv[s] ? 0.0 : beta;
       e.F[s] = (beta > 0.0 && !e.conv[s]) ? (T)(1.0 / beta) : T(0);
     }
-  } else if (e.kind == KE_LZ) {
+  } else if (is(KE_LZ)) {
     for (int q = tid; q < nqo * kc; q += FRAG_BS) e.cq[(q / kc) * k + e.c0 + q % kc] = (T)out[q];
+    if (flagged) {
+      const double d = kry_proj_sum<T>(a, nqo, out);
+      if ((tid & 31) == 0 && (tid >> 5) < kc) sm[tid >> 5] = d;
+      __syncthreads();
+    }
     if (tid < kc) {
       // alpha = v_j'w, beta = the previous step's norm; the update
       // subtracts V_j (F_j alpha), then V_{j-1} (F_{j-1} beta)
       const int s = e.c0 + tid;
-      const double alpha = (double)e.F[j * k + s] * out[nqo * kc + tid];
+      const double gj = flagged ? e.gam[j * k + s] : 0.0;
+      const double alpha = (double)e.F[j * k + s] * (out[nqo * kc + tid] - (flagged ? gj * sm[tid] : 0.0));
       const double beta = j > 0 ? sqrt(e.nf[s]) : 0.0;
       for (int i = 0; i + 1 < j; i++) e.H[((int64_t)i * m + j) * k + s] = 0.0;
       if (j > 0) e.H[((int64_t)(j - 1) * m + j) * k + s] = beta;
       e.H[((int64_t)j * m + j) * k + s] = alpha;
       e.hv[s] = (T)((double)e.F[j * k + s] * alpha);
       e.hv[k + s] = j > 0 ? (T)((double)e.F[(j - 1) * k + s] * beta) : T(0);
+      if (flagged)
+        e.gam[(j + 1) * k + s] = -(gj * (double)e.hv[s] + (j > 0 ? e.gam[(j - 1) * k + s] * (double)e.hv[k + s] : 0.0));
     }
-  } else if (e.kind == KE_GS) {
+  } else if (is(KE_GS)) {
     for (int q = tid; q < nqo * kc; q += FRAG_BS) e.cq[(q / kc) * k + e.c0 + q % kc] = (T)out[q];
+    if (flagged) {
+      if (e.i0 == 0) {
+        const double d = kry_proj_sum<T>(a, nqo, out);
+        if ((tid & 31) == 0 && (tid >> 5) < kc) sm[tid >> 5] = e.dq[e.c0 + (tid >> 5)] = d;
+      } else if (tid < kc) {
+        sm[tid] = __ldcg(&e.dq[e.c0 + tid]);
+      }
+      __syncthreads();
+    }
     for (int q = tid; q < nbo * kc; q += FRAG_BS) {
       const int p = (e.i0 + q / kc) * k + e.c0 + q % kc;
-      const double h = (double)e.F[p] * out[nqo * kc + q];
+      const double h = (double)e.F[p] * (out[nqo * kc + q] - (flagged ? __ldcg(&e.gam[p]) * sm[q % kc] : 0.0));
       e.h1[p] = h;
       e.hv[p] = (T)((double)e.F[p] * h);
     }
     if (tid < kc) e.nrm0[e.c0 + tid] = nrm[tid];
-  } else if (e.kind == KE_GS2) {
+  } else if (is(KE_GS2)) {
+    // A second subtraction where some norm fell below 1/sqrt(2) of its value
+    // before the pass ("twice is enough"), or where the first one has left
+    // more than rounding along the basis: parts of V_i in the span of Q grow
+    // from rounding as the steps go on, and Q may be orthonormal to less.
+    int need = 0;
     for (int q = tid; q < nbo * kc; q += FRAG_BS) {
       const int p = (e.i0 + q / kc) * k + e.c0 + q % kc;
       const double h = (double)e.F[p] * out[nqo * kc + q];
       e.h2[p] = h;
       e.hv2[p] = (T)((double)e.F[p] * h);
+      need |= h * h > e.h2_lim * nrm[q % kc];
     }
     if (!e.last) return;
-    // a second subtraction where some norm fell below 1/sqrt(2) of its value
-    // before the pass ("twice is enough")
-    const int need = tid < kc && nrm[tid] < 0.5 * e.nrm0[e.c0 + tid];
+    for (int q = tid; q < e.i0 * kc; q += FRAG_BS) {
+      const double h = __ldcg(&e.h2[(q / kc) * k + e.c0 + q % kc]);
+      need |= h * h > e.h2_lim * nrm[q % kc];
+    }
+    if (tid < kc) need |= nrm[tid] < 0.5 * e.nrm0[e.c0 + tid];
     __threadfence_block();
     const int any = __syncthreads_or(need);
+    if (flagged && tid < kc) {
+      const int s = e.c0 + tid;
+      double gn = 0.0;
+      for (int i = 0; i <= j; i++)
+        gn -= __ldcg(&e.gam[i * k + s]) *
+              ((double)__ldcg(&e.hv[i * k + s]) + (any ? (double)__ldcg(&e.hv2[i * k + s]) : 0.0));
+      e.gam[(j + 1) * k + s] = gn;
+    }
     for (int q = tid; q < (j + 1) * kc; q += FRAG_BS) {
       const int i = q / kc, s = e.c0 + q % kc;
       e.H[((int64_t)i * m + j) * k + s] = __ldcg(&e.h1[i * k + s]) + (any ? __ldcg(&e.h2[i * k + s]) : 0.0);
@@ -237,9 +316,9 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
     if (tid == 0) *e.reorth = any;
     __threadfence();
     if (!any) kry_step<T>(e, kc, nrm, sm);
-  } else if (e.kind == KE_STEP) {
+  } else if (is(KE_STEP)) {
     kry_step<T>(e, kc, nrm, sm);
-  } else if (e.kind == KE_NORM) {
+  } else if (is(KE_NORM)) {
     if (tid < kc) {
       const double nr = sqrt(fmax(nrm[tid], 0.0));
       e.finv[e.c0 + tid] = nr > 0.0 ? (T)(1.0 / nr) : T(0);
@@ -257,11 +336,14 @@ static_assert(KRY_MAXOUT + 3 * 64 * KRY_MAXC <= KRY_RED, "epilogue scratch fits 
 // red: the warps' sums, stride apart; from there the
 // block's, the blocks' and, in the block that holds the totals, the epilogue
 // (sm: shared scratch for it, may be red)
-template <class T>
+template <class T, int KINDS>
 __device__ __forceinline__ void kry_totals(const KryArgs<T>& a, int nqo, int nbo, const double* red, int stride,
                                            double* sm)
 {
   const int tid = threadIdx.x, nout = (nqo + nbo + 1) * a.kc;
+  // loaded ahead of the sums, whose latency covers it
+  constexpr bool uses = (KINDS & (1 << KE_LZ | 1 << KE_GS | 1 << KE_GS2)) != 0;
+  const int flag = uses && a.e.gflag && a.e.kind != KE_START ? __ldcg(a.e.gflag) : 0;
   __syncthreads();
   double tot[2];
 #pragma unroll
@@ -285,15 +367,16 @@ __device__ __forceinline__ void kry_totals(const KryArgs<T>& a, int nqo, int nbo
   for (int q = 0; q < 2; q++)
     if (tid + q * FRAG_BS < nout) sm[tid + q * FRAG_BS] = tot[q];
   __syncthreads();
-  kry_epilogue<T>(a, nqo, nbo, sm, sm + KRY_MAXOUT);
+  kry_epilogue<T, KINDS>(a, nqo, nbo, sm, sm + KRY_MAXOUT, flag != 0);
 }
 
 // after the row loop: the lanes' sums to the warps'
-template <class T, int MQ, int MJ>
+template <class T, int MQ, int MJ, int KINDS>
 __device__ __forceinline__ void kry_finish(const KryArgs<T>& a, int nqo, int nbo, double (&qa)[MQ > 0 ? MQ : 1][2],
                                            T (&va)[MJ], T na, double* sm)
 {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+  if (a.e.kind == KE_NONE) return;  // the update alone
   const int kc = a.kc, kp = a.kp, s = lane & (kp - 1);
   double nd = (double)na, vd[MJ];
 #pragma unroll
@@ -321,7 +404,7 @@ __device__ __forceinline__ void kry_finish(const KryArgs<T>& a, int nqo, int nbo
       if (i < nbo) red[(nqo + i) * kc + s] = vd[i];
     red[(nqo + nbo) * kc + s] = nd;
   }
-  kry_totals<T>(a, nqo, nbo, sm, KRY_MAXOUT, sm);
+  kry_totals<T, KINDS>(a, nqo, nbo, sm, KRY_MAXOUT, sm);
 }
 
 template <class T, int MQ, int MJ, bool UPD, bool DOTS>
@@ -442,7 +525,7 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
     }
     if (MQ > 0 && UPD) __syncwarp();
   }
-  kry_finish<T, MQ, MJ>(a, (DOTS && !UPD && MQ > 0) ? nq : 0, DOTS ? nb : 0, qa, va, na, sm);
+  kry_finish<T, MQ, MJ, kry_kinds(UPD, DOTS)>(a, (DOTS && !UPD && MQ > 0) ? nq : 0, DOTS ? nb : 0, qa, va, na, sm);
 }
 
 // W = R(:, idx) at the start, W = R(:, idx) - W (0 for converged systems) on
@@ -471,7 +554,7 @@ __global__ void __launch_bounds__(FRAG_BS) k_kry_start(const __grid_constant__ K
   }
   double qa[1][2];
   T va[1] = {T(0)};
-  kry_finish<T, 0, 1>(a, 0, 0, qa, va, na, sm);
+  kry_finish<T, 0, 1, 1 << KE_START>(a, 0, 0, qa, va, na, sm);
 }
 
 }  // namespace pb

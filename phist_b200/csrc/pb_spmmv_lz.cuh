@@ -28,6 +28,7 @@ struct EpiLanczos {
   static constexpr int RED = (LZ_MAXQ + 2) * NV;   // a warp's sums
   static constexpr int BUF = RPB * PY > FRAG_NW * RED ? RPB * PY : FRAG_NW * RED;
   static_assert(RPB % (4 * FRAG_NW) == 0 && NV <= KRY_MAXC, "bad tile");
+  static_assert(BUF >= KRY_MAXOUT + KRY_MAXC, "epilogue scratch of KE_LZ");
   const KryArgs<T>& a;
   T* ys;       // new rows of the tile
   int* rows;   // their row numbers, -1: none
@@ -104,7 +105,7 @@ struct EpiLanczos {
         red[(a.nq + 1) * NV + lane * VPT + q] = 0.0;
       }
     }
-    kry_totals<T>(a, a.nq, 1, buf, RED, buf);
+    kry_totals<T, 1 << KE_LZ>(a, a.nq, 1, buf, RED, buf);
   }
 };
 
