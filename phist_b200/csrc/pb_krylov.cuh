@@ -184,17 +184,22 @@ __device__ __forceinline__ void kry_step(const KryEpi<T>& e, int kc, const doubl
 // The start takes g0 with the norms and sets *gflag where an entry is above
 // rounding; the first coefficients then are F_i (V_i'W - gam_i d), d = g0'c.
 
-// Warp w < kc: d of system w in all lanes, for the c that the update subtracts
+// Warp w < kc: d (0 unless flagged) and ||c||^2 of system w in all lanes, for
+// the c that the update subtracts
 template <class T>
-__device__ __forceinline__ double kry_proj_sum(const KryArgs<T>& a, int nqo, const double* out)
+__device__ __forceinline__ void kry_proj_sums(const KryArgs<T>& a, int nqo, const double* out, bool flagged, double& d,
+                                              double& c2)
 {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool on = w < a.kc && lane < nqo;
   const double c = on ? (double)(T)out[lane * a.kc + w] : 0.0;
-  double d = on ? __ldcg(&a.e.g0[lane * a.e.k + a.e.c0 + w]) * c : 0.0;
+  c2 = c * c;
+  d = (on && flagged) ? __ldcg(&a.e.g0[lane * a.e.k + a.e.c0 + w]) * c : 0.0;
 #pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
-  return d;
+  for (int off = 16; off >= 1; off >>= 1) {
+    c2 += __shfl_xor_sync(0xffffffffu, c2, off);
+    d += __shfl_xor_sync(0xffffffffu, d, off);
+  }
 }
 
 // The kinds that a kernel can be asked for, as bits.  The last block runs this
@@ -243,7 +248,8 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
   } else if (is(KE_LZ)) {
     for (int q = tid; q < nqo * kc; q += FRAG_BS) e.cq[(q / kc) * k + e.c0 + q % kc] = (T)out[q];
     if (flagged) {
-      const double d = kry_proj_sum<T>(a, nqo, out);
+      double d, c2;
+      kry_proj_sums<T>(a, nqo, out, true, d, c2);
       if ((tid & 31) == 0 && (tid >> 5) < kc) sm[tid >> 5] = d;
       __syncthreads();
     }
@@ -264,22 +270,28 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
     }
   } else if (is(KE_GS)) {
     for (int q = tid; q < nqo * kc; q += FRAG_BS) e.cq[(q / kc) * k + e.c0 + q % kc] = (T)out[q];
-    if (flagged) {
-      if (e.i0 == 0) {
-        const double d = kry_proj_sum<T>(a, nqo, out);
-        if ((tid & 31) == 0 && (tid >> 5) < kc) sm[tid >> 5] = e.dq[e.c0 + (tid >> 5)] = d;
-      } else if (tid < kc) {
-        sm[tid] = __ldcg(&e.dq[e.c0 + tid]);
+    if (e.i0 == 0) {
+      // d, and ||P W||^2 = ||W||^2 - ||c||^2; where that is all cancellation
+      // the larger ||W||^2, with which the second subtraction is made
+      double d, c2;
+      kry_proj_sums<T>(a, nqo, out, flagged, d, c2);
+      const int w = tid >> 5;
+      if ((tid & 31) == 0 && w < kc) {
+        const double pw = nrm[w] - c2;
+        e.nrm0[e.c0 + w] = pw > 1e-3 * nrm[w] ? pw : nrm[w];
+        sm[w] = d;
+        if (flagged) e.dq[e.c0 + w] = d;
       }
-      __syncthreads();
+    } else if (flagged && tid < kc) {
+      sm[tid] = __ldcg(&e.dq[e.c0 + tid]);
     }
+    if (flagged) __syncthreads();
     for (int q = tid; q < nbo * kc; q += FRAG_BS) {
       const int p = (e.i0 + q / kc) * k + e.c0 + q % kc;
       const double h = (double)e.F[p] * (out[nqo * kc + q] - (flagged ? __ldcg(&e.gam[p]) * sm[q % kc] : 0.0));
       e.h1[p] = h;
       e.hv[p] = (T)((double)e.F[p] * h);
     }
-    if (tid < kc) e.nrm0[e.c0 + tid] = nrm[tid];
   } else if (is(KE_GS2)) {
     // A second subtraction where some norm fell below 1/sqrt(2) of its value
     // before the pass ("twice is enough"), or where the first one has left
