@@ -83,13 +83,17 @@ __global__ void k_gm_scale_cols(const T* __restrict__ src, int64_t lds, T* dst, 
 // y_s = H(0:J_s, 0:J_s, s)^{-1} g(0:J_s, s), J_s = jcount[s], stored negated
 // and with the basis factors as update coefficients: Y[i*k + s] = -F_i y_s(i)
 // for i < J_s, 0 up to Jmax (x -= sum_i V_i Y_i is then x += V y).  One warp
-// per system: lane l holds the rows l and l + 32 and the columns go from the
-// right, 4 columns of H loaded ahead of the chain of subtractions.
+// per system, 8 systems a block (the registers of 32 warps would not fit one
+// SM): lane l holds the rows l and l + 32 and the columns go from the right,
+// 4 columns of H loaded ahead of the chain of subtractions.
+constexpr int GM_SOLVE_NW = 8;
 template <class T>
-__global__ void k_gm_solve(const double* __restrict__ H, const double* __restrict__ g, const int* __restrict__ jcount,
-                           int k, int m, int Jmax, const T* __restrict__ F, T* Y)
+__global__ void __launch_bounds__(32 * GM_SOLVE_NW)
+k_gm_solve(const double* __restrict__ H, const double* __restrict__ g, const int* __restrict__ jcount, int k, int m,
+           int Jmax, const T* __restrict__ F, T* Y)
 {
-  const int s = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int s = blockIdx.x * GM_SOLVE_NW + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (s >= k) return;
   const int J = jcount[s];
   double v0 = lane < J ? g[lane * k + s] : 0.0;
   double v1 = lane + 32 < J ? g[(lane + 32) * k + s] : 0.0;
@@ -444,7 +448,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
     rt().sync();
     nconv = (int)(*hflags >> 32);
     const int J = steps;
-    k_gm_solve<T><<<1, 32 * k, 0, stream()>>>(H.p, g.p, jcount.p, k, m, J, F.p, Y.p);
+    k_gm_solve<T><<<(int)ceil_div(k, GM_SOLVE_NW), 32 * GM_SOLVE_NW, 0, stream()>>>(H.p, g.p, jcount.p, k, m, J, F.p, Y.p);
     PB_LAUNCH_CHECK();
     for_groups([&](KryArgs<T>& a0, int c0) {
       for (int i0 = 0; i0 < J; i0 += KRY_MAXJ) {

@@ -1,6 +1,6 @@
 """The passes of the device GMRES and MINRES (pb_krylov.cuh, pb_spmmv_lz.cuh)
 where their forms change: more than 24 basis blocks (several launches), more
-than 8 systems (groups of columns), projection blocks of 16, 17, 32 and 33
+than 8 systems (groups of columns; up to the 32 of a call), projection blocks of 16, 17, 32 and 33
 columns, no projection, 4 and 8 systems with the dots inside the SpMMV and
 the widths beside them, row counts that are no multiple of a tile, restarts,
 right-hand sides that are not orthogonal to the projection block.
@@ -21,6 +21,7 @@ pytestmark = pytest.mark.gpu
     ("LAPDIAG3D-9-S1", 5, 4, 27, 40), ("LAPDIAG3D-9-S1", 16, 8, 10, 10), ("LAPDIAG3D-9-S1", 17, 8, 10, 10),
     ("LAPDIAG3D-9-S2", 32, 4, 6, 6), ("LAPDIAG3D-9-S2", 33, 4, 6, 6), ("LAPDIAG3D-9-S3", 4, 9, 9, 9),
     ("LAPDIAG3D-9-S3", 20, 13, 6, 6), ("LAPDIAG3D-9-S3", 0, 17, 5, 5), ("LAPDIAG3D-10-S4", 3, 1, 12, 5),
+    ("LAPDIAG3D-9-S3", 4, 24, 6, 6), ("LAPDIAG3D-9-S3", 4, 25, 6, 4), ("LAPDIAG3D-9-S2", 0, 32, 7, 7),
     ("LAPDIAG3D-10-S4", 3, 5, 8, 8), ("HONEYCOMB-11x7-S3-W1", 2, 8, 7, 7)])
 def test_cut_off_iterate(session, oracle, problem, nq, k, steps, bas, solver):
     rp, c, v, Q, R, sigma = _setup(problem, nq, k, 7)
@@ -29,6 +30,15 @@ def test_cut_off_iterate(session, oracle, problem, nq, k, steps, bas, solver):
     ref, _ = getattr(oracle, "jada_" + solver)(A, Q, R, sigma, np.full(k, 1e-30), steps, bas)
     assert iflag == k
     assert relerr(t, ref) < 1e-9
+
+
+@pytest.mark.parametrize("solver", ["gmres", "minres"])
+def test_most_systems_single_precision(session, oracle, solver):
+    rp, c, v, Q, R, sigma = _setup("LAPDIAG3D-9-S5", 5, 32, 8)
+    R *= 1024.0 / np.linalg.norm(R, axis=0)
+    t, iflag = _run(rp, c, v, Q, R, sigma, 1e-30, 5, 5, dtype=np.float32, solver=solver)
+    ref, _ = getattr(oracle, "jada_" + solver)(_dense(rp, c, v), Q, R, sigma, np.full(32, 1e-30), 5, 5)
+    assert iflag == 32 and relerr(t, ref) < 1e-5
 
 
 @pytest.mark.parametrize("k", [4, 8])
