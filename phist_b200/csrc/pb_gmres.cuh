@@ -257,6 +257,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
     const int idx = resIndex ? resIndex[s] : s;
     PB_REQUIRE(idx >= 0 && idx < R->nvec, PB_INVALID_INPUT, "resIndex[%d] = %d out of range", s, idx);
   }
+  if (n == 0) return 0;  // every residual is zero: converged with no step
   const int nq = Q ? Q->nvec : 0;
   const int m = std::max(1, std::min(std::min(maxBas > 0 ? maxBas : maxIter, maxIter), 63));
   const int64_t nk = n * (int64_t)k;  // one basis block

@@ -98,3 +98,13 @@ def test_single_precision_not_orthogonal_to_q(session, oracle, solver):
     t, _ = _run(rp, c, v, Q, 1024 * R, sigma, 1e-30, 5, 5, dtype=np.float32, solver=solver)
     ref, _ = getattr(oracle, "jada_" + solver)(_dense(rp, c, v), Q, 1024 * R, sigma, np.full(4, 1e-30), 5, 5)
     assert relerr(t, ref) < 1e-5
+
+
+@pytest.mark.parametrize("solver", ["gmres", "minres"])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_no_rows(session, solver, dtype):
+    """a matrix without rows: every residual is zero, all systems converged"""
+    for nq in (0, 3):
+        t, iflag = _run(np.zeros(1, np.int64), np.zeros(0, np.int32), np.zeros(0), np.zeros((0, nq)), np.zeros((0, 4)),
+                        np.ones(4), 1e-6, 5, 5, dtype=dtype, solver=solver)
+        assert iflag == 0 and t.shape == (0, 4)
