@@ -118,7 +118,7 @@ __global__ void k_copy(const TI* __restrict__ x, int64_t ldx, TO* y, int64_t ldy
       const int64_t e = t + u * step, i = pb_elem_row(e < tot ? e : t, nvec, tot);
       const int64_t j = (e < tot ? e : t) - i * nvec;
       at[u] = i * ldy + j;
-      v[u] = __ldg(x + i * ldx + j);
+      GlobalLd<TI, 1>::ld(x + i * ldx + j, &v[u]);
     }
 #pragma unroll
     for (int u = 0; u < 4; u++)

@@ -260,7 +260,9 @@ inline cudaStream_t stream() { return rt().stream(); }
 // Launch with a programmatic dependency on the previous kernel of the stream:
 // the blocks may start while that kernel drains, do what does not depend on
 // it and wait in pdl_wait() (pb_reduce.cuh) for its end and its memory.  Only
-// for kernels that call pdl_wait() before they touch anything a kernel writes.
+// for kernels that call pdl_wait() before they touch anything a kernel writes,
+// and read that with coherent loads (GlobalLd, frag_ld1, __ldcg): it is not
+// read-only for their lifetime.
 template <class... KA, class... A>
 inline void launch_pdl(void (*kern)(KA...), int grid, int block, size_t smem, const A&... args)
 {

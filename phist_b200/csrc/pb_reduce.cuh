@@ -20,6 +20,72 @@ namespace pb {
 __device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Coherent loads of W consecutive elements, W * sizeof(T) bytes at a boundary
+// of that size.  The blocks of a kernel with a programmatic dependency are
+// there while the kernel before still writes, so what that one may have
+// written is not read-only for their lifetime: no non-coherent loads (__ldg,
+// ld.global.nc), and none that the compiler may move over pdl_wait().
+// Volatile, so that they are issued in the order they are written down.
+template <class T, int W>
+struct GlobalLd;
+template <>
+struct GlobalLd<double, 1> {
+  static __device__ __forceinline__ void ld(const double* p, double* o)
+  {
+    asm volatile("ld.global.f64 %0, [%1];\n" : "=d"(o[0]) : "l"(p));
+  }
+};
+template <>
+struct GlobalLd<float, 1> {
+  static __device__ __forceinline__ void ld(const float* p, float* o)
+  {
+    asm volatile("ld.global.f32 %0, [%1];\n" : "=f"(o[0]) : "l"(p));
+  }
+};
+template <>
+struct GlobalLd<double, 2> {
+  static __device__ __forceinline__ void ld(const double* p, double* o)
+  {
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];\n" : "=d"(o[0]), "=d"(o[1]) : "l"(p));
+  }
+};
+template <>
+struct GlobalLd<float, 2> {
+  static __device__ __forceinline__ void ld(const float* p, float* o)
+  {
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];\n" : "=f"(o[0]), "=f"(o[1]) : "l"(p));
+  }
+};
+template <>
+struct GlobalLd<float, 4> {
+  static __device__ __forceinline__ void ld(const float* p, float* o)
+  {
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3])
+                 : "l"(p));
+  }
+};
+// 256-bit forms (sm_100)
+template <>
+struct GlobalLd<double, 4> {
+  static __device__ __forceinline__ void ld(const double* p, double* o)
+  {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];\n"
+                 : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
+                 : "l"(p)
+                );
+  }
+};
+template <>
+struct GlobalLd<float, 8> {
+  static __device__ __forceinline__ void ld(const float* p, float* o)
+  {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
+                 : "l"(p));
+  }
+};
+
 template <class T>
 struct Acc;  // accumulation type
 template <>

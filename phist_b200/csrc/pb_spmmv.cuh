@@ -64,140 +64,49 @@ struct SpmvArgs {
   int no_store;
 };
 
+// W consecutive elements of a block row: coherent loads, issued in program
+// order (GlobalLd), and stores
 template <class T, int W>
-struct VecLd;
-template <>
-struct VecLd<double, 2> {
-  static __device__ __forceinline__ void ld(const double* p, double* o)
+struct Vec : GlobalLd<T, W> {
+  // the same without the order; 16 bytes at most also from shared memory
+  static __device__ __forceinline__ void ld_plain(const T* p, T* o)
   {
-    double2 v = __ldg(reinterpret_cast<const double2*>(p));
-    o[0] = v.x; o[1] = v.y;
+    if constexpr (W * sizeof(T) == 32) {
+      GlobalLd<T, W>::ld(p, o);
+    } else if constexpr (W == 4) {
+      const float4 v = *reinterpret_cast<const float4*>(p);
+      o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+    } else if constexpr (W == 2 && sizeof(T) == 8) {
+      const double2 v = *reinterpret_cast<const double2*>(p);
+      o[0] = v.x; o[1] = v.y;
+    } else if constexpr (W == 2) {
+      const float2 v = *reinterpret_cast<const float2*>(p);
+      o[0] = v.x; o[1] = v.y;
+    } else {
+      o[0] = *p;
+    }
   }
-  static __device__ __forceinline__ void ld_plain(const double* p, double* o)
+  static __device__ __forceinline__ void st(T* p, const T* o)
   {
-    double2 v = *reinterpret_cast<const double2*>(p);
-    o[0] = v.x; o[1] = v.y;
-  }
-  static __device__ __forceinline__ void ld_ordered(const double* p, double* o)
-  {
-    asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];\n" : "=d"(o[0]), "=d"(o[1]) : "l"(p));
-  }
-  static __device__ __forceinline__ void st(double* p, const double* o)
-  {
-    *reinterpret_cast<double2*>(p) = make_double2(o[0], o[1]);
-  }
-};
-// 256-bit forms (sm_100): one load or store moves 32 bytes
-template <>
-struct VecLd<double, 4> {
-  static __device__ __forceinline__ void ld(const double* p, double* o) { ld_ordered(p, o); }
-  static __device__ __forceinline__ void ld_plain(const double* p, double* o)
-  {
-    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];\n"
-                 : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
-                 : "l"(p));
-  }
-  static __device__ __forceinline__ void ld_ordered(const double* p, double* o)
-  {
-    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];\n"
-                 : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
-                 : "l"(p));
-  }
-  static __device__ __forceinline__ void st(double* p, const double* o)
-  {
-    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "d"(o[0]), "d"(o[1]), "d"(o[2]), "d"(o[3])
-                 : "memory");
+    if constexpr (sizeof(T) == 8 && W == 4)
+      asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "d"(o[0]), "d"(o[1]), "d"(o[2]), "d"(o[3])
+                   : "memory");
+    else if constexpr (sizeof(T) == 4 && W == 8)
+      asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(p), "f"(o[0]), "f"(o[1]),
+                   "f"(o[2]), "f"(o[3]), "f"(o[4]), "f"(o[5]), "f"(o[6]), "f"(o[7])
+                   : "memory");
+    else if constexpr (W == 4)
+      *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
+    else if constexpr (W == 2 && sizeof(T) == 8)
+      *reinterpret_cast<double2*>(p) = make_double2(o[0], o[1]);
+    else if constexpr (W == 2)
+      *reinterpret_cast<float2*>(p) = make_float2(o[0], o[1]);
+    else
+      *p = o[0];
   }
 };
-template <>
-struct VecLd<float, 8> {
-  static __device__ __forceinline__ void ld(const float* p, float* o) { ld_ordered(p, o); }
-  static __device__ __forceinline__ void ld_plain(const float* p, float* o)
-  {
-    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
-                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
-                 : "l"(p));
-  }
-  static __device__ __forceinline__ void ld_ordered(const float* p, float* o)
-  {
-    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
-                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
-                 : "l"(p));
-  }
-  static __device__ __forceinline__ void st(float* p, const float* o)
-  {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(p), "f"(o[0]), "f"(o[1]),
-                 "f"(o[2]), "f"(o[3]), "f"(o[4]), "f"(o[5]), "f"(o[6]), "f"(o[7])
-                 : "memory");
-  }
-};
-template <>
-struct VecLd<float, 4> {
-  static __device__ __forceinline__ void ld(const float* p, float* o)
-  {
-    float4 v = __ldg(reinterpret_cast<const float4*>(p));
-    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-  }
-  static __device__ __forceinline__ void ld_plain(const float* p, float* o)
-  {
-    float4 v = *reinterpret_cast<const float4*>(p);
-    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-  }
-  static __device__ __forceinline__ void ld_ordered(const float* p, float* o)
-  {
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n"
-                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3])
-                 : "l"(p));
-  }
-  static __device__ __forceinline__ void st(float* p, const float* o)
-  {
-    *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
-  }
-};
-template <>
-struct VecLd<float, 2> {
-  static __device__ __forceinline__ void ld(const float* p, float* o)
-  {
-    float2 v = __ldg(reinterpret_cast<const float2*>(p));
-    o[0] = v.x; o[1] = v.y;
-  }
-  static __device__ __forceinline__ void ld_plain(const float* p, float* o)
-  {
-    float2 v = *reinterpret_cast<const float2*>(p);
-    o[0] = v.x; o[1] = v.y;
-  }
-  static __device__ __forceinline__ void ld_ordered(const float* p, float* o)
-  {
-    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];\n" : "=f"(o[0]), "=f"(o[1]) : "l"(p));
-  }
-  static __device__ __forceinline__ void st(float* p, const float* o)
-  {
-    *reinterpret_cast<float2*>(p) = make_float2(o[0], o[1]);
-  }
-};
-__device__ __forceinline__ void ld_ordered1(const double* p, double* o)
-{
-  asm volatile("ld.global.nc.f64 %0, [%1];\n" : "=d"(o[0]) : "l"(p));
-}
-__device__ __forceinline__ void ld_ordered1(const float* p, float* o)
-{
-  asm volatile("ld.global.nc.f32 %0, [%1];\n" : "=f"(o[0]) : "l"(p));
-}
 __device__ __forceinline__ void reg_fence(double& v) { asm volatile("" : "+d"(v)); }
 __device__ __forceinline__ void reg_fence(float& v) { asm volatile("" : "+f"(v)); }
-template <class T>
-struct VecLd1 {
-  static __device__ __forceinline__ void ld(const T* p, T* o) { o[0] = __ldg(p); }
-  static __device__ __forceinline__ void ld_ordered(const T* p, T* o) { ld_ordered1(p, o); }
-  static __device__ __forceinline__ void ld_plain(const T* p, T* o) { o[0] = *p; }
-  static __device__ __forceinline__ void st(T* p, const T* o) { *p = o[0]; }
-};
-template <class T, int W>
-struct Vec : VecLd<T, W> {};
-template <>
-struct Vec<double, 1> : VecLd1<double> {};
-template <>
-struct Vec<float, 1> : VecLd1<float> {};
 
 // column handled by (lane-in-row s, vector v, element w)
 template <int TPR, int VW>
@@ -213,7 +122,11 @@ __device__ __forceinline__ void spmv_cscale(const SpmvArgs<T>& p, int c, AT* acc
 {
   if (p.cscale) {
 #pragma unroll
-    for (int w = 0; w < VW; w++) acc[w] *= AT(__ldg(p.cscale + p.col0 + c + w));
+    for (int w = 0; w < VW; w++) {
+      T f;
+      GlobalLd<T, 1>::ld(p.cscale + p.col0 + c + w, &f);  // the pass before has written it
+      acc[w] *= AT(f);
+    }
   }
 }
 
@@ -308,7 +221,7 @@ k_sell_spmmv(SellDev<T> A, SpmvArgs<T> p)
       for (int v = 0; v < NVV; v++) {
         const int c = spmv_col<TPR, VW>(s, v, 0);
         if (VEC || c < nv) {
-          Vec<T, VW>::ld_ordered(xr + c, &xv[k][v * VW]);
+          Vec<T, VW>::ld(xr + c, &xv[k][v * VW]);
         } else {
 #pragma unroll
           for (int w = 0; w < VW; w++) xv[k][v * VW + w] = T(0);

@@ -400,7 +400,7 @@ __device__ __forceinline__ void sell_spmmv_pf(const SellDev<T>& A, const SpmvArg
       for (int k = 0; k < KMAX; k++) {
         const T* xr = x + (int64_t)cv[k] * p.ldx;
 #pragma unroll
-        for (int v = 0; v < NVV; v++) Vec<T, VW>::ld_ordered(xr + lcol(v), &xv[k][v * VW]);
+        for (int v = 0; v < NVV; v++) Vec<T, VW>::ld(xr + lcol(v), &xv[k][v * VW]);
       }
 #pragma unroll
       for (int k = 0; k < KMAX; k++)
@@ -641,7 +641,7 @@ __global__ void __launch_bounds__(NT) k_sell_spmmv_long(SellDev<T> A, SpmvArgs<T
       a[q] = av[q];
       const T* xr = x + (int64_t)cv[q] * p.ldx;
 #pragma unroll
-      for (int v = 0; v < NVV; v++) Vec<T, VW>::ld_ordered(xr + lcol(v), &xv[q][v * VW]);
+      for (int v = 0; v < NVV; v++) Vec<T, VW>::ld(xr + lcol(v), &xv[q][v * VW]);
     }
     if (k0 + KB < len) entries(k0 + KB);
 #pragma unroll
