@@ -241,6 +241,23 @@ static void gm_mvsd(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, c
   launch_rowgemm<T>(a);
 }
 
+// More than KRY_MAXC systems: in one solve, whose passes go over groups of
+// KRY_MAXC columns of blocks that are k columns wide and share the SpMMV and
+// the products with a wide Q, or in solves of KRY_MAXC systems each, whose
+// blocks are contiguous.  A pass over a part of wide rows moves its data at
+// three quarters of the rate, but the fewer launches win on small problems.
+// 15 steps, us, one solve | several (nq = 32 unless named):
+//   GMRES FP64 16 systems  32^3 1,621 | 1,609  40^3 2,260 | 1,801  64^3 6,549 | 4,977
+//   GMRES FP32 16 systems  40^3 1,521 | 1,564  48^3 2,259 | 2,055  64^3 4,161 | 3,579
+//   MINRES FP64 16 / 24    48^3 1,447 | 1,470, 2,496 | 2,220  64^3 2,714 | 2,561, 4,869 | 3,841
+//   MINRES FP32 16 / 24    48^3 1,190 | 1,228, 1,836 | 1,849  64^3 1,964 | 1,955, 3,330 | 2,941
+//   MINRES FP64 16, nq = 40 (projection in products of its own)  64^3 2,664 | 2,814
+inline bool gm_split(bool lanczos, bool fuse, int64_t n, size_t elem)
+{
+  const size_t column = (size_t)n * elem;
+  return lanczos ? fuse && column >= (1u << 20) : column >= (400u << 10);
+}
+
 // lanczos: MINRES (three-term recurrence), else GMRES
 template <class T>
 int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const int* resIndex, int k,
@@ -259,6 +276,21 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
   }
   if (n == 0) return 0;  // every residual is zero: converged with no step
   const int nq = Q ? Q->nvec : 0;
+  // a projection block of at most KRY_MAXQ columns goes with the passes over
+  // the basis, a wider one in products of its own
+  const bool fuse = nq > 0 && nq <= KRY_MAXQ;
+  if (k > KRY_MAXC && gm_split(lanczos, fuse || nq == 0, n, sizeof(T))) {
+    int unconverged = 0;
+    for (int c0 = 0; c0 < k; c0 += KRY_MAXC) {
+      const int kc = std::min(KRY_MAXC, k - c0);
+      std::vector<int> idx(kc);
+      for (int s = 0; s < kc; s++) idx[s] = resIndex ? resIndex[c0 + s] : c0 + s;
+      Mvec<T> tc;
+      raw_view(tc, t->d() + c0, n, kc, t->lda);
+      unconverged += jada_krylov<T>(A, Q, R, idx.data(), kc, sigma + c0, tol + c0, maxIter, maxBas, &tc, lanczos);
+    }
+    return unconverged;
+  }
   const int m = std::max(1, std::min(std::min(maxBas > 0 ? maxBas : maxIter, maxIter), 63));
   const int64_t nk = n * (int64_t)k;  // one basis block
   const double eps_abs = (lanczos ? 100.0 : 1000.0) * std::numeric_limits<T>::epsilon();
@@ -274,9 +306,6 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
   for (int s = 0; s < k; s++) negsig[s] = (T)(-sigma[s]);
   volatile unsigned long long* hflags = (volatile unsigned long long*)rt().mailbox_host();
   const int gw = grid_for(n * (int64_t)k);
-  // a projection block of at most KRY_MAXQ columns goes with the passes over
-  // the basis, a wider one in products of its own
-  const bool fuse = nq > 0 && nq <= KRY_MAXQ;
   DBuf<double> gq((size_t)(fuse ? nq + m + 2 : 0) * k);  // g0, gam, dq
 
   Mvec<T> mX, mW, mVj;
