@@ -1482,8 +1482,13 @@ bool launch_rowgemm(RowGemmArgs<T>& a, T* mbox = nullptr)
     PB_LAUNCH_CHECK();
     return false;
   }
-  // fused Gram at the other widths: a second pass over the new W
-  if (a.gram != GM_NONE && a.mode != RM_VCWD && (a.gram == GM_WW || a.mv <= 64) && frag_mvsd(a)) {
+  // fused Gram at the other widths: a second pass over the new W (4 columns of
+  // W with 20 of V, n = 2,097,152: 116 us, in one pass of the tiled kernel
+  // below 362; at 2,048 rows 25 and 27)
+  if (a.gram != GM_NONE && a.mode != RM_VCWD && a.m <= 64 && a.k <= 64 && (a.gram == GM_WW || a.mv <= 64)) {
+    RowGemmArgs<T> p = a;
+    p.gram = GM_NONE;
+    launch_rowgemm<T>(p);
     if (a.gram == GM_WW)
       launch_mvTmv<T>(a.n, a.k, a.k, T(1), a.W, a.ldw, a.W, a.ldw, T(0), a.Gd, a.ldg);
     else

@@ -124,3 +124,29 @@ def test_product_with_gram(session, n, m, k, ld, dtype):
     assert np.abs(D.get() - (2.0 * new.T @ new + np.eye(k))).max() <= 2 * (n + 3) * (n * np.finfo(np.float64).eps + eps)
     for o in (X, D, V, W, C, G, Vb, Wb, mp, mq):
         o.delete()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("mv,k,off", [(1, 4, 0), (8, 4, 0), (9, 4, 0), (20, 4, 0), (10, 2, 1), (37, 3, 1), (64, 1, 0), (16, 16, 0),
+                                      (24, 24, 0), (32, 32, 0), (64, 32, 0), (33, 33, 1), (40, 64, 0), (64, 64, 0)])
+@pytest.mark.parametrize("n", [0, 1, 5003])
+def test_in_place_product_with_another_block(session, n, mv, k, off, dtype):
+    """W = W C in place and D = a V'W + b D of the new W, V another block.  A
+    row of W is a sum of k products of size at most 1/k; the sum over n rows of
+    products of size at most 1 rounds by at most n eps per term in FP32"""
+    from phist_b200 import kernels as K
+    from phist_b200.objects import SdMat, fn
+    rng = np.random.default_rng(n + mv + k)
+    eps = np.finfo(dtype).eps
+    mp, Vb, V, v = _block(n, mv + 2 * off, off, mv, rng, dtype)
+    mq, Wb, W, w = _block(n, k + 2 * off, off, k, rng, dtype)
+    c = (rng.uniform(-1, 1, (k, k)) / k).astype(dtype)
+    d0 = rng.uniform(-1, 1, (mv, k)).astype(dtype)
+    C, D = SdMat(k, k, dtype).set(c), SdMat(mv, k, dtype).set(d0)
+    K.chk(fn(dtype, "fused_mvsdi_mvTmv"), 0.5, V.h, W.h, C.h, 2.0, D.h)
+    new = W.get().astype(np.float64)
+    assert np.abs(new - w @ c.astype(np.float64)).max(initial=0) <= (k + 3) * 2 * eps
+    terms = np.abs(v).T @ np.abs(new)
+    assert (np.abs(D.get() - (0.5 * v.T @ new + 2.0 * d0)) <= (n + 3) * eps * (terms + 4)).all()
+    for o in (V, W, C, D, Vb, Wb, mp, mq):
+        o.delete()
