@@ -1455,10 +1455,16 @@ bool launch_rowgemm(RowGemmArgs<T>& a, T* mbox = nullptr)
 {
   if (a.n == 0 && a.gram == GM_NONE) return false;
   // fused V*C + Gram in one pass on the tensor cores
-  if (a.gram == GM_WW && a.mode != RM_VCWD && frag_mvsd_gram<T>(a, mbox)) return mbox != nullptr;
+  // Thin blocks of many rows stay with the register kernel, whose rows cost
+  // less (us, fragments | registers: FP64 4 x 4 at 1,048,576 rows 37.5 | 39.5, at
+  // 1,572,864 53 | 52; 1 x 1 at 524,288 24.8 | 27.1, at 786,432 29.2 | 27.2; FP32
+  // 4 x 4 at 262,144 23.6 | 26.8, at 524,288 30.3 | 28.5, at 2,097,152 69 | 39),
+  // the others have the shorter cross-block sum and the result in the mailbox
+  const bool thin = a.k <= 4 && a.m <= (sizeof(T) == 4 ? 8 : 4);
+  const bool many = a.n > (sizeof(T) == 8 && a.k >= 2 ? 1 << 20 : 1 << 19);
+  if (a.gram == GM_WW && a.mode != RM_VCWD && !(thin && many) && frag_mvsd_gram<T>(a, mbox)) return mbox != nullptr;
   if (mvsd_gram_dmma(a)) return false;
   if (a.gram == GM_NONE && a.mode != RM_VCWD && frag_mvsd(a)) return false;
-  const bool thin = a.k <= 4 && a.m <= (sizeof(T) == 4 ? 8 : 4);
   if (a.m <= 8 && a.k <= 8 && (thin || a.mode == RM_VCWD) && (a.gram != GM_VW || a.mv <= 8)) {
     // register kernel (thin blocks, V C + W D): padded widths M (4|8), K (1|4|8), MV (1, or 8 for V'W)
     const int M = a.m <= 4 ? 4 : 8, K = a.k == 1 ? 1 : a.k <= 4 ? 4 : 8;

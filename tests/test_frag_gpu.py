@@ -150,3 +150,28 @@ def test_in_place_product_with_another_block(session, n, mv, k, off, dtype):
     assert (np.abs(D.get() - (0.5 * v.T @ new + 2.0 * d0)) <= (n + 3) * eps * (terms + 4)).all()
     for o in (V, W, C, D, Vb, Wb, mp, mq):
         o.delete()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("m,k", [(1, 1), (4, 1), (3, 2), (4, 4), (8, 4)])
+@pytest.mark.parametrize("n", [(1 << 19) + 3, (1 << 20) + 3])
+def test_thin_product_with_gram_of_many_rows(session, n, m, k, dtype):
+    """where the fused W'W of thin blocks changes its kernel; bounds as above"""
+    from phist_b200 import kernels as K
+    from phist_b200.objects import SdMat, fn
+    rng = np.random.default_rng(m + k)
+    eps = np.finfo(dtype).eps
+    mp, Vb, V, v = _block(n, m, 0, m, rng, dtype)
+    mq, Wb, W, w = _block(n, k, 0, k, rng, dtype)
+    c = (rng.uniform(-1, 1, (m, k)) / m).astype(dtype)
+    C, G = SdMat(m, k, dtype).set(c), SdMat(k, k, dtype)
+    K.chk(fn(dtype, "fused_mvsd_mvTmv"), 0.5, V.h, C.h, -0.5, W.h, G.h)
+    new = W.get().astype(np.float64)
+    assert np.abs(new - (0.5 * (v @ c.astype(np.float64)) - 0.5 * w)).max() <= (m + 3) * 2 * eps
+    # FP32 sums: lanes of at most 2^20 / (256 * 148) rows, then the tree over
+    # lanes, warps and blocks, some 60 roundings of the terms' sum in all
+    g = G.get()
+    assert (np.abs(g - new.T @ new) <= 100 * eps * (np.abs(new).T @ np.abs(new))).all()
+    assert np.array_equal(G.host(), g)
+    for o in (V, W, C, G, Vb, Wb, mp, mq):
+        o.delete()
