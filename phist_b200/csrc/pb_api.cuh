@@ -1470,7 +1470,7 @@ bool launch_rowgemm(RowGemmArgs<T>& a, T* mbox = nullptr)
     const int M = a.m <= 4 ? 4 : 8, K = a.k == 1 ? 1 : a.k <= 4 ? 4 : 8;
     const int grid = std::max(1, std::min(grid_for(a.n), rt().num_sms() * 4));
     if (a.gram != GM_NONE) {
-      a.part = (T*)rt().scratch(sizeof(T) * (size_t)grid * 64);
+      a.part = (T*)rt().scratch(sizeof(double) * (size_t)grid * 64);
       a.counter = rt().counters();
     }
 #define PB_RGR(Mv, Kv, MVv) k_rowgemm_reg<T, Mv, Kv, MVv><<<grid, 256, 0, stream()>>>(a)

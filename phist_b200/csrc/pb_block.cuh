@@ -417,7 +417,9 @@ __global__ void __launch_bounds__(256) k_mvTmv_v4(MvTmvArgs<double> a)
   last_block_reduce<double>(a.part, M * K, gridDim.x, a.counter, a.Cd, 1, M, a.ldc, a.alpha, a.beta, a.m, a.k, a.mbox);
 }
 
-// row-local products for m, k, mv <= 8 (modes and Gram as k_rowgemm)
+// Row-local products for m, k, mv <= 8 (modes and Gram as k_rowgemm, the Gram
+// for k <= 4 only).  The Gram products are formed and summed in FP64 in both
+// precisions, as in pb_frag.cuh, and rounded once; a.part is FP64.
 template <class T, int M, int K, int MV>
 __global__ void __launch_bounds__(256) k_rowgemm_reg(RowGemmArgs<T> a)
 {
@@ -433,10 +435,11 @@ __global__ void __launch_bounds__(256) k_rowgemm_reg(RowGemmArgs<T> a)
       sD[t] = (i < a.k && j < a.k) ? a.D[i + j * a.ldd] : T(0);
     }
   __syncthreads();
-  constexpr int GM = (MV > K) ? MV : K;
-  T gacc[GM * K];
+  constexpr bool GRAM = K <= 4;
+  constexpr int GM = (MV > K) ? MV : K, NG = GRAM ? GM * K : 1;
+  double gacc[NG];
 #pragma unroll
-  for (int q = 0; q < GM * K; q++) gacc[q] = T(0);
+  for (int q = 0; q < NG; q++) gacc[q] = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
        i += (int64_t)gridDim.x * blockDim.x) {
     T v[8], w[8], out[8];
@@ -460,28 +463,33 @@ __global__ void __launch_bounds__(256) k_rowgemm_reg(RowGemmArgs<T> a)
 #pragma unroll
     for (int q = 0; q < K; q++)
       if (q < a.k) a.W[i * a.ldw + q] = out[q];
-    if (a.gram == GM_WW) {
+    if constexpr (GRAM) {
+      if (a.gram == GM_WW) {
 #pragma unroll
-      for (int q = 0; q < K; q++)
+        for (int q = 0; q < K; q++)
 #pragma unroll
-        for (int p = 0; p < K; p++) gacc[p + q * K] += out[p] * out[q];
-    } else if (a.gram == GM_VW) {
-      T g[8];
-      load_row(a.Vg + i * a.ldvg, a.mv, MV, g);
+          for (int p = 0; p < K; p++) gacc[p + q * K] += (double)out[p] * (double)out[q];
+      } else if (a.gram == GM_VW) {
+        T g[8];
+        load_row(a.Vg + i * a.ldvg, a.mv, MV, g);
 #pragma unroll
-      for (int q = 0; q < K; q++)
+        for (int q = 0; q < K; q++)
 #pragma unroll
-        for (int p = 0; p < MV; p++) gacc[p + q * MV] += g[p] * out[q];
+          for (int p = 0; p < MV; p++) gacc[p + q * MV] += (double)g[p] * (double)out[q];
+      }
     }
   }
-  if (a.gram == GM_NONE) return;
-  const int gmax = (a.gram == GM_WW) ? K : MV;
-  // partial layout: gmax rows (padded), K columns
-  block_partial<T, GM * K>(gacc, a.part, gmax * K);
-  const T al = (a.gram == GM_WW) ? T(1) : a.galpha;
-  const T be = (a.gram == GM_WW) ? T(0) : a.gbeta;
-  last_block_reduce<T>(a.part, gmax * K, gridDim.x, a.counter, a.Gd, 1, gmax, a.ldg, al, be,
-                       (a.gram == GM_WW) ? a.k : a.mv, a.k);
+  if constexpr (GRAM) {
+    if (a.gram == GM_NONE) return;
+    const int gmax = (a.gram == GM_WW) ? K : MV;
+    // partial layout: gmax rows (padded), K columns
+    double* part = reinterpret_cast<double*>(a.part);
+    block_partial<double, NG>(gacc, part, gmax * K);
+    const double al = (a.gram == GM_WW) ? 1.0 : (double)a.galpha;
+    const double be = (a.gram == GM_WW) ? 0.0 : (double)a.gbeta;
+    last_block_reduce<double>(part, gmax * K, gridDim.x, a.counter, a.Gd, 1, gmax, a.ldg, al, be,
+                              (a.gram == GM_WW) ? a.k : a.mv, a.k);
+  }
 }
 
 }  // namespace pb

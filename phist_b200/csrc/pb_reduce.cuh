@@ -120,12 +120,12 @@ __device__ __forceinline__ T block_sum_mod(T v, int w, T* red)
   return s;
 }
 
-template <class T>
+template <class T, class TO = T>
 __device__ __forceinline__ bool last_block_reduce(const T* part, int nout, int nblocks,
-                                                  unsigned int* counter, T* out,
+                                                  unsigned int* counter, TO* out,
                                                   int64_t out_stride_rows, int out_rows,
                                                   int64_t ld_out, T alpha, T beta,
-                                                  int vrows = 1 << 30, int vcols = 1 << 30, T* mbox = nullptr)
+                                                  int vrows = 1 << 30, int vcols = 1 << 30, TO* mbox = nullptr)
 {
   __shared__ bool am_last;
   __shared__ T red[256];  // all callers launch at most 256 threads per block
@@ -183,8 +183,8 @@ __device__ __forceinline__ bool last_block_reduce(const T* part, int nout, int n
       const int o = o0 + threadIdx.x;
       const int r = o % out_rows, c = o / out_rows;
       if (r < vrows && c < vcols) {
-        T* dst = out + r * out_stride_rows + (int64_t)c * ld_out;
-        const T v = (beta == T(0)) ? alpha * s : alpha * s + beta * (*dst);
+        TO* dst = out + r * out_stride_rows + (int64_t)c * ld_out;
+        const TO v = (TO)((beta == T(0)) ? alpha * s : alpha * s + beta * (T)*dst);
         *dst = v;
         if (mbox) mbox[r + c * min(vrows, out_rows)] = v;
       }
