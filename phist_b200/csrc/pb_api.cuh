@@ -1473,6 +1473,15 @@ bool launch_rowgemm(RowGemmArgs<T>& a, T* mbox = nullptr)
       a.part = (T*)rt().scratch(sizeof(double) * (size_t)grid * 64);
       a.counter = rt().counters();
     }
+    if constexpr (sizeof(T) == 8) {
+      auto rows32 = [](const T* p, int64_t ld) { return (uintptr_t)p % 32 == 0 && ld % 4 == 0; };
+      if (a.m == 4 && a.k == 4 && rows32(a.W, a.ldw) && (a.mode == RM_MVSDI || rows32(a.V, a.ldv))) {
+        if (a.gram == GM_VW) k_rowgemm_reg<T, 4, 4, 8, true><<<grid, 256, 0, stream()>>>(a);
+        else k_rowgemm_reg<T, 4, 4, 1, true><<<grid, 256, 0, stream()>>>(a);
+        PB_LAUNCH_CHECK();
+        return false;
+      }
+    }
 #define PB_RGR(Mv, Kv, MVv) k_rowgemm_reg<T, Mv, Kv, MVv><<<grid, 256, 0, stream()>>>(a)
 #define PB_RGR_K(Mv, MVv)                                   \
   if (K == 1) PB_RGR(Mv, 1, MVv);                           \

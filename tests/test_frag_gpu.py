@@ -173,3 +173,38 @@ def test_thin_product_with_gram_of_many_rows(session, n, m, k, dtype):
     assert np.array_equal(G.host(), g)
     for o in (V, W, C, G, Vb, Wb, mp, mq):
         o.delete()
+
+
+@pytest.mark.parametrize("vld,vo,wld,wo", [(4, 0, 4, 0), (8, 4, 12, 4), (8, 2, 4, 0), (4, 0, 6, 0), (5, 1, 8, 4)])
+@pytest.mark.parametrize("n", [1, 255, 5003])
+def test_four_columns(session, n, vld, vo, wld, wo):
+    """4 x 4 in FP64, rows on 32-byte boundaries (moved whole) and off them:
+    every form of the row kernel; columns beside the views stay as they are"""
+    from phist_b200 import kernels as K
+    from phist_b200.objects import SdMat
+    rng = np.random.default_rng(n + vld)
+    eps = np.finfo(np.float64).eps
+    mp, Vb, V, v = _block(n, vld, vo, 4, rng, np.float64)
+    mq, Wb, W, w = _block(n, wld, wo, 4, rng, np.float64)
+    c, d = rng.uniform(-1, 1, (4, 4)) / 4, rng.uniform(-1, 1, (4, 4)) / 4
+    C, D, G = SdMat(4, 4).set(c), SdMat(4, 4).set(d), SdMat(4, 4)
+
+    def check(ref):
+        got = Wb.get()
+        assert np.abs(got[:, wo:wo + 4] - ref).max() <= 14 * eps
+        assert np.isnan(np.delete(got, np.s_[wo:wo + 4], axis=1)).all()
+        return got[:, wo:wo + 4]
+
+    K.chk(K.phist_Dmvec_times_sdMat, 0.5, V.h, C.h, 0.0, W.h)
+    w = check(0.5 * v @ c)
+    K.chk(K.phist_Dmvec_times_sdMat, 0.5, V.h, C.h, 2.0, W.h)
+    w = check(0.5 * v @ c + 2.0 * w)
+    K.chk(K.phist_Dmvec_times_sdMat_inplace, W.h, D.h)
+    w = check(w @ d)
+    K.chk(K.phist_Dmvec_times_sdMat_add_mvec_times_sdMat, V.h, C.h, W.h, D.h)
+    w = check(v @ c + w @ d)
+    K.chk(K.phist_Dfused_mvsdi_mvTmv, 1.0, V.h, W.h, C.h, 0.0, G.h)
+    w = check(w @ c)
+    assert np.abs(G.get() - v.T @ w).max() <= (n + 3) * (n + 3) * eps
+    for o in (V, W, C, D, G, Vb, Wb, mp, mq):
+        o.delete()
