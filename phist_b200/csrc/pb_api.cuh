@@ -1433,18 +1433,25 @@ bool mvsd_gram_dmma_mv(RowGemmArgs<double>& a, int MV)
 }
 
 // True if the fused tensor-core kernel took W(:,0:k) = W C with V'W of another
-// block V.  Up to 16 columns: beyond, its shared-memory tiles leave one or two
-// blocks per SM and the product followed by V'W is faster (n = 2,097,152,
-// square: fused 80 / 150 / 395 us at 8 / 16 / 32 columns, the two passes of
-// pb_frag.cuh 113 / 208 / 389 us).
+// block V.  Up to 16 columns always; beyond, its shared-memory tiles leave one
+// or two blocks per SM, but up to a number of rows the one launch still wins
+// over the product followed by V'W, fewer where the padding to 32 or 64
+// columns is more than a quarter, and not with 16 columns of V or fewer (V x W
+// columns, us, two passes | fused: 24 x 24 at 131,072 rows 57 | 55, at 262,144 72 |
+// 80; 64 x 32 at 32,768 58 | 44, at 524,288 185 | 169; 32 x 32 at 1,048,576 229 |
+// 228, at 2,097,152 394 | 413; 40 x 40 at 131,072 107 | 105, at 262,144 169 | 180;
+// 64 x 64 at 65,536 84 | 72, at 524,288 345 | 341; 16 x 40 at 131,072 72 | 80).
 inline bool mvsd_gram_dmma(RowGemmArgs<double>& a)
 {
   if (!rt().use_tma || !rt().use_dmma || a.mode == RM_VCWD || a.gram != GM_VW) return false;
-  if (a.m > 16 || a.k > 16 || a.m < 5 || a.k < 5) return false;  // widths <= 4: register kernel
+  if (a.m > 64 || a.k > 64 || a.m < 5 || a.k < 5) return false;  // widths <= 4: register kernel
   const int BM = pad_width5(a.m), BK = pad_width5(a.k);
   if (a.mv < 5 || a.mv > 64 || BM != BK) return false;  // square blocks only
   const int MV = pad_width5(a.mv);
-  return BM == 8 ? mvsd_gram_dmma_mv<8, 8>(a, MV) : mvsd_gram_dmma_mv<16, 16>(a, MV);
+  if (BK <= 16) return BK == 8 ? mvsd_gram_dmma_mv<8, 8>(a, MV) : mvsd_gram_dmma_mv<16, 16>(a, MV);
+  if (MV <= 16 || a.n > (4 * a.k > 3 * BK ? 1 << 19 : 1 << 17)) return false;
+  if (BK == 32) return MV == 32 ? mvsd_gram_dmma_launch<32, 32, 32>(a) : mvsd_gram_dmma_launch<32, 32, 64>(a);
+  return MV == 32 ? mvsd_gram_dmma_launch<64, 64, 32>(a) : mvsd_gram_dmma_launch<64, 64, 64>(a);
 }
 inline bool mvsd_gram_dmma(RowGemmArgs<float>&) { return false; }
 

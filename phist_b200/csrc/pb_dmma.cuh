@@ -4,7 +4,7 @@
 //
 //   k_mvtmv_dmma     : C = alpha V'W + beta C (the wide products: pb_frag.cu
 //                      has the rule)
-//   k_mvsd_gram_dmma : V*C with the Gram matrix of the result, up to 16 columns
+//   k_mvsd_gram_dmma : W C in place with V'W of another block (rule: pb_api.cuh)
 //
 // Fragment layout of mma.m8n8k4.row.col.f64 (lane l, g = l/4, t = l%4):
 //   A (8x4, row-major): a = A[g][t];  B (4x8, column-major): b = B[t][g];

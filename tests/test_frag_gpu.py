@@ -128,8 +128,9 @@ def test_product_with_gram(session, n, m, k, ld, dtype):
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("mv,k,off", [(1, 4, 0), (8, 4, 0), (9, 4, 0), (20, 4, 0), (10, 2, 1), (37, 3, 1), (64, 1, 0), (16, 16, 0),
-                                      (24, 24, 0), (32, 32, 0), (64, 32, 0), (33, 33, 1), (40, 64, 0), (64, 64, 0)])
-@pytest.mark.parametrize("n", [0, 1, 5003])
+                                      (24, 24, 0), (32, 32, 0), (64, 32, 0), (33, 33, 1), (40, 64, 0), (64, 64, 0),
+                                      (17, 18, 0), (32, 56, 0), (16, 32, 0)])
+@pytest.mark.parametrize("n", [0, 1, 64, 65, 5003])
 def test_in_place_product_with_another_block(session, n, mv, k, off, dtype):
     """W = W C in place and D = a V'W + b D of the new W, V another block.  A
     row of W is a sum of k products of size at most 1/k; the sum over n rows of
