@@ -319,8 +319,8 @@ __device__ __forceinline__ void load_row(const T* __restrict__ p, int ncols, int
 
 // sum the NOUT per-thread values of every thread of the block in a fixed
 // order (warp butterfly, then warps in order) and write the block partial
-template <class T, int NOUT>
-__device__ __forceinline__ void block_partial(T* vals, T* part, int nout)
+template <class T, int NOUT, class TP>
+__device__ __forceinline__ void block_partial(T* vals, TP* part, int nout)
 {
   __shared__ T red[8][NOUT];
 #pragma unroll
@@ -333,8 +333,8 @@ __device__ __forceinline__ void block_partial(T* vals, T* part, int nout)
     for (int q = 0; q < NOUT; q++) red[warp][q] = vals[q];
   __syncthreads();
   for (int q = threadIdx.x; q < nout; q += blockDim.x) {
-    T s = T(0);
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += red[w][q];
+    TP s = TP(0);
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += (TP)red[w][q];
     part[(int64_t)blockIdx.x * nout + q] = s;
   }
 }
@@ -424,8 +424,11 @@ __device__ __forceinline__ void st_row4(double* p, const double* v)
 }
 
 // Row-local products for m, k, mv <= 8 (modes and Gram as k_rowgemm, the Gram
-// for k <= 4 only).  The Gram products are formed and summed in FP64 in both
-// precisions, as in pb_frag.cuh, and rounded once; a.part is FP64.
+// for k <= 4 only).  The Gram sums of the lanes and of a warp are formed in T,
+// from there on in FP64 (a.part): the errors of some 4,700 warps average out
+// below the rounding of the result.  FP64 in the lanes of FP32 blocks, too,
+// costs conversions and registers that the gram-free calls pay as well (4
+// columns in place at 2,097,152 rows 14 -> 19 us).
 // V4: V and W have 4 FP64 columns and rows on 32-byte boundaries, which are
 // moved whole (us, element by element | so: in place at 1,048,576 rows 20.4 |
 // 12.3, at 2,097,152 35.8 | 20.4; W = V C 17.2 | 12.3, 36.7 | 30.8).
@@ -447,9 +450,9 @@ __global__ void __launch_bounds__(256) k_rowgemm_reg(RowGemmArgs<T> a)
   __syncthreads();
   constexpr bool GRAM = K <= 4;
   constexpr int GM = (MV > K) ? MV : K, NG = GRAM ? GM * K : 1;
-  double gacc[NG];
+  T gacc[NG];
 #pragma unroll
-  for (int q = 0; q < NG; q++) gacc[q] = 0.0;
+  for (int q = 0; q < NG; q++) gacc[q] = T(0);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
        i += (int64_t)gridDim.x * blockDim.x) {
     T v[8], w[8], out[8];
@@ -486,14 +489,14 @@ __global__ void __launch_bounds__(256) k_rowgemm_reg(RowGemmArgs<T> a)
 #pragma unroll
         for (int q = 0; q < K; q++)
 #pragma unroll
-          for (int p = 0; p < K; p++) gacc[p + q * K] += (double)out[p] * (double)out[q];
+          for (int p = 0; p < K; p++) gacc[p + q * K] += out[p] * out[q];
       } else if (a.gram == GM_VW) {
         T g[8];
         load_row(a.Vg + i * a.ldvg, a.mv, MV, g);
 #pragma unroll
         for (int q = 0; q < K; q++)
 #pragma unroll
-          for (int p = 0; p < MV; p++) gacc[p + q * MV] += (double)g[p] * (double)out[q];
+          for (int p = 0; p < MV; p++) gacc[p + q * MV] += g[p] * out[q];
       }
     }
   }
@@ -502,7 +505,7 @@ __global__ void __launch_bounds__(256) k_rowgemm_reg(RowGemmArgs<T> a)
     const int gmax = (a.gram == GM_WW) ? K : MV;
     // partial layout: gmax rows (padded), K columns
     double* part = reinterpret_cast<double*>(a.part);
-    block_partial<double, NG>(gacc, part, gmax * K);
+    block_partial<T, NG>(gacc, part, gmax * K);
     const double al = (a.gram == GM_WW) ? 1.0 : (double)a.galpha;
     const double be = (a.gram == GM_WW) ? 0.0 : (double)a.gbeta;
     last_block_reduce<double>(part, gmax * K, gridDim.x, a.counter, a.Gd, 1, gmax, a.ldg, al, be,

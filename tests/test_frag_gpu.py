@@ -169,8 +169,10 @@ def test_thin_product_with_gram_of_many_rows(session, n, m, k, dtype):
     K.chk(fn(dtype, "fused_mvsd_mvTmv"), 0.5, V.h, C.h, -0.5, W.h, G.h)
     new = W.get().astype(np.float64)
     assert np.abs(new - (0.5 * (v @ c.astype(np.float64)) - 0.5 * w)).max() <= (m + 3) * 2 * eps
-    g = G.get()  # formed in FP64, rounded once
-    assert (np.abs(g - new.T @ new) <= (n * np.finfo(np.float64).eps + eps) * (np.abs(new).T @ np.abs(new))).all()
+    # a lane adds at most 2^20 / (4 * 148 * 256) < 8 products in the precision of
+    # the block and a warp its lanes in 5 steps; from there on FP64, rounded once
+    g = G.get()
+    assert (np.abs(g - new.T @ new) <= (n * np.finfo(np.float64).eps + 15 * eps) * (np.abs(new).T @ np.abs(new))).all()
     assert np.array_equal(G.host(), g)
     for o in (V, W, C, G, Vb, Wb, mp, mq):
         o.delete()
