@@ -264,11 +264,11 @@ inline cudaStream_t stream() { return rt().stream(); }
 // and read that with coherent loads (GlobalLd, frag_ld1, __ldcg): it is not
 // read-only for their lifetime.
 template <class... KA, class... A>
-inline void launch_pdl(void (*kern)(KA...), int grid, int block, size_t smem, const A&... args)
+inline void launch_pdl(void (*kern)(KA...), dim3 grid, int block, size_t smem, const A&... args)
 {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream();

@@ -123,16 +123,27 @@ k_gm_solve(const double* __restrict__ H, const double* __restrict__ g, const int
   if (lane + 32 < Jmax) Y[(lane + 32) * k + s] = lane + 32 < J ? (T)(-(double)F[(lane + 32) * k + s] * y1) : T(0);
 }
 
+// The grid of a pass: want blocks for all groups of systems, the groups side by
+// side, at most one wave of perSM blocks; partials and counters for it (the
+// first level of the sum as in pb_frag.cu, the lane's 64 counters shared out)
+template <class T>
+dim3 kry_grid(KryArgs<T>& a, int64_t want, int perSM)
+{
+  const int ngrp = (int)ceil_div(a.k, KRY_MAXC);
+  const int grid = (int)std::min<int64_t>(want, std::max(1, perSM * rt().num_sms() / ngrp));
+  a.cnt_step = 64 / ngrp;
+  a.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, a.cnt_step - 2));
+  a.part_step = (grid + ceil_div(grid, a.gsz)) * KRY_MAXOUT;
+  a.part = (double*)rt().scratch(sizeof(double) * (size_t)a.part_step * ngrp);
+  a.counters = rt().counters();
+  return dim3((unsigned)grid, (unsigned)ngrp);
+}
+
 template <class T, int MQ, int MJ, bool UPD, bool DOTS>
 void kry_launch(KryArgs<T>& a)
 {
-  // two blocks per SM (the launch bound); groups of the first level of the
-  // sum as in pb_frag.cu
-  const int grid = (int)std::min<int64_t>(ceil_div(a.n, 32 * FRAG_NW), 2 * (int64_t)rt().num_sms());
-  a.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
-  a.part = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ceil_div(grid, a.gsz)) * KRY_MAXOUT);
-  a.counters = rt().counters();
-  launch_pdl(k_kry<T, MQ, MJ, UPD, DOTS>, grid, FRAG_BS, 0, a);
+  // two blocks per SM: the launch bound
+  launch_pdl(k_kry<T, MQ, MJ, UPD, DOTS>, kry_grid(a, ceil_div(a.n, 32 * FRAG_NW), 2), FRAG_BS, 0, a);
   PB_LAUNCH_CHECK();
 }
 
@@ -196,11 +207,7 @@ bool spmv_lanczos_nv(const SparseMat<T>* A, const T* negsig, const Mvec<T>* X, M
     o = std::max(1, o);
     occ.store(o);
   }
-  const int grid = (int)std::min<int64_t>(ceil_div(A->nchunks, LZ_NT / TPR / 32), (int64_t)rt().num_sms() * o);
-  a.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
-  a.part = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ceil_div(grid, a.gsz)) * KRY_MAXOUT);
-  a.counters = rt().counters();
-  launch_pdl(kern, grid, LZ_NT, 0, sell_dev(A), p, a);
+  launch_pdl(kern, kry_grid(a, ceil_div(A->nchunks, LZ_NT / TPR / 32), o), LZ_NT, 0, sell_dev(A), p, a);
   PB_LAUNCH_CHECK();
   return true;
 }
@@ -241,23 +248,6 @@ static void gm_mvsd(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, c
   launch_rowgemm<T>(a);
 }
 
-// More than KRY_MAXC systems: in one solve, whose passes go over groups of
-// KRY_MAXC columns of blocks that are k columns wide and share the SpMMV and
-// the products with a wide Q, or in solves of KRY_MAXC systems each, whose
-// blocks are contiguous.  A pass over a part of wide rows moves its data at
-// three quarters of the rate, but the fewer launches win on small problems.
-// 15 steps, us, one solve | several (nq = 32 unless named):
-//   GMRES FP64 16 systems  32^3 1,621 | 1,609  40^3 2,260 | 1,801  64^3 6,549 | 4,977
-//   GMRES FP32 16 systems  40^3 1,521 | 1,564  48^3 2,259 | 2,055  64^3 4,161 | 3,579
-//   MINRES FP64 16 / 24    48^3 1,447 | 1,470, 2,496 | 2,220  64^3 2,714 | 2,561, 4,869 | 3,841
-//   MINRES FP32 16 / 24    48^3 1,190 | 1,228, 1,836 | 1,849  64^3 1,964 | 1,955, 3,330 | 2,941
-//   MINRES FP64 16, nq = 40 (projection in products of its own)  64^3 2,664 | 2,814
-inline bool gm_split(bool lanczos, bool fuse, int64_t n, size_t elem)
-{
-  const size_t column = (size_t)n * elem;
-  return lanczos ? fuse && column >= (1u << 20) : column >= (400u << 10);
-}
-
 // lanczos: MINRES (three-term recurrence), else GMRES
 template <class T>
 int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const int* resIndex, int k,
@@ -279,18 +269,6 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
   // a projection block of at most KRY_MAXQ columns goes with the passes over
   // the basis, a wider one in products of its own
   const bool fuse = nq > 0 && nq <= KRY_MAXQ;
-  if (k > KRY_MAXC && gm_split(lanczos, fuse || nq == 0, n, sizeof(T))) {
-    int unconverged = 0;
-    for (int c0 = 0; c0 < k; c0 += KRY_MAXC) {
-      const int kc = std::min(KRY_MAXC, k - c0);
-      std::vector<int> idx(kc);
-      for (int s = 0; s < kc; s++) idx[s] = resIndex ? resIndex[c0 + s] : c0 + s;
-      Mvec<T> tc;
-      raw_view(tc, t->d() + c0, n, kc, t->lda);
-      unconverged += jada_krylov<T>(A, Q, R, idx.data(), kc, sigma + c0, tol + c0, maxIter, maxBas, &tc, lanczos);
-    }
-    return unconverged;
-  }
   const int m = std::max(1, std::min(std::min(maxBas > 0 ? maxBas : maxIter, maxIter), 63));
   const int64_t nk = n * (int64_t)k;  // one basis block
   const double eps_abs = (lanczos ? 100.0 : 1000.0) * std::numeric_limits<T>::epsilon();
@@ -315,6 +293,7 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
   memset(&base, 0, sizeof(base));
   base.n = n;
   base.k = k;
+  base.per = (int)ceil_div(k, ngrp);  // even groups: they share the SMs evenly
   base.Q = fuse ? Q->d() : nullptr;
   base.ldq = fuse ? Q->lda : 0;
   base.vstep = nk;
@@ -336,26 +315,13 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
     e.h2_lim = lim * lim;
     e.g0 = gq.p; e.gam = gq.p + (size_t)nq * k; e.dq = e.gam + (size_t)(m + 1) * k;
     e.flags = (unsigned long long*)rt().mailbox_dev();
+    e.reorth = reorth.p;
+    e.gflag = fuse ? gflag.p : nullptr;
     for (int s = 0; s < k; s++) {
       base.idx.v[s] = resIndex ? resIndex[s] : s;
       e.tol.v[s] = tol[s];
     }
   }
-  // the pass for each group of at most KRY_MAXC systems: W the block it works
-  // on, blocks i0.. (count nb, step vstep)
-  auto for_groups = [&](auto pass) {
-    for (int q = 0; q < ngrp; q++) {
-      KryArgs<T> a = base;
-      const int c0 = q * KRY_MAXC;
-      a.kc = std::min(KRY_MAXC, k - c0);
-      a.kp = a.kc <= 1 ? 1 : a.kc <= 2 ? 2 : a.kc <= 4 ? 4 : 8;
-      a.e.c0 = c0;
-      a.e.last = q == ngrp - 1;
-      a.e.reorth = reorth.p + q;
-      a.e.gflag = fuse ? gflag.p + q : nullptr;
-      pass(a, c0);
-    }
-  };
   // W = P W with P = I - Q Q' (outside the fused passes)
   auto project = [&](T* W) {
     if (nq == 0) return;
@@ -363,6 +329,11 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
     gm_mvsd<T>(n, nq, k, T(-1), Q->d(), Q->lda, Cq.p, nq, T(1), W, k);
   };
 
+  auto converged = [&] {
+    int c = 0;
+    for (int q = 0; q < ngrp; q++) c += (int)(hflags[q] >> 32);
+    return c;
+  };
   int total = 0, nconv = 0;
   for (int cycle = 0; total < maxIter && nconv < k; cycle++) {
     if (cycle > 0) {
@@ -371,16 +342,13 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
       spmv_general<T>(T(1), A, negsig.data(), &mX, T(0), &mW, nullptr, nullptr, T(0), T(0), nullptr);
       project(V.p);
     }
-    for_groups([&](KryArgs<T>& a, int c0) {
-      a.W = V.p + c0;
+    {
+      KryArgs<T> a = base;
+      a.W = V.p;
       a.restart = cycle > 0 ? 1 : 0;
       a.e.first = cycle == 0 ? 1 : 0;
       a.e.kind = fuse ? KE_NONE : KE_START;
-      const int grid = (int)std::min<int64_t>(ceil_div(n * a.kp, 4 * FRAG_BS), 4 * (int64_t)rt().num_sms());
-      a.gsz = std::max((int)std::ceil(std::sqrt((double)grid)), (int)ceil_div(grid, 62));
-      a.part = (double*)rt().scratch(sizeof(double) * (size_t)(grid + ceil_div(grid, a.gsz)) * KRY_MAXOUT);
-      a.counters = rt().counters();
-      launch_pdl(k_kry_start<T>, grid, FRAG_BS, 0, a);
+      launch_pdl(k_kry_start<T>, kry_grid(a, ceil_div(n * std::min(k, KRY_MAXC), 4 * FRAG_BS), 4), FRAG_BS, 0, a);
       PB_LAUNCH_CHECK();
       if (fuse) {
         // the norms together with Q'V_0
@@ -390,8 +358,8 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
         a.e.kind = KE_START;
         kry_dots<T, false>(a);
       }
-    });
-    *hflags = 0;
+    }
+    for (int q = 0; q < ngrp; q++) hflags[q] = 0;
     int j = 0, steps = 0;
     const int jmax = std::min(m, maxIter - total);
     bool stop = false;
@@ -402,56 +370,52 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
       raw_view(mW, Wj, n, k, k);
       bool dotted = false;  // Q'W and V_j'W came with the SpMMV
       if (lanczos && fuse && ngrp == 1) {
-        for_groups([&](KryArgs<T>& a, int) {
-          a.nq = nq;
-          a.e.j = j;
-          a.e.kind = KE_LZ;
-          dotted = spmv_lanczos<T>(A, negsig.data(), &mVj, &mW, F.p + (int64_t)j * k, a);
-        });
+        KryArgs<T> a = base;
+        a.nq = nq;
+        a.e.j = j;
+        a.e.kind = KE_LZ;
+        dotted = spmv_lanczos<T>(A, negsig.data(), &mVj, &mW, F.p + (int64_t)j * k, a);
       }
       if (!dotted)
         spmv_general<T>(T(1), A, negsig.data(), &mVj, T(0), &mW, nullptr, nullptr, T(0), T(0), nullptr,
                         F.p + (int64_t)j * k);
       if (!fuse) project(Wj);
       const int J = j + 1;
-      for_groups([&](KryArgs<T>& a0, int c0) {
-        a0.W = Wj + c0;
-        a0.Win = a0.W;
-        a0.e.j = j;
-        // one pass: blocks [i0, i0 + nb), with Q when it is the first
-        auto pass = [&](bool upd, bool dots, int i0, int nb, bool withq, const T* hc, int kind, bool last,
-                        const int* skip) {
-          KryArgs<T> a = a0;
-          a.nq = (fuse && withq) ? nq : 0;
-          a.V = V.p + (int64_t)i0 * nk + c0;
-          a.nb = nb;
-          a.cq = Cq.p + c0;
-          a.hv = hc ? hc + c0 : nullptr;
-          a.skip = skip;
-          a.e.i0 = i0;
-          a.e.kind = kind;
-          a.e.last = last;
-          if (upd && lanczos) a.vstep = -nk;  // V_j, then V_{j-1}
-          if (upd && dots) kry_dots<T, true>(a);
-          else if (dots) kry_dots<T, false>(a);
-          else kry_update<T>(a);
-        };
-        const bool lastg = a0.e.last;
-        if (lanczos) {
-          // [Q V_j]'W; W -= Q (Q'W) + v_j alpha + v_{j-1} beta and its norm
-          // (alpha = v_j'(P W) from both dots; PHIST's order: projection,
-          // then the Lanczos terms)
-          if (!dotted) pass(false, true, j, 1, true, nullptr, KE_LZ, true, nullptr);
-          pass(true, false, j, j > 0 ? 2 : 1, true, hv.p, KE_STEP, lastg, nullptr);
-          return;
-        }
+      // one pass: blocks [i0, i0 + nb), with Q when it is the first
+      auto pass = [&](bool upd, bool dots, int i0, int nb, bool withq, const T* hc, int kind, bool last,
+                      const int* skip) {
+        KryArgs<T> a = base;
+        a.W = Wj;
+        a.Win = Wj;
+        a.nq = (fuse && withq) ? nq : 0;
+        a.V = V.p + (int64_t)i0 * nk;
+        a.nb = nb;
+        a.cq = Cq.p;
+        a.hv = hc;
+        a.skip = skip;
+        a.e.j = j;
+        a.e.i0 = i0;
+        a.e.kind = kind;
+        a.e.last = last;
+        if (upd && lanczos) a.vstep = -nk;  // V_j, then V_{j-1}
+        if (upd && dots) kry_dots<T, true>(a);
+        else if (dots) kry_dots<T, false>(a);
+        else kry_update<T>(a);
+      };
+      if (lanczos) {
+        // [Q V_j]'W; W -= Q (Q'W) + v_j alpha + v_{j-1} beta and its norm
+        // (alpha = v_j'(P W) from both dots; PHIST's order: projection,
+        // then the Lanczos terms)
+        if (!dotted) pass(false, true, j, 1, true, nullptr, KE_LZ, true, nullptr);
+        pass(true, false, j, j > 0 ? 2 : 1, true, hv.p, KE_STEP, true, nullptr);
+      } else {
         // Gram-Schmidt against Q and V_0..V_j: h1 = V'(P W) from V'W and Q'W
         // (kry_epilogue); W -= Q (Q'W) + V h1 and h2 = V'W of the result; a
-        // second subtraction only where that is needed (a device flag)
+        // second subtraction only where that is needed (a device flag); the
+        // rest of the step follows in whichever launch finishes W
         if (J <= KRY_MAXJ) {
           pass(false, true, 0, J, true, nullptr, KE_GS, true, nullptr);
           pass(true, true, 0, J, true, hv.p, KE_GS2, true, nullptr);
-          // the step follows the second pass in whichever launch finishes W
         } else {
           for (int i0 = 0; i0 < J; i0 += KRY_MAXJ)
             pass(false, true, i0, std::min(KRY_MAXJ, J - i0), i0 == 0, nullptr, KE_GS, true, nullptr);
@@ -464,34 +428,32 @@ int jada_krylov(const SparseMat<T>* A, const Mvec<T>* Q, const Mvec<T>* R, const
         for (int i0 = 0; i0 < J; i0 += KRY_MAXJ) {
           const bool end = i0 + KRY_MAXJ >= J;
           pass(true, false, i0, std::min(KRY_MAXJ, J - i0), false, hv2.p + (int64_t)i0 * k, end ? KE_STEP : KE_NONE,
-               lastg, a0.e.reorth);
+               true, reorth.p);
         }
-      });
+      }
       steps = j + 1;
       // stop launching once the device reports every system converged (a
       // look at the flags, no wait: the host never blocks inside a cycle,
       // so concurrent solves on other threads keep their cores)
-      if ((int)(*hflags >> 32) >= k) stop = true;
+      if (converged() >= k) stop = true;
     }
     total += steps;
     // x += [V_0..V_{J-1}] y with J the largest step count of a system
     rt().sync();
-    nconv = (int)(*hflags >> 32);
+    nconv = converged();
     const int J = steps;
     k_gm_solve<T><<<(int)ceil_div(k, GM_SOLVE_NW), 32 * GM_SOLVE_NW, 0, stream()>>>(H.p, g.p, jcount.p, k, m, J, F.p, Y.p);
     PB_LAUNCH_CHECK();
-    for_groups([&](KryArgs<T>& a0, int c0) {
-      for (int i0 = 0; i0 < J; i0 += KRY_MAXJ) {
-        KryArgs<T> a = a0;
-        a.W = X.p + c0;
-        a.Win = (cycle == 0 && i0 == 0) ? nullptr : a.W;
-        a.V = V.p + (int64_t)i0 * nk + c0;
-        a.nb = std::min(KRY_MAXJ, J - i0);
-        a.hv = Y.p + (int64_t)i0 * k + c0;
-        a.e.kind = KE_NORM;
-        kry_update<T>(a);
-      }
-    });
+    for (int i0 = 0; i0 < J; i0 += KRY_MAXJ) {
+      KryArgs<T> a = base;
+      a.W = X.p;
+      a.Win = (cycle == 0 && i0 == 0) ? nullptr : a.W;
+      a.V = V.p + (int64_t)i0 * nk;
+      a.nb = std::min(KRY_MAXJ, J - i0);
+      a.hv = Y.p + (int64_t)i0 * k;
+      a.e.kind = KE_NORM;
+      kry_update<T>(a);
+    }
   }
   // t = x / ||x||, column by column
   k_gm_scale_cols<T><<<gw, 256, 0, stream()>>>(X.p, k, t->d(), t->lda, n, k, f.p);

@@ -17,6 +17,12 @@
 // column of H, rotations, residual estimate, convergence test, F_{j+1}.  A
 // MINRES step is SpMMV + 2 launches, a GMRES step SpMMV + 3.
 //
+// More than 8 systems are split evenly into groups, gridDim.y of them, each
+// with its own sums and epilogue; they run side by side over the same rows, so
+// that Q and the lines that two groups share come from HBM once.  15 steps, nq
+// = 32, us, a launch per group of 8 | so: GMRES FP64 32 systems, 24^3 2,871 | 907;
+// 16 systems, 64^3 6,549 | 4,063; 12 systems, 100^3 18,548 | 13,628.
+//
 // A warp takes 32 rows at a time.  Q (row-major, any stride) meets W on the
 // FP64 tensor pipe with fragments straight from global memory as in
 // pb_frag.cuh; Q cq goes through a warp's own shared-memory tile into the
@@ -32,7 +38,7 @@ namespace pb {
 
 constexpr int KRY_MAXQ = 32;  // projection columns of one launch
 constexpr int KRY_MAXJ = 24;  // basis blocks of one launch
-constexpr int KRY_MAXC = 8;   // systems of one launch
+constexpr int KRY_MAXC = 8;   // most systems of one group (blockIdx.y) of a launch
 constexpr int KRY_MAXOUT = (KRY_MAXQ + KRY_MAXJ + 1) * KRY_MAXC;
 
 struct GmTol {
@@ -54,11 +60,12 @@ enum KryKind {
 };
 
 // H(:, :, s) at H[(i*m + j)*k + s]; per-system arrays have stride k and are
-// indexed by the system number (c0 + the launch's column)
+// indexed by the system number (c0 + the group's column); reorth, gflag and
+// flags have one entry a group
 template <class T>
 struct KryEpi {
-  int kind, last;             // last: last launch of a group of chunks (KE_GS2) / of systems (flags)
-  int c0, k, m, j, i0;
+  int kind, last;             // last: last launch of a row of chunks (KE_GS2)
+  int k, m, j, i0;
   int lanczos, first;
   double *H, *cs, *sn, *g, *bnorm;
   double *h1, *h2;            // [i*k + s] coefficients of the two Gram-Schmidt passes
@@ -72,23 +79,33 @@ struct KryEpi {
   // Q'V_i = gam[i*k + s] g0 (nq values g0[l*k + s]); used while *gflag != 0
   double *g0, *gam, *dq;
   int* gflag;                 // NULL: no projection in the passes
-  volatile unsigned long long* flags;  // mapped host memory: converged systems << 32 | steps done
+  volatile unsigned long long* flags;  // mapped host memory: converged systems of the group << 32 | steps done
 };
 
 template <class T>
 struct KryArgs {
   int64_t n;
-  int k, kc, kp;              // row stride of W and V_i; systems here; kc rounded up to a power of two
+  int k, per;                 // systems, the row stride of W and V_i; systems of a group (the last may have fewer)
   int nq; const T* Q; int64_t ldq;
   const T* V; int64_t vstep; int nb;   // blocks at V + i*vstep
   const T* Win;               // NULL: W starts from zero
   T* W;
   const T* cq; const T* hv;
-  const int* skip;            // the kernel does nothing when *skip == 0
-  double* part; int gsz; unsigned int* counters;
+  const int* skip;            // a group with skip[group] == 0 has nothing to do
+  double* part; int gsz; unsigned int* counters;   // of group 0; the others' follow
+  int64_t part_step; int cnt_step;                 // at these distances
   KryEpi<T> e;
   // KE_START: W = R(:, idx) (- W on a restart, converged systems zero)
   const T* R; int64_t ldr; GmIndex idx; int restart;
+};
+
+// the block's group: first system, systems, and that rounded up to a power of two
+struct KryGrp {
+  int c0, kc, kp;
+  __device__ __forceinline__ KryGrp(int k, int per) : c0(blockIdx.y * per), kc(min(KRY_MAXC, min(per, k - c0)))
+  {
+    kp = kc <= 1 ? 1 : kc <= 2 ? 2 : kc <= 4 ? 4 : 8;
+  }
 };
 
 __device__ __forceinline__ void kry_ldp(const double* p, bool ok, double& v)
@@ -109,7 +126,7 @@ __device__ __forceinline__ void kry_ldp(const float* p, bool ok, float& v)
 // nrm: ||W||^2 per column of the launch; sm: shared scratch, 3*64*8 doubles.
 // A Lanczos column is zero above j-1, so only the rotations from j-2 on act.
 template <class T>
-__device__ __forceinline__ void kry_step(const KryEpi<T>& e, int kc, const double* nrm, double* sm)
+__device__ __forceinline__ void kry_step(const KryEpi<T>& e, int c0, int kc, const double* nrm, double* sm)
 {
   const int tid = threadIdx.x, j = e.j, k = e.k, m = e.m;
   const int lo = e.lanczos ? max(0, j - 2) : 0;
@@ -120,13 +137,13 @@ __device__ __forceinline__ void kry_step(const KryEpi<T>& e, int kc, const doubl
   double gj = 0.0, bn = 0.0;
   int done = 0;
   if (tid < kc) {
-    gj = __ldcg(&e.g[j * k + e.c0 + tid]);
-    bn = __ldcg(&e.bnorm[e.c0 + tid]);
-    done = __ldcg(&e.conv[e.c0 + tid]);
+    gj = __ldcg(&e.g[j * k + c0 + tid]);
+    bn = __ldcg(&e.bnorm[c0 + tid]);
+    done = __ldcg(&e.conv[c0 + tid]);
   }
   __syncthreads();
   for (int q = tid; q < (j + 1 - lo) * kc; q += FRAG_BS) {
-    const int i = lo + q / kc, c = q % kc, s = e.c0 + c;
+    const int i = lo + q / kc, c = q % kc, s = c0 + c;
     sh[i * kc + c] = __ldcg(&e.H[((int64_t)i * m + j) * k + s]);
     if (i < j) {
       sc[i * kc + c] = __ldcg(&e.cs[i * k + s]);
@@ -135,7 +152,7 @@ __device__ __forceinline__ void kry_step(const KryEpi<T>& e, int kc, const doubl
   }
   __syncthreads();
   if (tid < kc) {
-    const int c = tid, s = e.c0 + c;
+    const int c = tid, s = c0 + c;
     const double n2 = fmax(nrm[c], 0.0), hn = sqrt(n2);
     double a = sh[lo * kc + c];
     for (int i = lo; i < j; i++) {
@@ -163,17 +180,13 @@ __device__ __forceinline__ void kry_step(const KryEpi<T>& e, int kc, const doubl
     e.nf[s] = n2;
     e.F[(j + 1) * k + s] = (hn > 0.0) ? (T)(1.0 / hn) : T(0);
   }
-  int nconv = __syncthreads_count(tid < kc && done);
+  const int nconv = __syncthreads_count(tid < kc && done);
   for (int q = tid; q < (j + 1 - lo) * kc; q += FRAG_BS) {
     const int i = lo + q / kc, c = q % kc;
-    e.H[((int64_t)i * m + j) * k + e.c0 + c] = sh[i * kc + c];
+    e.H[((int64_t)i * m + j) * k + c0 + c] = sh[i * kc + c];
   }
-  if (tid == 0 && e.last) {
-    for (int s = 0; s < k; s++)
-      if (s < e.c0 || s >= e.c0 + kc) nconv += __ldcg(&e.conv[s]) ? 1 : 0;
-    // step and count in one store: the host reads them together
-    *e.flags = ((unsigned long long)(unsigned)nconv << 32) | (unsigned)(j + 1);
-  }
+  // step and count in one store: the host reads them together
+  if (tid == 0) e.flags[blockIdx.y] = ((unsigned long long)(unsigned)nconv << 32) | (unsigned)(j + 1);
 }
 
 // The dots of a pass see W before the projection: V_i'W, where the step wants
@@ -191,10 +204,11 @@ __device__ __forceinline__ void kry_proj_sums(const KryArgs<T>& a, int nqo, cons
                                               double& c2)
 {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const bool on = w < a.kc && lane < nqo;
-  const double c = on ? (double)(T)out[lane * a.kc + w] : 0.0;
+  const KryGrp gr(a.k, a.per);
+  const bool on = w < gr.kc && lane < nqo;
+  const double c = on ? (double)(T)out[lane * gr.kc + w] : 0.0;
   c2 = c * c;
-  d = (on && flagged) ? __ldcg(&a.e.g0[lane * a.e.k + a.e.c0 + w]) * c : 0.0;
+  d = (on && flagged) ? __ldcg(&a.e.g0[lane * a.e.k + gr.c0 + w]) * c : 0.0;
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) {
     c2 += __shfl_xor_sync(0xffffffffu, c2, off);
@@ -217,7 +231,8 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
                                              bool flagged)
 {
   const KryEpi<T>& e = a.e;
-  const int tid = threadIdx.x, kc = a.kc, k = e.k, j = e.j, m = e.m;
+  const KryGrp gr(a.k, a.per);
+  const int tid = threadIdx.x, c0 = gr.c0, kc = gr.kc, k = e.k, j = e.j, m = e.m;
   const double* nrm = out + (nqo + nbo) * kc;
   auto is = [&](int kind) { return ((KINDS >> kind) & 1) && e.kind == kind; };
   if (is(KE_START)) {
@@ -226,15 +241,15 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
       for (int q = tid; q < nqo * kc; q += FRAG_BS) {
         const double v = out[q];
         const double eps = sizeof(T) == 8 ? 2.3e-16 : 1.2e-7;
-        e.g0[(q / kc) * k + e.c0 + q % kc] = v;
+        e.g0[(q / kc) * k + c0 + q % kc] = v;
         big |= v * v > 256.0 * eps * eps * nrm[q % kc];
       }
       big = __syncthreads_or(big);
-      if (tid == 0) *e.gflag = big;
-      if (tid < kc) e.gam[e.c0 + tid] = 1.0;
+      if (tid == 0) e.gflag[blockIdx.y] = big;
+      if (tid < kc) e.gam[c0 + tid] = 1.0;
     }
     if (tid < kc) {
-      const int s = e.c0 + tid;
+      const int s = c0 + tid;
       const double beta = sqrt(fmax(nrm[tid], 0.0));
       if (e.first) {
         e.bnorm[s] = beta;
@@ -246,7 +261,7 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
       e.F[s] = (beta > 0.0 && !e.conv[s]) ? (T)(1.0 / beta) : T(0);
     }
   } else if (is(KE_LZ)) {
-    for (int q = tid; q < nqo * kc; q += FRAG_BS) e.cq[(q / kc) * k + e.c0 + q % kc] = (T)out[q];
+    for (int q = tid; q < nqo * kc; q += FRAG_BS) e.cq[(q / kc) * k + c0 + q % kc] = (T)out[q];
     if (flagged) {
       double d, c2;
       kry_proj_sums<T>(a, nqo, out, true, d, c2);
@@ -256,7 +271,7 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
     if (tid < kc) {
       // alpha = v_j'w, beta = the previous step's norm; the update
       // subtracts V_j (F_j alpha), then V_{j-1} (F_{j-1} beta)
-      const int s = e.c0 + tid;
+      const int s = c0 + tid;
       const double gj = flagged ? e.gam[j * k + s] : 0.0;
       const double alpha = (double)e.F[j * k + s] * (out[nqo * kc + tid] - (flagged ? gj * sm[tid] : 0.0));
       const double beta = j > 0 ? sqrt(e.nf[s]) : 0.0;
@@ -269,7 +284,7 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
         e.gam[(j + 1) * k + s] = -(gj * (double)e.hv[s] + (j > 0 ? e.gam[(j - 1) * k + s] * (double)e.hv[k + s] : 0.0));
     }
   } else if (is(KE_GS)) {
-    for (int q = tid; q < nqo * kc; q += FRAG_BS) e.cq[(q / kc) * k + e.c0 + q % kc] = (T)out[q];
+    for (int q = tid; q < nqo * kc; q += FRAG_BS) e.cq[(q / kc) * k + c0 + q % kc] = (T)out[q];
     if (e.i0 == 0) {
       // d, and ||P W||^2 = ||W||^2 - ||c||^2; where that is all cancellation
       // the larger ||W||^2, with which the second subtraction is made
@@ -278,16 +293,16 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
       const int w = tid >> 5;
       if ((tid & 31) == 0 && w < kc) {
         const double pw = nrm[w] - c2;
-        e.nrm0[e.c0 + w] = pw > 1e-3 * nrm[w] ? pw : nrm[w];
+        e.nrm0[c0 + w] = pw > 1e-3 * nrm[w] ? pw : nrm[w];
         sm[w] = d;
-        if (flagged) e.dq[e.c0 + w] = d;
+        if (flagged) e.dq[c0 + w] = d;
       }
     } else if (flagged && tid < kc) {
-      sm[tid] = __ldcg(&e.dq[e.c0 + tid]);
+      sm[tid] = __ldcg(&e.dq[c0 + tid]);
     }
     if (flagged) __syncthreads();
     for (int q = tid; q < nbo * kc; q += FRAG_BS) {
-      const int p = (e.i0 + q / kc) * k + e.c0 + q % kc;
+      const int p = (e.i0 + q / kc) * k + c0 + q % kc;
       const double h = (double)e.F[p] * (out[nqo * kc + q] - (flagged ? __ldcg(&e.gam[p]) * sm[q % kc] : 0.0));
       e.h1[p] = h;
       e.hv[p] = (T)((double)e.F[p] * h);
@@ -299,7 +314,7 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
     // from rounding as the steps go on, and Q may be orthonormal to less.
     int need = 0;
     for (int q = tid; q < nbo * kc; q += FRAG_BS) {
-      const int p = (e.i0 + q / kc) * k + e.c0 + q % kc;
+      const int p = (e.i0 + q / kc) * k + c0 + q % kc;
       const double h = (double)e.F[p] * out[nqo * kc + q];
       e.h2[p] = h;
       e.hv2[p] = (T)((double)e.F[p] * h);
@@ -307,14 +322,14 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
     }
     if (!e.last) return;
     for (int q = tid; q < e.i0 * kc; q += FRAG_BS) {
-      const double h = __ldcg(&e.h2[(q / kc) * k + e.c0 + q % kc]);
+      const double h = __ldcg(&e.h2[(q / kc) * k + c0 + q % kc]);
       need |= h * h > e.h2_lim * nrm[q % kc];
     }
-    if (tid < kc) need |= nrm[tid] < 0.5 * e.nrm0[e.c0 + tid];
+    if (tid < kc) need |= nrm[tid] < 0.5 * e.nrm0[c0 + tid];
     __threadfence_block();
     const int any = __syncthreads_or(need);
     if (flagged && tid < kc) {
-      const int s = e.c0 + tid;
+      const int s = c0 + tid;
       double gn = 0.0;
       for (int i = 0; i <= j; i++)
         gn -= __ldcg(&e.gam[i * k + s]) *
@@ -322,18 +337,18 @@ __device__ __forceinline__ void kry_epilogue(const KryArgs<T>& a, int nqo, int n
       e.gam[(j + 1) * k + s] = gn;
     }
     for (int q = tid; q < (j + 1) * kc; q += FRAG_BS) {
-      const int i = q / kc, s = e.c0 + q % kc;
+      const int i = q / kc, s = c0 + q % kc;
       e.H[((int64_t)i * m + j) * k + s] = __ldcg(&e.h1[i * k + s]) + (any ? __ldcg(&e.h2[i * k + s]) : 0.0);
     }
-    if (tid == 0) *e.reorth = any;
+    if (tid == 0) e.reorth[blockIdx.y] = any;
     __threadfence();
-    if (!any) kry_step<T>(e, kc, nrm, sm);
+    if (!any) kry_step<T>(e, c0, kc, nrm, sm);
   } else if (is(KE_STEP)) {
-    kry_step<T>(e, kc, nrm, sm);
+    kry_step<T>(e, c0, kc, nrm, sm);
   } else if (is(KE_NORM)) {
     if (tid < kc) {
       const double nr = sqrt(fmax(nrm[tid], 0.0));
-      e.finv[e.c0 + tid] = nr > 0.0 ? (T)(1.0 / nr) : T(0);
+      e.finv[c0 + tid] = nr > 0.0 ? (T)(1.0 / nr) : T(0);
     }
   }
 }
@@ -352,10 +367,12 @@ template <class T, int KINDS>
 __device__ __forceinline__ void kry_totals(const KryArgs<T>& a, int nqo, int nbo, const double* red, int stride,
                                            double* sm)
 {
-  const int tid = threadIdx.x, nout = (nqo + nbo + 1) * a.kc;
+  const int tid = threadIdx.x, nout = (nqo + nbo + 1) * KryGrp(a.k, a.per).kc;
   // loaded ahead of the sums, whose latency covers it
   constexpr bool uses = (KINDS & (1 << KE_LZ | 1 << KE_GS | 1 << KE_GS2)) != 0;
-  const int flag = uses && a.e.gflag && a.e.kind != KE_START ? __ldcg(a.e.gflag) : 0;
+  const int flag = uses && a.e.gflag && a.e.kind != KE_START ? __ldcg(a.e.gflag + blockIdx.y) : 0;
+  double* const part = a.part + blockIdx.y * a.part_step;
+  unsigned int* const counters = a.counters + blockIdx.y * a.cnt_step;
   __syncthreads();
   double tot[2];
 #pragma unroll
@@ -365,14 +382,14 @@ __device__ __forceinline__ void kry_totals(const KryArgs<T>& a, int nqo, int nbo
     if (o < nout) {
 #pragma unroll
       for (int b = 0; b < FRAG_NW; b++) tot[q] += red[b * stride + o];
-      a.part[(int64_t)blockIdx.x * nout + o] = tot[q];
+      part[(int64_t)blockIdx.x * nout + o] = tot[q];
     }
   }
   if (nout <= FRAG_BS) {
     double one[1] = {tot[0]};
-    if (!frag_tree_sum<1>(a.part, nout, a.gsz, a.counters, one)) return;
+    if (!frag_tree_sum<1>(part, nout, a.gsz, counters, one)) return;
     tot[0] = one[0];
-  } else if (!frag_tree_sum<2>(a.part, nout, a.gsz, a.counters, tot)) {
+  } else if (!frag_tree_sum<2>(part, nout, a.gsz, counters, tot)) {
     return;
   }
 #pragma unroll
@@ -389,7 +406,8 @@ __device__ __forceinline__ void kry_finish(const KryArgs<T>& a, int nqo, int nbo
 {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
   if (a.e.kind == KE_NONE) return;  // the update alone
-  const int kc = a.kc, kp = a.kp, s = lane & (kp - 1);
+  const KryGrp gr(a.k, a.per);
+  const int kc = gr.kc, kp = gr.kp, s = lane & (kp - 1);
   double nd = (double)na, vd[MJ];
 #pragma unroll
   for (int i = 0; i < MJ; i++) vd[i] = i < nbo ? (double)va[i] : 0.0;
@@ -424,7 +442,7 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
 {
   pdl_begin();
   pdl_wait();
-  if (a.skip && *a.skip == 0) return;
+  if (a.skip && a.skip[blockIdx.y] == 0) return;
   // packed steps, 4-row steps of Q'W and row tiles of Q cq with their loads in flight
   constexpr int UB = MJ <= 2 ? 4 : sizeof(T) == 4 ? (MJ <= 8 ? 4 : 2) : (MJ <= 8 ? 2 : 1);
   constexpr int QU = sizeof(T) == 4 ? 8 : 4;
@@ -432,7 +450,8 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
   constexpr int RTB = MQ <= 2 ? 4 : 2;
   __shared__ double sm[KRY_RED];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int kc = a.kc, kp = a.kp, k = a.k, nb = a.nb, nq = a.nq;
+  const KryGrp gr(a.k, a.per);
+  const int c0 = gr.c0, kc = gr.kc, kp = gr.kp, k = a.k, nb = a.nb, nq = a.nq;
   const int s = lane & (kp - 1), rr = lane / kp, rs = 32 / kp;
   const bool mine = s < kc;
   double* sC = sm + KRY_SC;
@@ -441,11 +460,11 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
   if (UPD) {
     for (int q = tid; q < 2 * MQ * 32; q += FRAG_BS) {
       const int l = q & 31, i = 4 * (q >> 5) + (l & 3), c = l >> 2;
-      sC[q] = (i < nq && c < kc) ? (double)a.cq[i * k + c] : 0.0;
+      sC[q] = (i < nq && c < kc) ? (double)a.cq[i * k + c0 + c] : 0.0;
     }
     for (int q = tid; q < MJ * KRY_MAXC; q += FRAG_BS) {
       const int i = q / KRY_MAXC, c = q % KRY_MAXC;
-      sH[q] = (i < nb && c < kc) ? a.hv[i * k + c] : T(0);
+      sH[q] = (i < nb && c < kc) ? a.hv[i * k + c0 + c] : T(0);
     }
     __syncthreads();
   }
@@ -472,7 +491,7 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
           const T* pq = a.Q + (ok ? row : 0) * a.ldq;
 #pragma unroll
           for (int i = 0; i < MQ; i++) kry_ldp(pq + min(8 * i + g, nq - 1), ok, qv[u][i]);
-          kry_ldp(a.W + (ok ? row : 0) * k + min(g, kc - 1), ok, wv[u]);
+          kry_ldp(a.W + (ok ? row : 0) * k + c0 + min(g, kc - 1), ok, wv[u]);
         }
 #pragma unroll
         for (int u = 0; u < QU; u++)
@@ -510,7 +529,7 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
       for (int u = 0; u < UB; u++) {
         const int64_t row = r0 + (int64_t)(u0 + u) * rs + rr;
         const bool ok = mine && u0 + u < kp && row < a.n;
-        const int64_t at = ok ? row * k + s : 0;
+        const int64_t at = ok ? row * k + c0 + s : 0;
         kry_ldp(a.Win + at, ok && a.Win, wv[u]);
 #pragma unroll
         for (int i = 0; i < MJ; i++) kry_ldp(a.V + i * a.vstep + at, ok && i < nb, v[u][i]);
@@ -525,7 +544,7 @@ __global__ void __launch_bounds__(FRAG_BS, 2) k_kry(const __grid_constant__ KryA
           if (MQ > 0 && ok) x -= (T)tile[lr * 9 + s];
 #pragma unroll
           for (int i = 0; i < MJ; i++) x -= v[u][i] * sH[i * KRY_MAXC + s];
-          if (ok) a.W[row * k + s] = x;
+          if (ok) a.W[row * k + c0 + s] = x;
           else x = T(0);
         }
         if (DOTS) {
@@ -549,18 +568,19 @@ __global__ void __launch_bounds__(FRAG_BS) k_kry_start(const __grid_constant__ K
   pdl_wait();
   __shared__ double sm[KRY_RED];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int kc = a.kc, kp = a.kp, k = a.k;
+  const KryGrp gr(a.k, a.per);
+  const int c0 = gr.c0, kc = gr.kc, kp = gr.kp, k = a.k;
   const int s = lane & (kp - 1), rs = 32 / kp;
   T na = T(0);
   if (s < kc) {
-    const int col = a.idx.v[a.e.c0 + s];
-    const bool zero = a.restart && a.e.conv[a.e.c0 + s];
+    const int col = a.idx.v[c0 + s];
+    const bool zero = a.restart && a.e.conv[c0 + s];
     const int64_t step = gridDim.x * (int64_t)FRAG_NW * rs;
 #pragma unroll 4
     for (int64_t row = (blockIdx.x * (int64_t)FRAG_NW + w) * rs + lane / kp; row < a.n; row += step) {
       T x = a.R[row * a.ldr + col];
-      if (a.restart) x = zero ? T(0) : x - a.W[row * k + s];
-      a.W[row * k + s] = x;
+      if (a.restart) x = zero ? T(0) : x - a.W[row * k + c0 + s];
+      a.W[row * k + c0 + s] = x;
       na += x * x;
     }
   }
