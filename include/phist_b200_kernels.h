@@ -460,8 +460,11 @@ void phist_b200_set_spmv_prefetch(int on, int* iflag);
  * (0); both give bitwise identical results */
 void phist_b200_set_graphs(int on, int* iflag);
 /* kernel-path switches, all on by default (1) and each also read from the
- * environment at init: "tma" (TMA-staged block products, PHIST_B200_TMA),
- * "dmma" (FP64 tensor-core tiles, PHIST_B200_DMMA), "graphs" (as
+ * environment at init: "tma" (TMA staging of the block products that stage
+ * their rows in shared memory: the wide aligned ones and W C in place with V'W
+ * of another block, PHIST_B200_TMA), "dmma" (FP64 tensor-core tiles in these
+ * staged products, PHIST_B200_DMMA; all other block products take their
+ * fragments straight from global memory whatever the two say), "graphs" (as
  * phist_b200_set_graphs, PHIST_B200_GRAPHS), "carp_blocks" (CARP sweeps
  * over a block colouring with X staged in shared memory, else one launch per
  * row colour class; PHIST_B200_CARP_BLOCKS; applies to CARP work set up

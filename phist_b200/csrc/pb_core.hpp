@@ -211,9 +211,11 @@ class Runtime {
   // 12 / 17 / 21 % more bandwidth at widths 4 / 8 / 16 on the L=128 Anderson
   // matrix (bitwise the same results)
   bool spmv_v256 = true;
-  // stage block-vector tiles of the Gram kernels with TMA (else cp.async)
+  // the block products that stage row tiles in shared memory (pb_tile.cuh,
+  // pb_dmma.cuh) do it with TMA (else cp.async)
   bool use_tma = true;
-  // FP64 block products on the tensor cores (DMMA) for widths multiple of 8
+  // and form FP64 products on the tensor cores (DMMA); the fragment kernels
+  // (pb_frag.cuh), which take most shapes, look at neither
   bool use_dmma = true;
   // batched CARP-CG replays its iteration as a CUDA graph (PHIST_B200_GRAPHS=0: plain launches)
   bool use_graphs = true;
