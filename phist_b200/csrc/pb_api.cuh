@@ -1276,6 +1276,7 @@ template <class T>
 bool launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const T* W,
                   int64_t ldw, T beta, T* Cd, int64_t ldc, T* mbox = nullptr)
 {
+  if (m < 1 || k < 1) return false;  // no outputs
   if (frag_mvTmv<T>(n, m, k, alpha, V, ldv, W, ldw, beta, Cd, ldc, mbox)) return mbox != nullptr;
   MvTmvArgs<T> a;
   a.n = n; a.m = m; a.k = k; a.V = V; a.ldv = ldv; a.W = W; a.ldw = ldw;
@@ -1460,7 +1461,7 @@ inline bool mvsd_gram_dmma(RowGemmArgs<float>&) { return false; }
 template <class T>
 bool launch_rowgemm(RowGemmArgs<T>& a, T* mbox = nullptr)
 {
-  if (a.n == 0 && a.gram == GM_NONE) return false;
+  if ((a.n == 0 && a.gram == GM_NONE) || a.k < 1) return false;
   // fused V*C + Gram in one pass on the tensor cores
   // Thin blocks of many rows stay with the register kernel, whose rows cost
   // less (us, fragments | registers: FP64 4 x 4 at 1,048,576 rows 37.5 | 39.5, at

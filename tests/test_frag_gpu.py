@@ -211,3 +211,18 @@ def test_four_columns(session, n, vld, vo, wld, wo):
     assert np.abs(G.get() - v.T @ w).max() <= (n + 3) * (n + 3) * eps
     for o in (V, W, C, D, G, Vb, Wb, mp, mq):
         o.delete()
+
+
+def test_no_columns_in_the_result(session):
+    """a factor of no columns: nothing to form, whatever the other block"""
+    from phist_b200 import kernels as K
+    from phist_b200.objects import Map, Mvec, SdMat
+    mp = Map(1000)
+    for mv in (1, 5, 20, 64):
+        V, W = Mvec(mp.h, mv), Mvec(mp.h, 4).set(np.ones((1000, 4)))
+        C, D = SdMat(4, 0), SdMat(mv, 0)
+        K.chk(K.phist_Dfused_mvsdi_mvTmv, 1.0, V.h, W.h, C.h, 0.0, D.h)
+        assert (W.get() == 1.0).all()
+        for o in (V, W, C, D):
+            o.delete()
+    mp.delete()
