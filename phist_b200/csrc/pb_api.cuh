@@ -880,7 +880,7 @@ void spmv_any(const SparseMat<T>* A, const SellDev<T>& S, SpmvArgs<T>& p)
   } else {
     const int u = p.nvec;
     if (u <= 8) switch (u) {
-        PB_ANY(1, 1, 1) PB_ANY(1, 1, 2) PB_ANY(1, 1, 3) PB_ANY(1, 1, 4) PB_ANY(1, 1, 5) PB_ANY(1, 1, 6)
+        PB_ANY(1, 1, 2) PB_ANY(1, 1, 3) PB_ANY(1, 1, 4) PB_ANY(1, 1, 5) PB_ANY(1, 1, 6)
         PB_ANY(1, 1, 7) PB_ANY(1, 1, 8)
       }
     else if (u <= 16) switch ((u + 1) / 2) { PB_ANY(1, 2, 5) PB_ANY(1, 2, 6) PB_ANY(1, 2, 7) PB_ANY(1, 2, 8) }
@@ -1316,8 +1316,8 @@ bool launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, con
     PB_LAUNCH_CHECK();
     return false;
   }
-  if (m <= 8 && k <= 8) {
-    // register kernel (odd or unaligned widths): padded widths M (4|8) and K (1|4|8)
+  if (thin) {
+    // register kernel: padded widths M (4, FP32 also 8) and K (1|4, FP32 also 8)
     const int M = m <= 4 ? 4 : 8, K = k == 1 ? 1 : k <= 4 ? 4 : 8;
     const int grid = std::max(1, std::min(grid_for(n), rt().num_sms() * 4));
     a.part = (T*)rt().scratch(sizeof(T) * (size_t)grid * M * K);
@@ -1325,10 +1325,12 @@ bool launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, con
     a.R = 0;
     a.mbox = mbox;
 #define PB_MVR(Mv, Kv) k_mvTmv_reg<T, Mv, Kv><<<grid, 256, 0, stream()>>>(a)
-    if (M == 4) {
+    if constexpr (sizeof(T) == 8) {
+      if (K == 1) PB_MVR(4, 1); else PB_MVR(4, 4);
+    } else if (M == 4) {
       if (K == 1) PB_MVR(4, 1); else if (K == 4) PB_MVR(4, 4); else PB_MVR(4, 8);
     } else {
-      if (K == 1) PB_MVR(8, 1); else if (K == 4) PB_MVR(8, 4); else PB_MVR(8, 8);
+      if (K == 1) PB_MVR(8, 1); else PB_MVR(8, 4);
     }
 #undef PB_MVR
     PB_LAUNCH_CHECK();
@@ -1474,7 +1476,8 @@ bool launch_rowgemm(RowGemmArgs<T>& a, T* mbox = nullptr)
   if (mvsd_gram_dmma(a)) return false;
   if (a.gram == GM_NONE && a.mode != RM_VCWD && frag_mvsd(a)) return false;
   if (a.m <= 8 && a.k <= 8 && (thin || a.mode == RM_VCWD) && (a.gram != GM_VW || a.mv <= 8)) {
-    // register kernel (thin blocks, V C + W D): padded widths M (4|8), K (1|4|8), MV (1, or 8 for V'W)
+    // register kernel (thin blocks, V C + W D): padded widths M (4|8), K (1|4|8), MV (1, or 8 for V'W;
+    // the products with a Gram have K <= 4, in FP64 M = 4)
     const int M = a.m <= 4 ? 4 : 8, K = a.k == 1 ? 1 : a.k <= 4 ? 4 : 8;
     const int grid = std::max(1, std::min(grid_for(a.n), rt().num_sms() * 4));
     if (a.gram != GM_NONE) {
@@ -1491,16 +1494,15 @@ bool launch_rowgemm(RowGemmArgs<T>& a, T* mbox = nullptr)
       }
     }
 #define PB_RGR(Mv, Kv, MVv) k_rowgemm_reg<T, Mv, Kv, MVv><<<grid, 256, 0, stream()>>>(a)
-#define PB_RGR_K(Mv, MVv)                                   \
-  if (K == 1) PB_RGR(Mv, 1, MVv);                           \
-  else if (K == 4) PB_RGR(Mv, 4, MVv);                      \
-  else PB_RGR(Mv, 8, MVv);
     if (a.gram == GM_VW) {
-      if (M == 4) { PB_RGR_K(4, 8) } else { PB_RGR_K(8, 8) }
+      if constexpr (sizeof(T) == 4)
+        if (M == 8) { if (K == 1) PB_RGR(8, 1, 8); else PB_RGR(8, 4, 8); }
+      if (M == 4) { if (K == 1) PB_RGR(4, 1, 8); else PB_RGR(4, 4, 8); }
+    } else if (M == 4) {
+      if (K == 1) PB_RGR(4, 1, 1); else if (K == 4) PB_RGR(4, 4, 1); else PB_RGR(4, 8, 1);
     } else {
-      if (M == 4) { PB_RGR_K(4, 1) } else { PB_RGR_K(8, 1) }
+      if (K == 1) PB_RGR(8, 1, 1); else if (K == 4) PB_RGR(8, 4, 1); else PB_RGR(8, 8, 1);
     }
-#undef PB_RGR_K
 #undef PB_RGR
     PB_LAUNCH_CHECK();
     return false;
