@@ -31,6 +31,8 @@
 //   FP64 64 x 64                      (staged kernel)  | 1,751 -> 641 [484]
 //   FP64 W'W, 8 / 16 / 32 columns      56 -> 39, 71 -> 64, 171 -> 119
 //   FP32 10 x 4                       260 -> 51 [18]   | 145 -> 46 [23]
+// and back to back with a warm L2, FP32 V*C of 32 x 32 373 -> 212 (beta = 0: 156
+// -> 170), of 64 x 64 1,020 -> 618 (516 -> 580, bound by the FP64 pipe).
 // The launch bound is part of that: with the two blocks per SM named, ptxas
 // keeps a whole chunk of loads in flight; without it 4 x 4 took 94 us, not 45.
 #pragma once
