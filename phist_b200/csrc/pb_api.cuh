@@ -1320,7 +1320,7 @@ bool launch_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, con
     // register kernel: padded widths M (4, FP32 also 8) and K (1|4, FP32 also 8)
     const int M = m <= 4 ? 4 : 8, K = k == 1 ? 1 : k <= 4 ? 4 : 8;
     const int grid = std::max(1, std::min(grid_for(n), rt().num_sms() * 4));
-    a.part = (T*)rt().scratch(sizeof(T) * (size_t)grid * M * K);
+    a.part = (T*)rt().scratch(sizeof(double) * (size_t)grid * M * K);
     a.counter = rt().counters();
     a.R = 0;
     a.mbox = mbox;

@@ -362,9 +362,12 @@ __global__ void __launch_bounds__(256) k_mvTmv_reg(MvTmvArgs<T> a)
   for (int q = 0; q < K; q++)
 #pragma unroll
     for (int p = 0; p < M; p++) vals[p + q * M] = acc[p + q * M];
-  block_partial<T, M * K>(vals, a.part, M * K);
+  // lanes and warps in T, from there on FP64 in both precisions (a.part)
+  double* part = reinterpret_cast<double*>(a.part);
+  block_partial<T, M * K>(vals, part, M * K);
   // outputs are laid out with row stride M in the partials: map to (m, k)
-  last_block_reduce<T>(a.part, M * K, gridDim.x, a.counter, a.Cd, 1, M, a.ldc, a.alpha, a.beta, a.m, a.k, a.mbox);
+  last_block_reduce<double>(part, M * K, gridDim.x, a.counter, a.Cd, 1, M, a.ldc, (double)a.alpha, (double)a.beta, a.m,
+                            a.k, a.mbox);
 }
 
 // Thin blocks of exactly M and K columns (multiples of 4) whose rows start

@@ -40,6 +40,13 @@ bool rows16(const T* p, int64_t ld, int ncol)
   return ((uintptr_t)p) % 16 == 0 && ld % vw == 0 && ncol % vw == 0;
 }
 
+// every row starts on a 32-byte boundary
+template <class T>
+bool rows32(const T* p, int64_t ld)
+{
+  return ((uintptr_t)p) % 32 == 0 && ld * sizeof(T) % 32 == 0;
+}
+
 template <class T, int MT, int KT, bool SYM, bool VEC>
 void tn_launch(FragTnArgs<T>& a)
 {
@@ -201,11 +208,17 @@ void launch_mvTmv_prec(int64_t n, int m, int k, double alpha, const double* V, i
 }
 
 // Which products go here (us at n = 2,097,152, fragment | other kernel):
-//   * thin ones (at most 4 columns against 4, FP32 8) of many rows stay with
-//     the register kernel, one row per thread: FP32 3 x 3 33 | 25, FP64 4 x 4
-//     43 | 39; up to 2^20 rows the shorter cross-block sum decides (n =
-//     262,144, W'W of 4 columns 12.3 | 16.4), and for W'W of 2 to 4 FP64
-//     columns always (26.7 | 28.7);
+//   * thin ones (at most 4 columns against 4, FP32 8): up to a number of rows
+//     the shorter cross-block sum decides, beyond it the row per thread of the
+//     register kernels costs less.  FP64 against one column from 2^19 rows
+//     (whole calls, back to back: 1 x 1 at 524,288 rows 17.9 | 18.0, at 1,048,576
+//     20.6 | 19.0), else the fragments are as fast or faster (3 x 3 40.6 | 42.6,
+//     W'W of 4 25.6 | 25.5) but for 4 x 4 in whole 32-byte rows (39.7 | 38.3).
+//     FP32 from 2^20 (4 x 4 at 1,048,576 21.7 | 23.0, at 2,097,152 27.3 | 26.9; 4 x 2
+//     21.3 | 21.6, 26.7 | 24.6), not with 5 to 8 columns against 2 to 4 (8 x 4 at
+//     2,097,152 34.6 | 42.4), and against one column no earlier either, though it
+//     would be faster from 2^19 on (4 x 1 18.0 | 17.4): the register kernel's
+//     lanes sum in FP32;
 //   * W'W up to 32 columns: half the tiles, one read (see pb_frag.cuh);
 //   * blocks on 16-byte rows keep the TMA-staged kernels where those share
 //     every row among many tiles: 64 x 8 207 | 202, 64 x 16 269 | 222,
@@ -220,7 +233,9 @@ bool frag_mvTmv(int64_t n, int m, int k, T alpha, const T* V, int64_t ldv, const
   const bool sym = V == W && ldv == ldw && m == k;
   const int big = std::max(m, k), small = std::min(m, k);
   const bool thin = small <= 4 && big <= (sizeof(T) == 4 ? 8 : 4);
-  if (thin && n > (1 << 20) && !(sym && sizeof(T) == 8 && m >= 2)) return false;
+  if (thin && n > (sizeof(T) == 8 && small == 1 ? 1 << 19 : 1 << 20) &&
+      (small == 1 || (sizeof(T) == 4 ? big <= 4 : !sym && small == 4 && rows32(V, ldv) && rows32(W, ldw))))
+    return false;
   const bool staged = rows16(V, ldv, m) && rows16(W, ldw, k);
   if (staged && (sym ? m > 32 : small > 8 ? big > 16 : big > 40)) return false;
   FragTnArgs<T> a;

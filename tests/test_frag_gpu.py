@@ -181,6 +181,14 @@ def test_thin_product_with_gram_of_many_rows(session, n, m, k, dtype):
     g = G.get()
     assert (np.abs(g - new.T @ new) <= (n * np.finfo(np.float64).eps + 15 * eps) * (np.abs(new).T @ np.abs(new))).all()
     assert np.array_equal(G.host(), g)
+    # the products alone, as above
+    D = SdMat(m, k, dtype)
+    for x, y, xm, S in ((V, W, v, D), (W, W, new, G)):
+        K.chk(fn(dtype, "mvecT_times_mvec"), 1.0, x.h, y.h, 0.0, S.h)
+        terms = np.abs(xm).T @ np.abs(new)
+        assert (np.abs(S.get() - xm.T @ new) <= (n * np.finfo(np.float64).eps + 15 * eps) * terms).all()
+        assert np.array_equal(S.host(), S.get())
+    D.delete()
     for o in (V, W, C, G, Vb, Wb, mp, mq):
         o.delete()
 
