@@ -1458,6 +1458,19 @@ inline bool mvsd_gram_dmma(RowGemmArgs<double>& a)
 }
 inline bool mvsd_gram_dmma(RowGemmArgs<float>&) { return false; }
 
+// V*C with W'W: thin blocks of many rows, which stay with the register kernel.
+// Its rows cost less (us, fragments | registers: FP64 4 x 4 at 1,048,576 rows
+// 37.5 | 39.5, at 1,572,864 53 | 40; 1 x 1 at 524,288 24.8 | 27.1, at 786,432 29 |
+// 28; FP32 4 x 4 at 262,144 23.6 | 26.8, at 786,432 36 | 32, at 2,097,152 69 | 40; 7 x 4
+// at 1,048,576 39 | 40, at 1,572,864 51 | 42), the fragment kernel has the shorter
+// cross-block sum and puts the result in the mailbox.
+template <class T>
+bool thin_gram_rows(int64_t n, int m, int k)
+{
+  const bool later = sizeof(T) == 8 ? k >= 2 : m > 4;
+  return k <= 4 && m <= (sizeof(T) == 4 ? 8 : 4) && n > (later ? 1 << 20 : 1 << 19);
+}
+
 // mbox: mapped host memory for a dense copy of the Gram matrix, or NULL; true
 // when the kernel wrote it
 template <class T>
@@ -1465,44 +1478,45 @@ bool launch_rowgemm(RowGemmArgs<T>& a, T* mbox = nullptr)
 {
   if ((a.n == 0 && a.gram == GM_NONE) || a.k < 1) return false;
   // fused V*C + Gram in one pass on the tensor cores
-  // Thin blocks of many rows stay with the register kernel, whose rows cost
-  // less (us, fragments | registers: FP64 4 x 4 at 1,048,576 rows 37.5 | 39.5, at
-  // 1,572,864 53 | 52; 1 x 1 at 524,288 24.8 | 27.1, at 786,432 29.2 | 27.2; FP32
-  // 4 x 4 at 262,144 23.6 | 26.8, at 524,288 30.3 | 28.5, at 2,097,152 69 | 39),
-  // the others have the shorter cross-block sum and the result in the mailbox
   const bool thin = a.k <= 4 && a.m <= (sizeof(T) == 4 ? 8 : 4);
-  const bool many = a.n > (sizeof(T) == 8 && a.k >= 2 ? 1 << 20 : 1 << 19);
-  if (a.gram == GM_WW && a.mode != RM_VCWD && !(thin && many) && frag_mvsd_gram<T>(a, mbox)) return mbox != nullptr;
+  if (a.gram == GM_WW && a.mode != RM_VCWD && !thin_gram_rows<T>(a.n, a.m, a.k) && frag_mvsd_gram<T>(a, mbox))
+    return mbox != nullptr;
   if (mvsd_gram_dmma(a)) return false;
   if (a.gram == GM_NONE && a.mode != RM_VCWD && frag_mvsd(a)) return false;
   if (a.m <= 8 && a.k <= 8 && (thin || a.mode == RM_VCWD) && (a.gram != GM_VW || a.mv <= 8)) {
-    // register kernel (thin blocks, V C + W D): padded widths M (4|8), K (1|4|8), MV (1, or 8 for V'W;
-    // the products with a Gram have K <= 4, in FP64 M = 4)
+    // register kernel (thin blocks, V C + W D): padded widths M (4|8) and K
+    // (1|4|8); the products with a Gram have K <= 4 and in FP64 M = 4
     const int M = a.m <= 4 ? 4 : 8, K = a.k == 1 ? 1 : a.k <= 4 ? 4 : 8;
     const int grid = std::max(1, std::min(grid_for(a.n), rt().num_sms() * 4));
     if (a.gram != GM_NONE) {
-      a.part = (T*)rt().scratch(sizeof(double) * (size_t)grid * 64);
+      a.part = (T*)rt().scratch(sizeof(double) * (size_t)grid * 32);
       a.counter = rt().counters();
     }
+#define PB_RGR(Mv, Kv, G, ...) k_rowgemm_reg<T, Mv, Kv, G, ##__VA_ARGS__><<<grid, 256, 0, stream()>>>(a)
     if constexpr (sizeof(T) == 8) {
       auto rows32 = [](const T* p, int64_t ld) { return (uintptr_t)p % 32 == 0 && ld % 4 == 0; };
       if (a.m == 4 && a.k == 4 && rows32(a.W, a.ldw) && (a.mode == RM_MVSDI || rows32(a.V, a.ldv))) {
-        if (a.gram == GM_VW) k_rowgemm_reg<T, 4, 4, 8, true><<<grid, 256, 0, stream()>>>(a);
-        else k_rowgemm_reg<T, 4, 4, 1, true><<<grid, 256, 0, stream()>>>(a);
+        if (a.gram == GM_NONE) PB_RGR(4, 4, GM_NONE, true);
+        else if (a.gram == GM_WW) PB_RGR(4, 4, GM_WW, true);
+        else PB_RGR(4, 4, GM_VW, true);
         PB_LAUNCH_CHECK();
         return false;
       }
     }
-#define PB_RGR(Mv, Kv, MVv) k_rowgemm_reg<T, Mv, Kv, MVv><<<grid, 256, 0, stream()>>>(a)
-    if (a.gram == GM_VW) {
-      if constexpr (sizeof(T) == 4)
-        if (M == 8) { if (K == 1) PB_RGR(8, 1, 8); else PB_RGR(8, 4, 8); }
-      if (M == 4) { if (K == 1) PB_RGR(4, 1, 8); else PB_RGR(4, 4, 8); }
-    } else if (M == 4) {
-      if (K == 1) PB_RGR(4, 1, 1); else if (K == 4) PB_RGR(4, 4, 1); else PB_RGR(4, 8, 1);
+#define PB_RGR_G(Mv)                                                                       \
+  if (a.gram == GM_WW) { if (K == 1) PB_RGR(Mv, 1, GM_WW); else PB_RGR(Mv, 4, GM_WW); }    \
+  else if (a.gram == GM_VW) { if (K == 1) PB_RGR(Mv, 1, GM_VW); else PB_RGR(Mv, 4, GM_VW); } \
+  else if (K == 1) PB_RGR(Mv, 1, GM_NONE);                                                 \
+  else if (K == 4) PB_RGR(Mv, 4, GM_NONE);                                                 \
+  else PB_RGR(Mv, 8, GM_NONE);
+    if (M == 4) {
+      PB_RGR_G(4)
+    } else if constexpr (sizeof(T) == 4) {
+      PB_RGR_G(8)
     } else {
-      if (K == 1) PB_RGR(8, 1, 1); else if (K == 4) PB_RGR(8, 4, 1); else PB_RGR(8, 8, 1);
+      if (K == 1) PB_RGR(8, 1, GM_NONE); else if (K == 4) PB_RGR(8, 4, GM_NONE); else PB_RGR(8, 8, GM_NONE);
     }
+#undef PB_RGR_G
 #undef PB_RGR
     PB_LAUNCH_CHECK();
     return false;

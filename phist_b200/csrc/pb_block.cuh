@@ -427,15 +427,15 @@ __device__ __forceinline__ void st_row4(double* p, const double* v)
 }
 
 // Row-local products for m, k, mv <= 8 (modes and Gram as k_rowgemm, the Gram
-// for k <= 4 only).  The Gram sums of the lanes and of a warp are formed in T,
-// from there on in FP64 (a.part): the errors of some 4,700 warps average out
-// below the rounding of the result.  FP64 in the lanes of FP32 blocks, too,
-// costs conversions and registers that the gram-free calls pay as well (4
-// columns in place at 2,097,152 rows 14 -> 19 us).
+// for k <= 4 only).  W'W is formed and summed in FP64 in both precisions, its
+// upper triangle alone, as in pb_frag.cuh; V'W of FP32 blocks in FP32 up to a
+// warp and in FP64 from there on (a.part).  The Gram is a compile-time form:
+// its sums cost registers that the plain product must not pay (4 FP32 columns
+// in place at 2,097,152 rows 14 -> 19 us).
 // V4: V and W have 4 FP64 columns and rows on 32-byte boundaries, which are
 // moved whole (us, element by element | so: in place at 1,048,576 rows 20.4 |
 // 12.3, at 2,097,152 35.8 | 20.4; W = V C 17.2 | 12.3, 36.7 | 30.8).
-template <class T, int M, int K, int MV, bool V4 = false>
+template <class T, int M, int K, int GRAM, bool V4 = false>
 __global__ void __launch_bounds__(256) k_rowgemm_reg(RowGemmArgs<T> a)
 {
   static_assert(!V4 || (M == 4 && K == 4 && sizeof(T) == 8), "rows of 32 bytes");
@@ -451,11 +451,12 @@ __global__ void __launch_bounds__(256) k_rowgemm_reg(RowGemmArgs<T> a)
       sD[t] = (i < a.k && j < a.k) ? a.D[i + j * a.ldd] : T(0);
     }
   __syncthreads();
-  constexpr bool GRAM = K <= 4;
-  constexpr int GM = (MV > K) ? MV : K, NG = GRAM ? GM * K : 1;
-  T gacc[NG];
+  static_assert(GRAM == GM_NONE || K <= 4, "Gram of at most 4 columns");
+  constexpr int GR = GRAM == GM_WW ? K : 8, NG = GRAM == GM_NONE ? 1 : GR * K;  // GR rows, padded
+  typedef typename std::conditional<GRAM == GM_WW, double, T>::type TG;
+  TG gacc[NG];
 #pragma unroll
-  for (int q = 0; q < NG; q++) gacc[q] = T(0);
+  for (int q = 0; q < NG; q++) gacc[q] = TG(0);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
        i += (int64_t)gridDim.x * blockDim.x) {
     T v[8], w[8], out[8];
@@ -487,32 +488,35 @@ __global__ void __launch_bounds__(256) k_rowgemm_reg(RowGemmArgs<T> a)
       for (int q = 0; q < K; q++)
         if (q < a.k) a.W[i * a.ldw + q] = out[q];
     }
-    if constexpr (GRAM) {
-      if (a.gram == GM_WW) {
+    if constexpr (GRAM == GM_WW) {
+      double od[K];
 #pragma unroll
-        for (int q = 0; q < K; q++)
+      for (int q = 0; q < K; q++) od[q] = (double)out[q];
 #pragma unroll
-          for (int p = 0; p < K; p++) gacc[p + q * K] += out[p] * out[q];
-      } else if (a.gram == GM_VW) {
-        T g[8];
-        load_row(a.Vg + i * a.ldvg, a.mv, MV, g);
+      for (int q = 0; q < K; q++)
 #pragma unroll
-        for (int q = 0; q < K; q++)
+        for (int p = 0; p <= q; p++) gacc[p + q * K] += od[p] * od[q];
+    } else if constexpr (GRAM == GM_VW) {
+      T g[8];
+      load_row(a.Vg + i * a.ldvg, a.mv, GR, g);
 #pragma unroll
-          for (int p = 0; p < MV; p++) gacc[p + q * MV] += g[p] * out[q];
-      }
+      for (int q = 0; q < K; q++)
+#pragma unroll
+        for (int p = 0; p < GR; p++) gacc[p + q * GR] += g[p] * out[q];
     }
   }
-  if constexpr (GRAM) {
-    if (a.gram == GM_NONE) return;
-    const int gmax = (a.gram == GM_WW) ? K : MV;
-    // partial layout: gmax rows (padded), K columns
+  if constexpr (GRAM != GM_NONE) {
+    if constexpr (GRAM == GM_WW) {
+#pragma unroll
+      for (int q = 0; q < K; q++)
+#pragma unroll
+        for (int p = q + 1; p < K; p++) gacc[p + q * K] = gacc[q + p * K];
+    }
     double* part = reinterpret_cast<double*>(a.part);
-    block_partial<T, NG>(gacc, part, gmax * K);
-    const double al = (a.gram == GM_WW) ? 1.0 : (double)a.galpha;
-    const double be = (a.gram == GM_WW) ? 0.0 : (double)a.gbeta;
-    last_block_reduce<double>(part, gmax * K, gridDim.x, a.counter, a.Gd, 1, gmax, a.ldg, al, be,
-                              (a.gram == GM_WW) ? a.k : a.mv, a.k);
+    block_partial<TG, NG>(gacc, part, NG);
+    const double al = GRAM == GM_WW ? 1.0 : (double)a.galpha, be = GRAM == GM_WW ? 0.0 : (double)a.gbeta;
+    last_block_reduce<double>(part, NG, gridDim.x, a.counter, a.Gd, 1, GR, a.ldg, al, be, GRAM == GM_WW ? a.k : a.mv,
+                              a.k);
   }
 }
 
