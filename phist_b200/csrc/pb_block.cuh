@@ -514,9 +514,8 @@ __global__ void __launch_bounds__(256) k_rowgemm_reg(RowGemmArgs<T> a)
     }
     double* part = reinterpret_cast<double*>(a.part);
     block_partial<TG, NG>(gacc, part, NG);
-    const double al = GRAM == GM_WW ? 1.0 : (double)a.galpha, be = GRAM == GM_WW ? 0.0 : (double)a.gbeta;
-    last_block_reduce<double>(part, NG, gridDim.x, a.counter, a.Gd, 1, GR, a.ldg, al, be, GRAM == GM_WW ? a.k : a.mv,
-                              a.k);
+    last_block_reduce<double>(part, NG, gridDim.x, a.counter, a.Gd, 1, GR, a.ldg, (double)a.galpha, (double)a.gbeta,
+                              GRAM == GM_WW ? a.k : a.mv, a.k);
   }
 }
 

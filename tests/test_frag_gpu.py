@@ -176,12 +176,23 @@ def test_thin_product_with_gram_of_many_rows(session, n, m, k, dtype):
     K.chk(fn(dtype, "fused_mvsd_mvTmv"), 0.5, V.h, C.h, -0.5, W.h, G.h)
     new = W.get().astype(np.float64)
     assert np.abs(new - (0.5 * (v @ c.astype(np.float64)) - 0.5 * w)).max() <= (m + 3) * 2 * eps
-    # a lane adds at most 2^20 / (4 * 148 * 256) < 8 products in the precision of
-    # the block and a warp its lanes in 5 steps; from there on FP64, rounded once
     g = G.get()
-    assert (np.abs(g - new.T @ new) <= (n * np.finfo(np.float64).eps + 15 * eps) * (np.abs(new).T @ np.abs(new))).all()
+    assert (np.abs(g - new.T @ new) <= (n * np.finfo(np.float64).eps + eps) * (np.abs(new).T @ np.abs(new))).all()
     assert np.array_equal(G.host(), g)
-    # the products alone, as above
+    # W = W C in place with W'W of the new W, the result scaled and added
+    S = SdMat(k, k, dtype).set((rng.uniform(-1, 1, (k, k)) / k).astype(dtype))
+    old, d0 = new, rng.uniform(-1, 1, (k, k)).astype(dtype)
+    G.set(d0)
+    K.chk(fn(dtype, "fused_mvsdi_mvTmv"), 0.5, W.h, W.h, S.h, 2.0, G.h)
+    new = W.get().astype(np.float64)
+    assert np.abs(new - old @ S.get().astype(np.float64)).max() <= (k + 3) * 2 * eps
+    terms = 0.5 * (np.abs(new).T @ np.abs(new)) + 2 * np.abs(d0)
+    assert (np.abs(G.get() - (0.5 * new.T @ new + 2.0 * d0)) <= (n * np.finfo(np.float64).eps + 2 * eps) * terms).all()
+    assert np.array_equal(G.host(), G.get())
+    S.delete()
+    # the products alone: a lane of the register kernel adds at most 2^20 / (4 *
+    # 148 * 256) < 8 products in the precision of the block and a warp its lanes
+    # in 5 steps; from there on FP64, rounded once
     D = SdMat(m, k, dtype)
     for x, y, xm, S in ((V, W, v, D), (W, W, new, G)):
         K.chk(fn(dtype, "mvecT_times_mvec"), 1.0, x.h, y.h, 0.0, S.h)
